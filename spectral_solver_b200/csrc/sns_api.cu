@@ -377,7 +377,7 @@ void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt
   mark(pm, 2, st);
   o->xpass_rot(h->work, u_src, h->xf, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->tw, g, st);
   mark(pm, 3, st);
-  o->nyq_reduce(h->work, h->nyq_part, g, st);  // the first 6 sums are the products'
+  o->nyq_reduce(h->work, 6, h->nyq_part, g, st);
   mark(pm, 4, st);
   o->yz_tma(h->map_work_y, 1, -1, 0, tma_args(h, 0, 6, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
             h->tma_grid, st);
@@ -389,9 +389,11 @@ void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt
   mark(pm, 7, st);
 }
 
-// One RK3 stage (or the RHS only, mode 1) on u_src: the five fused passes.
+// One RK3 stage (or the RHS only, mode 1; the unprojected nonlinear term, mode 2) on u_src: the
+// five fused passes.  The projected forms run on 5 products (the squares less u_2^2, a
+// gradient's difference that the projection removes), mode 2 on all 6, as separate kernels.
 void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, int mode, char* rhs_out,
-               double* partials, PassMarks* pm = nullptr) {
+               PassMarks* pm = nullptr) {
   if (h->form == 1) {
     run_stage_rot(h, u_src, g_buf, stage, dt, mode, rhs_out, pm);
     return;
@@ -401,7 +403,8 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   cudaStream_t st = h->stream;
   const int tiles_in = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   const int f_src = (int)((size_t)(u_src - h->state) / h->fbytes);  // u (0) or the g slot (3)
-  const bool fused = h->p5_grid > 0;
+  const int np = mode == 2 ? 6 : 5;
+  const bool fused = h->p5_grid > 0 && np == 5;
   // Sphere pruning (RK update with the fused P5 only).  A column-block tile (my, cb) outside
   // the disk 4 ((cb * TW)^2 + my^2) <= N^2 holds only modes outside the sphere: u is zero
   // there before the stage (every stage's sweep zeroes those modes, so stages 1 and 2 may
@@ -419,22 +422,22 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
             st);
   mark(pm, 2, st);
   int nparts = 1;
-  if (h->x2_grid > 0 && partials == nullptr) {
+  if (h->x2_grid > 0 && np == 5) {
     o->xpass2(h->work, u_src, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->nyq_part, h->tw2, g, h->x2_grid,
               h->err_word, st);
     nparts = h->x2_grid;
     mark(pm, 3, st);
   } else {
-    o->xpass_products(h->work, u_src, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, partials, h->tw, g, st);
+    o->xpass_products(h->work, np, u_src, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->tw, g, st);
     mark(pm, 3, st);
-    o->nyq_reduce(h->work, h->nyq_part, g, st);
+    o->nyq_reduce(h->work, 2 * np, h->nyq_part, g, st);
   }
   mark(pm, 4, st);
-  o->yz_tma(h->map_work_y, 1, -1, 0, tma_args(h, 0, 12, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
+  o->yz_tma(h->map_work_y, 1, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
             h->tma_grid, st);
   mark(pm, 5, st);
   if (!fused)
-    o->yz_tma(h->map_work_z, 2, -1, 0, tma_args(h, 0, 12, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
+    o->yz_tma(h->map_work_z, 2, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
               h->tma_grid, st);
   mark(pm, 6, st);
   const sns::SweepArgs a = stage_args(h, stage, dt, mode, u_src);
@@ -442,14 +445,14 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
     o->p5(h->map_work_z, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->tw, h->phase, a, h->tiles_data(),
           prune ? h->live : nullptr, prune ? h->nlive : 0, g, h->p5_grid, h->err_word, st);
   else
-    o->sweep(h->work, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->phase, a, g, st);
+    o->sweep(h->work, np, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->phase, a, g, st);
   mark(pm, 7, st);
 }
 
 void step_once(sns_handle* h, double dt) {
   const bool deferred = capturing(h->stream);  // a captured graph runs later, on whatever state
   for (int s = 0; s < 3; ++s) {
-    run_stage(h, h->u(), h->gb(), s, dt, 0, nullptr, nullptr);
+    run_stage(h, h->u(), h->gb(), s, dt, 0, nullptr);
     h->nyq_clean = true;  // the sweep zeroes the plane mx = N/2 off (N/2,0,0)
     // and every mode outside the sphere, once the stage has run
     if (!deferred) h->sphere_clean = true;
@@ -1122,7 +1125,7 @@ int sns_rhs(sns_handle* h, const double* const uhat_full[3], double* const rhs_f
     }
     const bool saved = h->nyq_clean;
     h->nyq_clean = !dirty;
-    run_stage(h, uin, nullptr, 0, 0.0, 1, h->work, nullptr);
+    run_stage(h, uin, nullptr, 0, 0.0, 1, h->work);
     h->nyq_clean = saved;
     for (int c = 0; c < 3; ++c) {
       download_full(h, h->wf(c), rhs_full[c]);
@@ -1146,7 +1149,7 @@ int sns_nonlinear(sns_handle* h, const double* const uhat_full[3], double* const
     }
     const bool saved = h->nyq_clean;
     h->nyq_clean = !dirty;
-    run_stage(h, uin, nullptr, 0, 0.0, 2, h->work, nullptr);
+    run_stage(h, uin, nullptr, 0, 0.0, 2, h->work);
     h->nyq_clean = saved;
     for (int c = 0; c < 3; ++c) {
       download_full(h, h->wf(c), out_full[c]);
@@ -1185,7 +1188,7 @@ int sns_profile_passes(sns_handle* h, double dt, int nsteps, double* pass_ms) {
     double acc[SNS_NUM_PASSES] = {0};
     for (int s = 0; s < nsteps; ++s) {
       for (int st = 0; st < 3; ++st) {
-        run_stage(h, h->u(), h->gb(), st, dt, 0, nullptr, nullptr, &pm);
+        run_stage(h, h->u(), h->gb(), st, dt, 0, nullptr, &pm);
         h->nyq_clean = true;
         h->sphere_clean = true;
         sync(h, "sns_profile_passes");

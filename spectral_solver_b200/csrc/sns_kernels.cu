@@ -7,9 +7,10 @@
 //   P1 zpass_inv_phase : inverse z transform of u_hat, both grids from one read
 //                        (the phase-shift kernel :866-873 fused in), 1/N^3 folded in
 //   P2 ypass (inverse) : 6 fields
-//   P3 xpass_products  : inverse x (c2r), the 6 products u_a*u_b on both grids,
-//                        forward x (r2c) of all 12 (product kernel :903-906 fused)
-//   P4 ypass (forward) : 12 fields
+//   P3 xpass_products  : inverse x (c2r), the 5 products on both grids (6 for the
+//                        unprojected term), forward x (r2c) of all 10 (product kernel
+//                        :903-906 fused)
+//   P4 ypass (forward) : 10 fields
 //   P5 zpass (forward) + sweep : dealias combine, mask, -i k, viscous term, Leray
 //                        projection, low-storage RK3 update, projection of u
 //                        (accumulate :926-936, add_viscous_project :955-974,
@@ -332,15 +333,28 @@ __device__ __forceinline__ void block_sum_max(double& s, double& m, double* red)
   }
 }
 
+// The products of the nonlinear term on one grid (or both: real and imaginary part).  The
+// conservative form needs u_a u_b, 6 products.  A field q added to all three diagonal ones
+// changes the term -i k_b FFT(u_a u_b) by -i k_a q_hat, a gradient, which the projection
+// removes; q = -u_2 u_2 makes the last product zero, so every projected right-hand side
+// (stepping, sns_rhs) runs on 5: u_0^2 - u_2^2, u_0 u_1, u_0 u_2, u_1^2 - u_2^2, u_1 u_2 --
+// 10 instead of 12 fields through the forward passes.  sns_nonlinear returns the term
+// unprojected and takes the 6.  The differences are formed as (a - b)(a + b), whose rounding
+// error is relative to the difference.  A stage moves 79 instead of 87 N^3 words: a step at
+// 512^3 29.1 -> 26.7 ms (FP32), at 256^3 7.1 -> 6.5 ms (FP64), error against 64 bits unchanged.
+template <class C>
+__device__ __forceinline__ C diff_squares(C a, C b) {
+  return cmk((a.x - b.x) * (a.x + b.x), (a.y - b.y) * (a.y + b.y));
+}
+
 // P3: fused inverse x / products / forward x.  One row (y, z) per CTA.
 // Input work fields 0..5 = (U_0, V_0, U_1, V_1, U_2, V_2) [V = shifted grid] after the
 // y and z inverse passes; output work fields 2p, 2p+1 = (P0_p, Ps_p) for the pairs
-// p = 00, 01, 02, 11, 12, 22, columns 0..N/2 (column N/2: per-row Nyquist value).
-template <int N, class C>
+// p = 00, 01, 02, 11, 12, 22 (NP = 6) or the 5 above, columns 0..N/2 (column N/2: per-row Nyquist value).
+template <int N, class C, int NP>
 __global__ void __launch_bounds__(nt_x<N>())
 k_xpass_products(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase,
-                 double scale, int nyq_scalar, double* __restrict__ partials, const C* __restrict__ tw,
-                 Geom g) {
+                 double scale, int nyq_scalar, const C* __restrict__ tw, Geom g) {
   constexpr int NT = nt_x<N>();
   constexpr int NH = N / 2;
   constexpr int RP = row_pitch(N);
@@ -348,11 +362,9 @@ k_xpass_products(C* __restrict__ work, const C* __restrict__ unyq, const C* __re
   C* smem = reinterpret_cast<C*>(smraw_x);
   C* s_tw = smem;
   C* seq = smem + N;  // 6 sequences of pitch RP
-  __shared__ double red[2 * (NT / 32)];
   const int tid = threadIdx.x;
   load_twiddles<N>(s_tw, tw, tid, NT);
-  const long long row = blockIdx.x;
-  const long long rbase = row * g.pitch;
+  const long long rbase = (long long)blockIdx.x * g.pitch;
   // pack Z_c = U_c + i V_c
   for (int e = tid; e < 3 * (NH + 1); e += NT) {
     const int c = e / (NH + 1), k = e % (NH + 1);
@@ -375,31 +387,19 @@ k_xpass_products(C* __restrict__ work, const C* __restrict__ unyq, const C* __re
   }
   __syncthreads();
   smem_fft<N, +1, 3, NT, RowTile<RP>>(seq, s_tw, tid);
-  double esum = 0.0, vmax2 = 0.0;
   for (int x = tid; x < N; x += NT) {
     const int p = x + (x >> 3);
     const C z0 = seq[p], z1 = seq[RP + p], z2 = seq[2 * RP + p];
-    const double a0 = z0.x, a1 = z1.x, a2 = z2.x;
-    const double s2 = a0 * a0 + a1 * a1 + a2 * a2;
-    esum += 0.5 * s2;
-    vmax2 = fmax(vmax2, s2);
-    seq[0 * RP + p] = cmk(z0.x * z0.x, z0.y * z0.y);
+    seq[0 * RP + p] = NP == 5 ? diff_squares(z0, z2) : cmk(z0.x * z0.x, z0.y * z0.y);
     seq[1 * RP + p] = cmk(z0.x * z1.x, z0.y * z1.y);
     seq[2 * RP + p] = cmk(z0.x * z2.x, z0.y * z2.y);
-    seq[3 * RP + p] = cmk(z1.x * z1.x, z1.y * z1.y);
+    seq[3 * RP + p] = NP == 5 ? diff_squares(z1, z2) : cmk(z1.x * z1.x, z1.y * z1.y);
     seq[4 * RP + p] = cmk(z1.x * z2.x, z1.y * z2.y);
-    seq[5 * RP + p] = cmk(z2.x * z2.x, z2.y * z2.y);
-  }
-  if (partials != nullptr) {
-    block_sum_max<NT>(esum, vmax2, red);
-    if (tid == 0) {
-      partials[2 * row] = esum;
-      partials[2 * row + 1] = vmax2;
-    }
+    if constexpr (NP == 6) seq[5 * RP + p] = cmk(z2.x * z2.x, z2.y * z2.y);
   }
   __syncthreads();
-  smem_fft<N, -1, 6, NT, RowTile<RP>>(seq, s_tw, tid);
-  for (int e = tid; e < 6 * (NH + 1); e += NT) {
+  smem_fft<N, -1, NP, NT, RowTile<RP>>(seq, s_tw, tid);
+  for (int e = tid; e < NP * (NH + 1); e += NT) {
     const int pr = e / (NH + 1), k = e % (NH + 1);
     const int km = (N - k) % N;
     const C Zk = seq[pr * RP + k + (k >> 3)];
@@ -440,13 +440,14 @@ struct XP {
   // warps busy in the inverse stages but one CTA per SM, measured slower)
   static constexpr int ROWS = (N == 256) ? 2 : 1;
   static constexpr int SP = N + N / 16;            // padded sequence (one slot per 16)
-  static constexpr int NT = 192;
+  static constexpr int NP = 5;                     // products (u_2^2 subtracted from the squares)
+  static constexpr int NT = 32 * NP;               // one warp (half-warp per row at N = 256) per product
   // resident CTAs per SM the register budget is built for
   static constexpr int MINB = 2;
   // staged row of one field: NH + 1 values rounded up to 16 bytes (the bulk-copy unit)
   static constexpr int RS = (int)(((NH + 1) * sizeof(C) + 15) / 16 * 16 / sizeof(C));
   static constexpr int ROWIN = 6 * RS;
-  static constexpr int STG = (ROWIN > 3 * SP ? ROWIN : 3 * SP);
+  static constexpr int STG = (ROWIN > 2 * SP ? ROWIN : 2 * SP);
   static constexpr uint32_t kRowBytes = RS * sizeof(C);
   static constexpr size_t smem = (size_t)(2 * ROWS * STG + ROWS * 6 * SP + N) * sizeof(C) + 128 +
                                  2 * sizeof(uint64_t);
@@ -479,7 +480,7 @@ __device__ __forceinline__ C shfl2_xor(C v, int m) {
 }
 
 template <int N, class C>
-__global__ void __launch_bounds__(192, XP<N, C>::MINB)
+__global__ void __launch_bounds__(XP<N, C>::NT, XP<N, C>::MINB)
 k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase,
          double scale, int nyq_scalar, double* __restrict__ nyq_part, const C* __restrict__ tw2_g, Geom g,
          int* err) {
@@ -487,14 +488,14 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
   constexpr int M = X::M, NH = X::NH, ROWS = X::ROWS, SP = X::SP, STG = X::STG, RS = X::RS;
   extern __shared__ unsigned char smraw[];
   __shared__ int s_fail;
-  __shared__ double s_nyq[2][12];
+  __shared__ double s_nyq[2][2 * X::NP];
   const uint32_t pad = (128u - (smem_u32(smraw) & 127u)) & 127u;
   C* stg = reinterpret_cast<C*>(smraw + pad);  // [2][ROWS][STG]
   C* W = stg + 2 * ROWS * STG;                       // [ROWS][6][SP]
   C* tw2 = W + ROWS * 6 * SP;                        // [M][16]: W_N^(r*j)
   uint64_t* bars = reinterpret_cast<uint64_t*>(tw2 + N);
   const int tid = threadIdx.x;
-  for (int t = tid; t < N; t += 192) tw2[t] = tw2_g[t];
+  for (int t = tid; t < N; t += X::NT) tw2[t] = tw2_g[t];
   if (tid == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
@@ -615,25 +616,25 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
     // ---- forward stages, per row group; the warp (half-warp for N = 256) of product ab
     // runs both stages of its FFT.  Product ab lands in work region ab (ab < 3, free since
     // the inverse stage B) or in the consumed staging rows (ab >= 3).
-    constexpr int FWD_ROWS = X::NT / (6 * M);  // rows one pass of the CTA covers
+    constexpr int FWD_ROWS = X::NT / (X::NP * M);  // rows one pass of the CTA covers
     static_assert(X::PAIR ? FWD_ROWS == 1 : FWD_ROWS == ROWS, "one forward pass per row group");
     auto prod = [&](int r, int ab) { return ab < 3 ? W + (r * 6 + ab) * SP : S + r * STG + (ab - 3) * SP; };
 #pragma unroll 1
     for (int r0 = 0; r0 < ROWS; r0 += FWD_ROWS) {
       {
         // forward stage A: products fused into the loads
-        const int t = tid % M, ab = (tid / M) % 6, r = r0 + tid / (6 * M);
-        // pairs 00 01 02 11 12 22
-        const int ca = (ab >= 3) + (ab >= 5), cb = ab < 3 ? ab : (ab < 5 ? ab - 2 : 2);
+        const int t = tid % M, ab = (tid / M) % X::NP, r = r0 + tid / (X::NP * M);
+        // 00 - 22, 01, 02, 11 - 22, 12
+        const bool sq = ab == 0 || ab == 3;
+        const int ca = ab >= 3 ? 1 : 0, cb = (sq || ab == 4) ? 2 : ab;
         const C* Za = W + (r * 6 + 3 + ca) * SP;
         const C* Zb = W + (r * 6 + 3 + cb) * SP;
         C v[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           const int x = SNS_IDX(pp16(t + M * q), SP);
-          const C za = Za[x];
-          const C zb = ca == cb ? za : Zb[x];  // squares 00, 11, 22: one load
-          v[q] = cmk(za.x * zb.x, za.y * zb.y);
+          const C za = Za[x], zb = Zb[x];
+          v[q] = sq ? diff_squares(za, zb) : cmk(za.x * zb.x, za.y * zb.y);
         }
         dft16<-1>(v);
         C* Wp = prod(r, ab);
@@ -685,7 +686,7 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
           }
         }
       } else {
-        const int j = tid & 15, sq = tid >> 4, r = sq / 6, ab = sq % 6;
+        const int j = tid & 15, sq = tid >> 4, r = sq / X::NP, ab = sq % X::NP;
         const C* Wp = prod(r, ab);
         C v[16];
 #pragma unroll
@@ -727,13 +728,13 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
       nyq_part[(2 * ab + 1) * gridDim.x + blockIdx.x] = nyq_ps;
     }
   } else {
-    const int j = tid & 15, sq = tid >> 4, r = sq / 6, ab = sq % 6;
+    const int j = tid & 15, sq = tid >> 4, r = sq / X::NP, ab = sq % X::NP;
     if (j == 0) {
       s_nyq[r][2 * ab] = nyq_p0;
       s_nyq[r][2 * ab + 1] = nyq_ps;
     }
     __syncthreads();
-    if (tid < 12) nyq_part[tid * gridDim.x + blockIdx.x] = s_nyq[0][tid] + s_nyq[1][tid];
+    if (tid < 2 * X::NP) nyq_part[tid * gridDim.x + blockIdx.x] = s_nyq[0][tid] + s_nyq[1][tid];
   }
 }
 
@@ -758,7 +759,7 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
 //                    W_N^(j k1) / 2 (the r2c unpack's factor 1/2, exact); out to P[ab][j][k1]
 //   forward stage B  lane k1: the 16-point DFT over j, outputs k1 + M k2; r2c unpack of the
 //                    two grids through the partner lane (N - k), 128-byte stores to HBM
-// The products run in two halves of three (00 01 02, then 11 12 22), each through Wc and its
+// The products run in two parts (00 - 22, 01, 02, then 11 - 22, 12), each through Wc and its
 // forward stage B, so a warp holds one staged row group and one transposition buffer.  Every
 // transposition goes through shared memory once, XOR-swizzled (no bank conflicts); the
 // products never do.  The kernel is bound by instruction issue, so its complex additions run
@@ -777,7 +778,7 @@ struct XW {
   static constexpr uint32_t kRowBytes = RS * sizeof(C);
   static constexpr int TWT = 16 * 32;     // four-step twiddles [i][lane], then the same halved
   static constexpr size_t smem = (size_t)(WARPS * PER_WARP + 2 * TWT) * sizeof(C) + 128 +
-                                 WARPS * (sizeof(uint64_t) + R * 12 * sizeof(double));
+                                 WARPS * (sizeof(uint64_t) + R * 10 * sizeof(double));
   static_assert(R * M == 32, "a warp covers its rows' lanes");
 };
 
@@ -804,8 +805,8 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
   C* const twh = twt + X::TWT;                   // [16][32], times 1/2
   uint64_t* const bar = reinterpret_cast<uint64_t*>(twh + X::TWT) + warp;
   double* const s_nyq = reinterpret_cast<double*>(reinterpret_cast<uint64_t*>(twh + X::TWT) + X::WARPS);
-  double* const my_nyq = s_nyq + warp * R * 12;  // [WARPS][R][12]
-  for (int e = lane; e < R * 12; e += 32) my_nyq[e] = 0.0;
+  double* const my_nyq = s_nyq + warp * R * 10;  // [WARPS][R][10]
+  for (int e = lane; e < R * 10; e += 32) my_nyq[e] = 0.0;
   if (lane == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -987,17 +988,22 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
 
 #pragma unroll
     for (int half = 0; half < (DIAG ? 0 : 2); ++half) {
+      const int ab0 = 3 * half, ab1 = half ? 5 : 3;
       // ---- products and forward stage A: P[ab % 3][j][k1] in Wc at pslot(j, k1, row)
 #pragma unroll
       for (int p = 0; p < MP; ++p) {
         const int rB = row_b(p);
 #pragma unroll
-        for (int ab = 3 * half; ab < 3 * half + 3; ++ab) {
-          // pairs 00 01 02 11 12 22
-          const int ca = (ab >= 3) + (ab >= 5), cb = ab < 3 ? ab : (ab < 5 ? ab - 2 : 2);
+        for (int ab = ab0; ab < ab1; ++ab) {
+          // 00 - 22, 01, 02, 11 - 22, 12
+          const bool sq = ab == 0 || ab == 3;
+          const int ca = ab >= 3 ? 1 : 0, cb = (sq || ab == 4) ? 2 : ab;
           C v[NZ];
 #pragma unroll
-          for (int q = 0; q < NZ; ++q) v[q] = pmul(z[p][ca][q], z[p][cb][q]);
+          for (int q = 0; q < NZ; ++q) {
+            const C za = z[p][ca][q], zb = z[p][cb][q];
+            v[q] = sq ? pmul(psub(za, zb), padd(za, zb)) : pmul(za, zb);
+          }
           if constexpr (N == 512) {
             // M = 32 split in frequency: h = 0 takes p(n) + p(n + 16) (even k1), h = 1 takes
             // (p(n) - p(n + 16)) W32^n (odd k1)
@@ -1028,7 +1034,7 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
         const int partner = (N == 512) ? ((32 - lane) & 31) : ((lane & ~(M - 1)) + ((M - k1) & (M - 1)));
         const long long row = it * R + r;
 #pragma unroll 1
-        for (int ab = 3 * half; ab < 3 * half + 3; ++ab) {
+        for (int ab = ab0; ab < ab1; ++ab) {
           const C* Pab = Wc + ((ab % 3) * R + r) * N;
           C v[16];
 #pragma unroll
@@ -1049,8 +1055,8 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
               o0[SNS_IDX(kk, g.pitch)] = A;
               o1[SNS_IDX(kk, g.pitch)] = B;
               if (kk == NH) {
-                my_nyq[r * 12 + 2 * ab] += A.x;
-                my_nyq[r * 12 + 2 * ab + 1] += B.x;
+                my_nyq[r * 10 + 2 * ab] += A.x;
+                my_nyq[r * 10 + 2 * ab + 1] += B.x;
               }
             }
           }
@@ -1086,17 +1092,17 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
   }
   // per-CTA Nyquist partials, fixed order: [field][cta]
   __syncthreads();
-  if (tid < 12) {
+  if (tid < 10) {
     double s = 0.0;
 #pragma unroll 1
-    for (int w = 0; w < X::WARPS * R; ++w) s += s_nyq[w * 12 + tid];
+    for (int w = 0; w < X::WARPS * R; ++w) s += s_nyq[w * 10 + tid];
     nyq_part[tid * gridDim.x + blockIdx.x] = s;
   }
 }
 
-// Nyquist-plane sums: column N/2 of each of the 12 product fields summed over all rows
+// Nyquist-plane sums: column N/2 of each product field summed over all rows
 // (the (N/2,0,0) output of the y/z forward transforms is the plain sum of the plane).
-// grid 12, fixed summation order.
+// grid: the fields, fixed summation order.
 template <class C>
 __global__ void __launch_bounds__(256) k_nyq_reduce(const C* __restrict__ work, double* __restrict__ sums,
                                                     Geom g) {
@@ -1117,10 +1123,10 @@ __global__ void __launch_bounds__(256) k_nyq_reduce(const C* __restrict__ work, 
 // ------------------------------------------------------------------------------------
 // P5 sweep: per mode, the reference's accumulate (:926-936), add_viscous_project
 // (:955-974), RK stage update (:994-1033) and project_truncate (:825-844).
-template <class C>
+template <class C, int NP>
 struct ModeIn {
-  C p0[6];
-  C ps[6];
+  C p0[NP];
+  C ps[NP];
 };
 
 template <class C>
@@ -1201,8 +1207,8 @@ __device__ __forceinline__ SweepArgs resolve_step(SweepArgs a) {
   return a;
 }
 
-template <class C>
-__device__ __forceinline__ void sweep_mode(const ModeIn<C>& in, int ix, int iy, int iz, int n, C phase,
+template <class C, int NP>
+__device__ __forceinline__ void sweep_mode(const ModeIn<C, NP>& in, int ix, int iy, int iz, int n, C phase,
                                            C uu[3], C gg[3], bool load_g, C rr[3],
                                            const SweepArgs& a, CompWord lo[3]) {
   const int m2 = ix * ix + iy * iy + iz * iz;
@@ -1212,7 +1218,7 @@ __device__ __forceinline__ void sweep_mode(const ModeIn<C>& in, int ix, int iy, 
   const int pa[6] = {0, 0, 0, 1, 1, 2};
   const int pb[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
-  for (int p = 0; p < 6; ++p) {
+  for (int p = 0; p < NP; ++p) {
     const C value = pair_value(in.p0[p], in.ps[p], phase, keep, a.dealias);
     r[pa[p]] = cadd(r[pa[p]], minus_i_k(value, kv[pb[p]]));
     if (pa[p] != pb[p]) r[pb[p]] = cadd(r[pb[p]], minus_i_k(value, kv[pa[p]]));
@@ -1313,7 +1319,7 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
   }
 }
 
-template <int N, class C>
+template <int N, class C, int NP>
 __global__ void __launch_bounds__(256)
 k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
         C* __restrict__ rhs, const double* __restrict__ nyq_part, int nparts, const C* __restrict__ phase,
@@ -1329,9 +1335,9 @@ k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
     const int my = signed_mode((int)(row % N), N);
     const int mz = signed_mode((int)(row / N), N);
     const long long idx = row * g.pitch + mx;
-    ModeIn<C> in;
+    ModeIn<C, NP> in;
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
+    for (int p = 0; p < NP; ++p) {
       in.p0[p] = work[(long long)(2 * p) * g.field + idx];
       in.ps[p] = work[(long long)(2 * p + 1) * g.field + idx];
     }
@@ -1375,9 +1381,9 @@ k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
   if (blockIdx.x == 0 && threadIdx.x < 32) {
     // the self-conjugate Nyquist mode (N/2, 0, 0), column nh of row (0, 0): warp 0 sums
     // the per-CTA plane sums (lane-strided, then a fixed shuffle tree: deterministic)
-    double part[12];
+    double part[2 * NP];
 #pragma unroll
-    for (int f = 0; f < 12; ++f) {
+    for (int f = 0; f < 2 * NP; ++f) {
       double acc = 0.0;
       for (int i = threadIdx.x; i < nparts; i += 32) acc += nyq_part[f * nparts + i];
 #pragma unroll
@@ -1385,9 +1391,9 @@ k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
       part[f] = acc;
     }
   if (threadIdx.x == 0) {
-    ModeIn<C> in;
+    ModeIn<C, NP> in;
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
+    for (int p = 0; p < NP; ++p) {
       in.p0[p] = cmk((real_of<C>)part[2 * p], real_of<C>(0));
       in.ps[p] = cmk((real_of<C>)part[2 * p + 1], real_of<C>(0));
     }
@@ -1429,9 +1435,9 @@ __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restric
   constexpr int NH = N / 2;
   const int tid = threadIdx.x;
   const bool load_g = a.stage > 0;
-  double part[12];
+  double part[10];
 #pragma unroll
-  for (int f = 0; f < 12; ++f) {
+  for (int f = 0; f < 10; ++f) {
     double acc = 0.0;
     for (int i = tid; i < nparts; i += 32) acc += nyq_part[f * nparts + i];
 #pragma unroll
@@ -1439,9 +1445,9 @@ __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restric
     part[f] = acc;
   }
   if (tid != 0) return;
-  ModeIn<C> in;
+  ModeIn<C, 5> in;
 #pragma unroll
-  for (int p = 0; p < 6; ++p) {
+  for (int p = 0; p < 5; ++p) {
     in.p0[p] = cmk((real_of<C>)part[2 * p], real_of<C>(0));
     in.ps[p] = cmk((real_of<C>)part[2 * p + 1], real_of<C>(0));
   }
@@ -1630,15 +1636,15 @@ k_sweep_rot(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
 }
 
 // ------------------------------------------------------------------------------------
-// P5 fused (N = 128, 256, 512): forward z pass of the 12 product fields and the whole
+// P5 fused (N = 128, 256, 512): forward z pass of the 10 product fields and the whole
 // k-space sweep in one persistent kernel, so the transformed products never return to HBM.
-// A tile is (TW columns mx, one my, all mz); its 12 field tiles arrive one after another
+// A tile is (TW columns mx, one my, all mz); its 10 field tiles arrive one after another
 // through TMA (double-buffered).  The z FFT leaves each thread 8 modes in registers:
 //   P0 field of pair p -> parked in tensor memory;
 //   Ps field of pair p -> combined with the parked P0 into the dealiased value, whose -i k
 //                          contributions accumulate into r_x, r_y, r_z in tensor memory, in
-//                          the reference's order (pairs 00 01 02 11 12 22);
-//   after the 12th      -> viscous term, Leray projection, RK3 update and projection of u.
+//                          the reference's order (pairs 00 01 02 11 12, the squares less u_2^2);
+//   after the 10th      -> viscous term, Leray projection, RK3 update and projection of u.
 // Tensor memory per thread: 4 blocks of CW columns (P0, r_x, r_y, r_z).
 template <int N>
 constexpr uint32_t p5_cols() { return N == 512 ? 512u : (N == 256 ? 256u : 128u); }
@@ -1663,6 +1669,7 @@ k_p5(const __grid_constant__ CUtensorMap map, C* __restrict__ u, C* __restrict__
   constexpr int WPC = tmem_words<C>();  // tensor-memory words per complex value
   constexpr int MPT = RO::KB * RO::R;    // modes per thread
   constexpr int CW = WPC * MPT;          // tensor-memory words per field of modes
+  constexpr int kF = 10;                 // product fields: 5 products on two grids
   static_assert(RO::R == 4 || RO::R == 8, "last radix moves through tensor memory");
   static_assert((NT / 32 + 3) / 4 * 4 * CW <= (int)COLS, "tensor memory budget");
   static_assert((TW * (N / RO::R)) % NT == 0, "every thread owns whole butterflies");
@@ -1702,10 +1709,10 @@ k_p5(const __grid_constant__ CUtensorMap map, C* __restrict__ u, C* __restrict__
     cb = idx - my * ncb;
   };
   const long long mytiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const long long nunits = 12 * mytiles;
+  const long long nunits = kF * mytiles;
   auto issue = [&](long long ul, int b) {
-    const long long t = blockIdx.x + (ul / 12) * gridDim.x;
-    const int f = (int)(ul % 12);
+    const long long t = blockIdx.x + (ul / kF) * gridDim.x;
+    const int f = (int)(ul % kF);
     int cb, my;
     tile_of(t, cb, my);
     C* dst = b ? in1 : in0;
@@ -1732,8 +1739,8 @@ k_p5(const __grid_constant__ CUtensorMap map, C* __restrict__ u, C* __restrict__
     }
     (void)mbar_try_wait(&bars[b], parity);
     const C* IN = b ? in1 : in0;
-    const long long t = blockIdx.x + (ul / 12) * gridDim.x;
-    const int f = (int)(ul % 12);
+    const long long t = blockIdx.x + (ul / kF) * gridDim.x;
+    const int f = (int)(ul % kF);
     int cb, my;
     tile_of(t, cb, my);
     const int mx0 = cb * TW;
@@ -1795,7 +1802,7 @@ k_p5(const __grid_constant__ CUtensorMap map, C* __restrict__ u, C* __restrict__
       const int j = (tid + (q / RO::R) * NT) / TW, r = q % RO::R;
       return (j / RO::NS) * RO::NS * RO::R + (j % RO::NS) + r * RO::NS;
     };
-    if (f == 11) {
+    if (f == kF - 1) {
       // Two-deep software pipeline over this thread's modes: the u, g loads of mode q + 1
       // are in flight while mode q is combined and stored (different modes, no aliasing).
       C uu_n[3], gg_n[3];
@@ -2239,19 +2246,20 @@ struct Launch {
       k_zpass<N, +1, C><<<grid, nt_yz<N>(), yz_smem(), st>>>(F(src), F(dst), scale, F(tw), g);
     }
   }
-  static void xpass_products(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar,
-                             double* partials, const void* tw, Geom g, cudaStream_t st) {
-    k_xpass_products<N, C><<<N * N, nt_x<N>(), x_smem(6), st>>>(F(work), F(unyq), F(phase), scale, nyq_scalar,
-                                                                  partials, F(tw), g);
+  static void xpass_products(void* work, int np, const void* unyq, const void* phase, double scale, int nyq_scalar,
+                             const void* tw, Geom g, cudaStream_t st) {
+    auto k = np == 6 ? k_xpass_products<N, C, 6> : k_xpass_products<N, C, 5>;
+    k<<<N * N, nt_x<N>(), x_smem(np), st>>>(F(work), F(unyq), F(phase), scale, nyq_scalar, F(tw), g);
   }
-  static void nyq_reduce(const void* work, double* sums, Geom g, cudaStream_t st) {
-    k_nyq_reduce<C><<<12, 256, 0, st>>>(F(work), sums, g);
+  static void nyq_reduce(const void* work, int nf, double* sums, Geom g, cudaStream_t st) {
+    k_nyq_reduce<C><<<nf, 256, 0, st>>>(F(work), sums, g);
   }
-  static void sweep(const void* work, void* u, void* gbuf, void* rhs, const double* nyq_part, int nparts,
+  static void sweep(const void* work, int np, void* u, void* gbuf, void* rhs, const double* nyq_part, int nparts,
                     const void* phase, SweepArgs a, Geom g, cudaStream_t st) {
     const long long total = (long long)N * N * (N / 2);
-    k_sweep<N, C><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(F(work), F(u), F(gbuf), F(rhs), nyq_part, nparts,
-                                                                   F(phase), a, g);
+    auto k = np == 6 ? k_sweep<N, C, 6> : k_sweep<N, C, 5>;
+    k<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(F(work), F(u), F(gbuf), F(rhs), nyq_part, nparts, F(phase), a,
+                                                       g);
   }
   static void xpass2(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar, double* nyq_part,
                      const void* tw2, Geom g, int grid, int* err, cudaStream_t st) {
@@ -2407,7 +2415,8 @@ struct Launch {
     set_smem(k_ypass<N, +1, C>, yz_smem());
     set_smem(k_zpass<N, -1, C>, yz_smem());
     set_smem(k_zpass<N, +1, C>, yz_smem());
-    set_smem(k_xpass_products<N, C>, x_smem(6));
+    set_smem(k_xpass_products<N, C, 6>, x_smem(6));
+    set_smem(k_xpass_products<N, C, 5>, x_smem(5));
     set_smem(k_xpass_r2c<N, C>, x_smem(1));
     set_smem(k_xpass_c2r<N, C>, x_smem(1));
     set_smem(k_xpass_diag<N, C>, x_smem(2));

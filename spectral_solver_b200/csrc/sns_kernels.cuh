@@ -86,14 +86,15 @@ struct Ops {
   // z pass src -> dst (may alias), optional scale applied on load
   void (*zpass)(const void* src, void* dst, int nf, int dir, int ntiles, double scale, const void* tw, Geom g,
                 cudaStream_t st);
-  // fused x pass: 6 inverse fields -> 12 product half-spectra; optional energy/vmax partials
-  void (*xpass_products)(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar,
-                         double* partials, const void* tw, Geom g, cudaStream_t st);
-  // Nyquist-plane sums of the 12 product fields (column nh, summed over rows)
-  void (*nyq_reduce)(const void* work, double* sums, Geom g, cudaStream_t st);
+  // fused x pass: 6 inverse fields -> 2 np product half-spectra (np = 5: the projected
+  // right-hand side's products, 6: all of u_a u_b)
+  void (*xpass_products)(void* work, int np, const void* unyq, const void* phase, double scale, int nyq_scalar,
+                         const void* tw, Geom g, cudaStream_t st);
+  // Nyquist-plane sums of the first nf product fields (column nh, summed over rows)
+  void (*nyq_reduce)(const void* work, int nf, double* sums, Geom g, cudaStream_t st);
   // fused k-space sweep; rhs may be null in RK mode; the (N/2,0,0) product values are the
   // fixed-order sums of nparts partials per field ([field][nparts])
-  void (*sweep)(const void* work, void* u, void* gbuf, void* rhs, const double* nyq_part, int nparts,
+  void (*sweep)(const void* work, int np, void* u, void* gbuf, void* rhs, const double* nyq_part, int nparts,
                 const void* phase, SweepArgs a, Geom g, cudaStream_t st);
   // generic real rows (doubles) -> half rows (x r2c), nf fields of real data with row pitch n
   void (*xpass_r2c)(const double* in, void* out, int nf, const void* tw, Geom g, cudaStream_t st);
@@ -106,7 +107,7 @@ struct Ops {
   void (*yz_tma)(const CUtensorMap& map, int axis, int dir, int variant, TmaArgs a, const void* tw,
                  const void* phase, Geom g, int grid, cudaStream_t st);
   int (*tma_blocks_per_sm)();
-  // two-stage persistent x pass (N = 256, 512); writes [12][grid] Nyquist partials
+  // two-stage persistent x pass (N = 256, 512), 5 products; writes [10][grid] Nyquist partials
   void (*xpass2)(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar, double* nyq_part,
                  const void* tw2, Geom g, int grid, int* err, cudaStream_t st);
   int (*xpass2_grid)(int nsm);
