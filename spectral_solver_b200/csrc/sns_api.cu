@@ -9,12 +9,14 @@
 //   tables: twiddles (N), phase exp(i*pi*(mx+my+mz)/N) for mx+my+mz in [-3N/2, 3N/2],
 //           reduction partials, the 12 Nyquist-plane sums.
 #include "sns_kernels.cuh"
+#include "sns_small.cuh"
 #include "../../include/sns_b200.h"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -74,6 +76,9 @@ struct sns_handle {
   int viscous_mode = 0;
   sns::Geom g{};
   const sns::Ops* ops = nullptr;
+  const sns::SmallOps* small = nullptr;  // the four-launch stage of small grids (small_rule)
+  // small path: the work fields already hold the inverse z (z and y) transform of u
+  bool z_ready = false, y_ready = false;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int cbytes = 16;          // bytes per complex value: 16 (FP64) or 8 (FP32)
@@ -132,6 +137,12 @@ struct sns_handle {
 };
 
 namespace {
+
+// Grids whose stage runs on the kernels of sns_small.cu.  At 128^3 they take 0.55 ms a step
+// (FP32; 0.60 on the streaming passes) and 1.00 ms (FP64; 1.30), at 96^3 0.28 (0.44) and 0.45
+// (0.75), at 64^3 0.12 (0.21) and 0.15 (0.30); at 256^3 a z tile of the ten product fields
+// takes a whole SM's shared memory.
+bool small_rule(int n) { return n <= 128; }
 
 int complex_bytes(int precision) { return precision == SNS_PRECISION_FP32 ? 8 : 16; }
 size_t field_bytes(int n, int precision) {
@@ -389,6 +400,40 @@ void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt
   mark(pm, 7, st);
 }
 
+// Is u known to be zero outside the sphere when this stage runs?  Stages 1 and 2 rely on stage
+// 0's sweep, stage 0 on the handle's flag, and never inside a graph capture, where the graph
+// may later be replayed on a new state.
+bool sphere_known(const sns_handle* h, int stage) {
+  return h->prune && (stage > 0 || (h->sphere_clean && !capturing(h->stream)));
+}
+
+// The same stage on a small grid: the inverse z and y transforms of u (unless the previous
+// kernels left them in the work fields), x, forward y, forward z with the sweep.  Pencils outside the sphere are
+// neither written nor read when u is known to be zero there.
+void run_stage_small(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, int mode, char* rhs_out,
+                     PassMarks* pm) {
+  const sns::SmallOps* o = h->small;
+  cudaStream_t st = h->stream;
+  const int clean = mode == 0 && sphere_known(h, stage) ? 1 : 0;
+  const int emit = mode == 0 && stage < 2 ? 1 : 0;
+  mark(pm, 0, st);
+  if (!h->z_ready) o->zphase(u_src, h->work, h->phase, h->tw, h->inv_size(), clean, h->g, st);
+  mark(pm, 1, st);
+  if (!h->y_ready) o->yinv(h->work, h->tw, 2, clean, h->g, st);
+  mark(pm, 2, st);
+  o->xpass(h->work, u_src, h->phase, h->tw, h->inv_size(), h->nyq_part, 0, h->g, st);
+  mark(pm, 3, st);
+  mark(pm, 4, st);
+  o->yfwd(h->work, h->tw, h->g, st);
+  mark(pm, 5, st);
+  mark(pm, 6, st);
+  h->y_ready = false;
+  o->zsweep(h->work, u_src, g_buf, rhs_out, h->nyq_part, o->nparts, h->phase, h->tw, stage_args(h, stage, dt, mode, u_src), clean,
+            emit, h->inv_size(), h->g, st);
+  mark(pm, 7, st);
+  h->z_ready = emit != 0;
+}
+
 // One RK3 stage (or the RHS only, mode 1; the unprojected nonlinear term, mode 2) on u_src: the
 // five fused passes.  The projected forms run on 5 products (the squares less u_2^2, a
 // gradient's difference that the projection removes), mode 2 on all 6, as separate kernels.
@@ -404,16 +449,18 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   const int tiles_in = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   const int f_src = (int)((size_t)(u_src - h->state) / h->fbytes);  // u (0) or the g slot (3)
   const int np = mode == 2 ? 6 : 5;
+  if (h->small && np == 5 && h->nyq_clean) {
+    run_stage_small(h, u_src, g_buf, stage, dt, mode, rhs_out, pm);
+    return;
+  }
+  h->z_ready = false;
   const bool fused = h->p5_grid > 0 && np == 5;
   // Sphere pruning (RK update with the fused P5 only).  A column-block tile (my, cb) outside
   // the disk 4 ((cb * TW)^2 + my^2) <= N^2 holds only modes outside the sphere: u is zero
-  // there before the stage (every stage's sweep zeroes those modes, so stages 1 and 2 may
-  // rely on stage 0; stage 0 relies on the handle's flag, and never inside a graph capture,
-  // where the graph may later be replayed on a new state) and the stage leaves it zero.  So
-  // P5 neither loads, transforms nor sweeps these tiles (their forward-z inputs are never
-  // needed); every other value is computed as without pruning.
-  const bool prune = h->prune && fused && mode == 0 && h->nyq_clean && h->nlive > 0 &&
-                     (stage > 0 || (h->sphere_clean && !capturing(st)));
+  // there before the stage (sphere_known) and the stage leaves it zero.  So P5 neither loads,
+  // transforms nor sweeps these tiles (their forward-z inputs are never needed); every other
+  // value is computed as without pruning.
+  const bool prune = fused && mode == 0 && h->nyq_clean && h->nlive > 0 && sphere_known(h, stage);
   mark(pm, 0, st);
   o->yz_tma(h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), h->tw, h->phase,
             g, h->tma_grid, st);
@@ -459,14 +506,15 @@ void step_once(sns_handle* h, double dt) {
   }
 }
 
-int velocity_partials(sns_handle* h);
+int velocity_partials(sns_handle* h, bool both = false);
 
 // One step with the adaptive CFL rule on the device: vmax of the current state (the same
 // per-row partials as sns_max_velocity; their max and the clock's next step in one launch),
 // then the three stages on that step.  Nothing here waits for the host, so the step can be
 // captured into a graph.
 void step_on_clock(sns_handle* h) {
-  const int pairs = velocity_partials(h);
+  const int pairs = velocity_partials(h, h->small && h->form == 0 && h->nyq_clean);
+  h->z_ready = h->small && h->form == 0 && h->nyq_clean;  // stage 0 starts from the same transform of u
   sns::launch_clock_step_partials(h->partials + 1, pairs, 2, h->clock, h->stream);
   h->on_clock = true;
   try {
@@ -519,9 +567,17 @@ void download_full(sns_handle* h, const void* src, double* host, const sns::Comp
 // Physical velocity of the state: inverse z and y passes of u without the phase shift, then
 // the diagnostic x pass; (energy, vmax^2) partials in h->partials, per row or per CTA of the
 // warp-per-row kernel; returns how many pairs.
-int velocity_partials(sns_handle* h) {
+int velocity_partials(sns_handle* h, bool both) {
   const sns::Ops* o = h->ops;
   const sns::Geom& g = h->g;
+  if (h->small && h->nyq_clean) {
+    const int clean = sphere_known(h, 0) ? 1 : 0;
+    h->small->zphase(h->u(), h->work, h->phase, h->tw, h->inv_size(), clean, g, h->stream);
+    h->small->yinv(h->work, h->tw, both ? 2 : 1, clean, g, h->stream);
+    h->small->xpass(h->work, h->u(), h->phase, h->tw, h->inv_size(), h->partials, 1, g, h->stream);
+    h->y_ready = both;
+    return h->small->nparts;
+  }
   const int tiles = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   o->yz_tma(h->map_state_z, 2, +1, 0, tma_args(h, 0, 3, tiles, h->work, 0, h->inv_size()), h->tw, h->phase, g,
             h->tma_grid, h->stream);
@@ -778,7 +834,12 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
     h->tma_grid = sns::small_grid_cap(n, nsm * ops->tma_blocks_per_sm());
     h->x2_grid = ops->xpass2_grid(nsm);
     h->p5_grid = ops->p5_grid(nsm);
-    alloc((void**)&h->nyq_part, (size_t)12 * (h->x2_grid > 0 ? h->x2_grid : 1) * sizeof(double));
+    if (small_rule(n)) {
+      h->small = sns::small_for(n, precision);
+      h->small->init();
+    }
+    const int nparts = std::max(std::max(1, h->x2_grid), h->small ? h->small->nparts : 1);
+    alloc((void**)&h->nyq_part, (size_t)12 * nparts * sizeof(double));
     alloc((void**)&h->tw2, (size_t)n * h->cbytes);
     {
       // tw2[r*16 + j] = exp(-2*pi*i*r*j/n) for r < n/16, j < 16
