@@ -88,10 +88,26 @@ struct sns_handle {
   void* tw = nullptr;
   void* phase = nullptr;
   double* partials = nullptr;
-  double* red = nullptr;  // reduction results
-  int* err_word = nullptr;  // device error word written by bounded waits
+  // Mapped pinned words the kernels write and the host reads after a synchronisation, with no
+  // copy: 16 reduction results, then the error word of bounded waits.  *_host: host addresses.
+  double* red = nullptr;
+  int* err_word = nullptr;
+  double* red_host = nullptr;
+  volatile int* err_host() const { return reinterpret_cast<volatile int*>(red_host + 16); }
   double* clock = nullptr;  // device clock of adaptive-CFL stepping (sns::kClock* slots)
-  bool on_clock = false;    // the stages being enqueued take their step from the clock
+  // device words the stages being enqueued take their step from (kClock* slots): the clock,
+  // fixed_step (a fixed step inside a step graph), or null (the step is an argument)
+  const double* step_src = nullptr;
+  // Step graphs (use_graph): one RK3 step at the size held in fixed_step, and one adaptive
+  // step on the clock.  `key` is the launch configuration a graph was captured with.
+  double* fixed_step = nullptr;
+  double fixed_dt = 0.0, fixed_nu = -1.0;  // what fixed_step holds
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<int> key;
+  } graph[2];
+  bool own_capture = false;  // capturing a step graph, replayed on sphere-clean states only
+  int warm_steps = 0;        // steps taken launch by launch
   int tma_grid = 0;         // persistent CTAs of the TMA passes
   int x2_grid = 0;          // persistent CTAs of the two-stage x pass (0: generic x pass)
   int p5_grid = 0;          // persistent CTAs of the fused forward-z + sweep pass (0: two kernels)
@@ -315,10 +331,9 @@ void check_inject(sns_handle* h) {
 void sync(sns_handle* h, const char* what) {
   ck(cudaGetLastError(), what);
   ck(cudaStreamSynchronize(h->stream), what);
-  int e = 0;
-  ck(cudaMemcpy(&e, h->err_word, sizeof(int), cudaMemcpyDeviceToHost), what);
+  const int e = *h->err_host();
   if (e != 0) {
-    cudaMemset(h->err_word, 0, sizeof(int));
+    *h->err_host() = 0;
     throw SnsError(SNS_ERR_CUDA, std::string(what) + ": a pass gave up waiting for its TMA tile (code " +
                                      std::to_string(e) + ")");
   }
@@ -346,7 +361,7 @@ sns::SweepArgs stage_args(const sns_handle* h, int stage, double dt, int mode, c
   // the compensated update applies to the handle's own state only (not to sns_rhs inputs)
   a.ulo = (h->comp && mode == 0 && u_src == h->u()) ? h->ulo : nullptr;
   // adaptive stepping: the step size comes from the device clock
-  a.clock = (h->on_clock && mode == 0) ? h->clock : nullptr;
+  a.clock = mode == 0 ? h->step_src : nullptr;
   a.stage = stage;
   a.mode = mode;
   a.dealias = 1;
@@ -401,10 +416,10 @@ void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt
 }
 
 // Is u known to be zero outside the sphere when this stage runs?  Stages 1 and 2 rely on stage
-// 0's sweep, stage 0 on the handle's flag, and never inside a graph capture, where the graph
-// may later be replayed on a new state.
+// 0's sweep, stage 0 on the handle's flag, and not inside a batch's or server's graph capture,
+// where the graph may later be replayed on a new state.
 bool sphere_known(const sns_handle* h, int stage) {
-  return h->prune && (stage > 0 || (h->sphere_clean && !capturing(h->stream)));
+  return h->prune && (stage > 0 || (h->sphere_clean && (h->own_capture || !capturing(h->stream))));
 }
 
 // The same stage on a small grid: the inverse z and y transforms of u (unless the previous
@@ -516,14 +531,70 @@ void step_on_clock(sns_handle* h) {
   const int pairs = velocity_partials(h, h->small && h->form == 0 && h->nyq_clean);
   h->z_ready = h->small && h->form == 0 && h->nyq_clean;  // stage 0 starts from the same transform of u
   sns::launch_clock_step_partials(h->partials + 1, pairs, 2, h->clock, h->stream);
-  h->on_clock = true;
-  try {
-    step_once(h, 0.0);
-  } catch (...) {
-    h->on_clock = false;
-    throw;
+  h->step_src = h->clock;
+  step_once(h, 0.0);
+  h->step_src = nullptr;
+}
+
+// Steps of a small grid replay a graph: launched one by one its kernels (a few microseconds
+// each on the device) cost about 5 us each of host time, the graph about 8 us in all.  From
+// N = 256 on the device time of a step covers its launches.
+constexpr int kGraphMaxN = 128;
+bool use_graph(const sns_handle* h) {
+  return h->n <= kGraphMaxN && h->nyq_clean && h->sphere_clean && h->warm_steps > 1;
+}
+
+// Capture (once per launch configuration) and replay one step; false when the capture failed,
+// the step then runs launch by launch.
+bool replay_step(sns_handle* h, bool on_clock) {
+  auto& sg = h->graph[on_clock ? 1 : 0];
+  const std::vector<int> key = {h->form, h->prune, h->comp, h->tma_grid, h->x2_grid, h->p5_grid};
+  if (sg.exec == nullptr || sg.key != key) {
+    if (sg.exec) cudaGraphExecDestroy(sg.exec);
+    sg.exec = nullptr;
+    if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    h->own_capture = true;
+    if (on_clock) {
+      step_on_clock(h);
+    } else {
+      h->step_src = h->fixed_step;
+      step_once(h, 0.0);
+      h->step_src = nullptr;
+    }
+    h->own_capture = false;
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&sg.exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      sg.exec = nullptr;
+      return false;
+    }
+    sg.key = key;
   }
-  h->on_clock = false;
+  ck(cudaGraphLaunch(sg.exec, h->stream), "cudaGraphLaunch");
+  return true;
+}
+
+// nsteps fixed steps of size dt, or (on_clock) adaptive steps on the device clock.
+void take_steps(sns_handle* h, double dt, int nsteps, bool on_clock) {
+  for (int s = 0; s < nsteps; ++s) {
+    if (use_graph(h)) {
+      if (!on_clock && (h->fixed_dt != dt || h->fixed_nu != h->nu)) {
+        sns::launch_set_step(h->fixed_step, dt, h->nu, h->stream);
+        h->fixed_dt = dt;
+        h->fixed_nu = h->nu;
+      }
+      if (replay_step(h, on_clock)) continue;
+    }
+    if (on_clock) step_on_clock(h);
+    else step_once(h, dt);
+    h->warm_steps++;
+  }
 }
 
 // Does a reference full-layout spectrum carry content on the plane mx = N/2 off (N/2,0,0)?
@@ -590,8 +661,7 @@ int velocity_partials(sns_handle* h, bool both) {
 // The same reduced: energy sum in h->red[0], vmax^2 in h->red[1].
 void velocity_reductions(sns_handle* h) {
   const int rows = velocity_partials(h);  // (energy, vmax^2) pairs
-  sns::launch_reduce(h->partials, rows, 2, 0, h->red + 0, h->stream);
-  sns::launch_reduce(h->partials + 1, rows, 2, 1, h->red + 1, h->stream);
+  sns::launch_reduce_pairs(h->partials, rows, h->red + 0, h->stream);
 }
 
 // The initial state on the handle's own memory: Taylor-Green at cell centres -> forward
@@ -656,14 +726,16 @@ void release(sns_handle* h) {
   cudaFree(h->tw);
   cudaFree(h->phase);
   cudaFree(h->partials);
-  cudaFree(h->red);
-  cudaFree(h->err_word);
+  if (h->red_host) cudaFreeHost(h->red_host);
   cudaFree(h->clock);
   cudaFree(h->tw2);
   cudaFree(h->nyq_part);
   cudaFree(h->xf);
   cudaFree(h->live);
   cudaFree(h->ulo);
+  cudaFree(h->fixed_step);
+  for (auto& sg : h->graph)
+    if (sg.exec) cudaGraphExecDestroy(sg.exec);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -742,7 +814,7 @@ size_t sns_bytes_required(int n, int precision) {
   if (n <= 0 || (precision != SNS_PRECISION_FP64 && precision != SNS_PRECISION_FP32)) return 0;
   return 18 * field_bytes(n, precision) + comp_bytes(n, precision) + partial_slots(n) * sizeof(double) +
          (size_t)(4 * n + 64) * complex_bytes(precision) + (size_t)n * (n / 16 + 1) * sizeof(int) +
-         sns::kClockWords * sizeof(double);
+         2 * sns::kClockWords * sizeof(double);
 }
 
 int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed, double pert_amp, int pert_kmax,
@@ -824,11 +896,13 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
     alloc((void**)&h->tw, (size_t)n * h->cbytes);
     alloc((void**)&h->phase, (size_t)(3 * n + 1) * h->cbytes);
     alloc((void**)&h->partials, h->partial_count * sizeof(double));
-    alloc((void**)&h->red, 16 * sizeof(double));
-    alloc((void**)&h->err_word, sizeof(int));
+    ck(cudaHostAlloc((void**)&h->red_host, 17 * sizeof(double), cudaHostAllocMapped), "cudaHostAlloc");
+    std::memset(h->red_host, 0, 17 * sizeof(double));
+    ck(cudaHostGetDevicePointer((void**)&h->red, h->red_host, 0), "cudaHostGetDevicePointer");
+    h->err_word = reinterpret_cast<int*>(h->red + 16);
     alloc((void**)&h->clock, sns::kClockWords * sizeof(double));
+    alloc((void**)&h->fixed_step, sns::kClockWords * sizeof(double));
     ck(cudaMemsetAsync(h->clock, 0, sns::kClockWords * sizeof(double), h->stream), "memset");
-    ck(cudaMemsetAsync(h->err_word, 0, sizeof(int), h->stream), "memset");
     int nsm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
     h->tma_grid = sns::small_grid_cap(n, nsm * ops->tma_blocks_per_sm());
@@ -1085,7 +1159,7 @@ int sns_set_clock(sns_handle* h, double t, double t_end, double cfl, double dt_m
 int sns_step_cfl(sns_handle* h, int nsteps) {
   return guarded(h, [&] {
     if (nsteps < 0) throw SnsError(SNS_ERR_INVALID, "negative step count");
-    for (int k = 0; k < nsteps; ++k) step_on_clock(h);
+    take_steps(h, 0.0, nsteps, true);
     sync(h, "sns_step_cfl");
   });
 }
@@ -1105,8 +1179,8 @@ int sns_get_clock(sns_handle* h, double* out, int count) {
 
 int sns_debug_set_error_word(sns_handle* h, int code) {
   return guarded(h, [&] {
-    ck(cudaMemcpyAsync(h->err_word, &code, sizeof(int), cudaMemcpyHostToDevice, h->stream), "error word");
     ck(cudaStreamSynchronize(h->stream), "error word");
+    *h->err_host() = code;
   });
 }
 
@@ -1222,7 +1296,7 @@ int sns_nonlinear(sns_handle* h, const double* const uhat_full[3], double* const
 int sns_step(sns_handle* h, double dt, int nsteps) {
   return guarded(h, [&] {
     if (nsteps < 0 || !std::isfinite(dt)) throw SnsError(SNS_ERR_INVALID, "invalid dt or step count");
-    for (int s = 0; s < nsteps; ++s) step_once(h, dt);
+    take_steps(h, dt, nsteps, false);
     sync(h, "sns_step");
   });
 }
@@ -1231,7 +1305,7 @@ int sns_time_steps(sns_handle* h, double dt, int nsteps, double* elapsed_ms) {
   return guarded(h, [&] {
     if (nsteps < 0 || !std::isfinite(dt) || !elapsed_ms) throw SnsError(SNS_ERR_INVALID, "invalid argument");
     ck(cudaEventRecord(h->ev0, h->stream), "event");
-    for (int s = 0; s < nsteps; ++s) step_once(h, dt);
+    take_steps(h, dt, nsteps, false);
     ck(cudaEventRecord(h->ev1, h->stream), "event");
     sync(h, "sns_time_steps");
     float ms = 0.f;
@@ -1269,10 +1343,8 @@ int sns_max_velocity(sns_handle* h, double* out) {
   return guarded(h, [&] {
     if (!out) throw SnsError(SNS_ERR_INVALID, "null output");
     velocity_reductions(h);
-    double r[2];
-    ck(cudaMemcpyAsync(r, h->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "download");
     sync(h, "sns_max_velocity");
-    *out = std::sqrt(r[1]);
+    *out = std::sqrt(h->red_host[1]);
   });
 }
 
@@ -1282,11 +1354,9 @@ int sns_diagnostics(sns_handle* h, double t, sns_diag* out) {
     velocity_reductions(h);
     const int nb = 1184;  // 8 CTAs per SM on 148 SMs
     sns::launch_spectral_diag(h->u(), h->precision, h->partials + 2 * (size_t)h->n * h->n, nb, h->g, h->stream);
-    sns::launch_reduce(h->partials + 2 * (size_t)h->n * h->n, nb, 2, 0, h->red + 2, h->stream);
-    sns::launch_reduce(h->partials + 2 * (size_t)h->n * h->n + 1, nb, 2, 1, h->red + 3, h->stream);
-    double r[4];
-    ck(cudaMemcpyAsync(r, h->red, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "download");
+    sns::launch_reduce_pairs(h->partials + 2 * (size_t)h->n * h->n, nb, h->red + 2, h->stream);
     sync(h, "sns_diagnostics");
+    const double* r = h->red_host;
     const double n3 = (double)h->n * h->n * h->n;
     out->t = t;
     out->kinetic_energy = r[0] / n3;

@@ -1963,6 +1963,33 @@ __global__ void __launch_bounds__(256) k_spectral_diag(const C* __restrict__ u, 
   }
 }
 
+// Fixed-order sum of the first and maximum of the second of `count` pairs (one CTA): out[0],
+// out[1].  One launch for a diagnostic's two reductions.
+__global__ void __launch_bounds__(1024) k_reduce_pairs(const double2* __restrict__ pairs, int count,
+                                                       double* __restrict__ out) {
+  __shared__ double2 red[1024];
+  const int tid = threadIdx.x;
+  double2 s[4] = {};
+  for (int i0 = tid; i0 < count; i0 += 4 * 1024) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * 1024;
+      if (i < count) s[u] = make_double2(s[u].x + pairs[i].x, fmax(s[u].y, pairs[i].y));
+    }
+  }
+  red[tid] = make_double2((s[0].x + s[1].x) + (s[2].x + s[3].x),
+                          fmax(fmax(s[0].y, s[1].y), fmax(s[2].y, s[3].y)));
+  __syncthreads();
+  for (int o = 512; o > 0; o >>= 1) {
+    if (tid < o) red[tid] = make_double2(red[tid].x + red[tid + o].x, fmax(red[tid].y, red[tid + o].y));
+    __syncthreads();
+  }
+  if (tid == 0) {
+    out[0] = red[0].x;
+    out[1] = red[0].y;
+  }
+}
+
 // Fixed-order reduction of `count` partials at stride `stride` (one CTA).
 // One CTA of 1024 threads; four independent loads in flight per thread (the partials are
 // read once, a few MB at most), then a fixed-order tree: the result does not depend on timing.
@@ -2301,10 +2328,6 @@ __device__ void clock_advance(const double* __restrict__ vmax2, double* __restri
   c[kClockT] = t + dt;
   c[kClockSteps] += 1.0;
 }
-__global__ void k_clock_step(const double* __restrict__ vmax2, double* __restrict__ c) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) clock_advance(vmax2, c);
-}
-
 // The index-check record of the debug build: {count, first line, first index}; count -1 in
 // the normal build, which has no checks.
 int bounds_record(long long* out3) {
@@ -2323,8 +2346,14 @@ int bounds_record(long long* out3) {
   return 0;
 }
 
-void launch_clock_step(const double* vmax2, double* clock, cudaStream_t st) {
-  k_clock_step<<<1, 32, 0, st>>>(vmax2, clock);
+// The words a step graph reads a fixed step from: its size and the viscosity, running.
+__global__ void k_set_step(double* __restrict__ c, double dt, double nu) {
+  c[kClockDt] = dt;
+  c[kClockStopped] = 0.0;
+  c[kClockNu] = nu;
+}
+void launch_set_step(double* words, double dt, double nu, cudaStream_t st) {
+  k_set_step<<<1, 1, 0, st>>>(words, dt, nu);
 }
 
 // The max of the per-row vmax^2 partials (as k_reduce: max is exact in any order) and the
@@ -2352,6 +2381,10 @@ __global__ void __launch_bounds__(1024) k_clock_step_partials(const double* __re
 
 void launch_clock_step_partials(const double* partials, int count, int stride, double* clock, cudaStream_t st) {
   k_clock_step_partials<<<1, 1024, 0, st>>>(partials, count, stride, clock);
+}
+
+void launch_reduce_pairs(const double* pairs, int count, double* out, cudaStream_t st) {
+  k_reduce_pairs<<<1, 1024, 0, st>>>(reinterpret_cast<const double2*>(pairs), count, out);
 }
 
 void launch_reduce(const double* partials, int count, int stride, int op_max, double* out, cudaStream_t st) {

@@ -149,11 +149,13 @@ void launch_half_to_full(const void* half, int precision, double2* full, Geom g,
 void launch_full_to_half(const double2* full, void* half, int precision, int hermitian_part, Geom g,
                          cudaStream_t st, CompWord* lo = nullptr, long long src_pitch = 0);
 void launch_spectral_diag(const void* u, int precision, double* partials, int nblocks, Geom g, cudaStream_t st);
+void launch_reduce_pairs(const double* pairs, int count, double* out, cudaStream_t st);
 void launch_reduce(const double* partials, int count, int stride, int op_max, double* out, cudaStream_t st);
-// The next step of a device clock from vmax^2 (the reference's adaptive rule,
+// A fixed step in the words a step graph reads it from.
+void launch_set_step(double* words, double dt, double nu, cudaStream_t st);
+// The next step of a device clock from the maximum of vmax^2 partials (the reference's adaptive rule,
 // ava_taylor_green_impl.hpp:1363-1368): dt = min(dt_max, cfl dx / vmax), clipped to the
 // horizon; stops the clock at the horizon; advances t and the step count.
-void launch_clock_step(const double* vmax2, double* clock, cudaStream_t st);
 void launch_clock_step_partials(const double* partials, int count, int stride, double* clock, cudaStream_t st);
 // the index-check record of the debug build (count -1 without checks); a cudaError_t or 0
 int bounds_record(long long* out3);
