@@ -306,9 +306,9 @@ int sns_grid_supported(int n);
  * sns_create handle serves the benchmark domain (cubic, L = 2 pi, N from a fixed list) on the
  * half spectrum; this handle serves any shape in the reference's own full complex storage.
  * It holds one complex and one real field (24 bytes per grid point) plus the per-axis
- * twiddles; the solver calls below add their working set (18 complex and 8 real fields) on
- * first use.  Axis lengths factor into radices up to 16, run as register butterflies, and
- * any larger prime, run as a direct DFT of that length (slow for large primes); one CTA's
+ * twiddles; the solver calls below add their working set (18 complex and 3 real fields) on
+ * first use.  Axis lengths factor into radices 2 .. 8, 12 and 16, run as register butterflies,
+ * and any prime above 7, run as a direct DFT of that length (slow for large primes); one CTA's
  * shared memory bounds an axis to 6400 points.  Errors: sns_fft3d_last_error
  * (sns_last_error(NULL) for sns_fft3d_create).  Calls are synchronous on the handle's own
  * stream. */

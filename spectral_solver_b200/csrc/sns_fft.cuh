@@ -239,11 +239,95 @@ __host__ __device__ __forceinline__ void dft16(C* v) {
   }
 }
 
+// 5 and 7 points: the real and imaginary parts of the pairs (v_p + v_{R-p}) and
+// (v_p - v_{R-p}) against cos and sin of 2 pi q p / R.
+template <int R, int DIR, class C>
+__host__ __device__ __forceinline__ void dft_odd(C* v, const real_of<C>* cs, const real_of<C>* sn) {
+  using RT = real_of<C>;
+  constexpr int H = (R - 1) / 2;
+  C a[H], b[H], sum = v[0];
+#pragma unroll
+  for (int p = 1; p <= H; ++p) {
+    a[p - 1] = cadd(v[p], v[R - p]);
+    b[p - 1] = csub(v[p], v[R - p]);
+    sum = cadd(sum, a[p - 1]);
+  }
+  C out[R];
+  out[0] = sum;
+#pragma unroll
+  for (int q = 1; q <= H; ++q) {
+    C re = v[0], im = czero<C>();
+#pragma unroll
+    for (int p = 1; p <= H; ++p) {
+      const int m = (p * q) % R;
+      const RT c = cs[m <= H ? m - 1 : R - m - 1], s = m <= H ? sn[m - 1] : -sn[R - m - 1];
+      re = cmk(re.x + c * a[p - 1].x, re.y + c * a[p - 1].y);
+      im = cmk(im.x + s * b[p - 1].x, im.y + s * b[p - 1].y);
+    }
+    const C t = mul_dir_i<DIR>(im);
+    out[q] = cadd(re, t);
+    out[R - q] = csub(re, t);
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q) v[q] = out[q];
+}
+template <int DIR, class C>
+__host__ __device__ __forceinline__ void dft5(C* v) {
+  using RT = real_of<C>;
+  const RT cs[2] = {RT(0.30901699437494742410), RT(-0.80901699437494742410)};  // cos(2 pi k / 5)
+  const RT sn[2] = {RT(0.95105651629515357212), RT(0.58778525229247312917)};
+  dft_odd<5, DIR>(v, cs, sn);
+}
+template <int DIR, class C>
+__host__ __device__ __forceinline__ void dft7(C* v) {
+  using RT = real_of<C>;
+  const RT cs[3] = {RT(0.62348980185873353053), RT(-0.22252093395631440429), RT(-0.90096886790241912624)};
+  const RT sn[3] = {RT(0.78183148246802980871), RT(0.97492791218182360702), RT(0.43388373911755812048)};
+  dft_odd<7, DIR>(v, cs, sn);
+}
+
+// Good-Thomas 6 = 2 x 3 and 12 = 3 x 4: no twiddles between the factors.
+template <int DIR, class C>
+__host__ __device__ __forceinline__ void dft6(C* v) {
+  C t[2][3];
+#pragma unroll
+  for (int n1 = 0; n1 < 2; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) t[n1][n2] = v[(3 * n1 + 2 * n2) % 6];
+    dft3<DIR>(t[n1]);
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < 3; ++k2) {
+    v[(4 * k2) % 6] = cadd(t[0][k2], t[1][k2]);
+    v[(3 + 4 * k2) % 6] = csub(t[0][k2], t[1][k2]);
+  }
+}
+template <int DIR, class C>
+__host__ __device__ __forceinline__ void dft12(C* v) {
+  C t[3][4];
+#pragma unroll
+  for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) t[n1][n2] = v[(4 * n1 + 3 * n2) % 12];
+    dft4<DIR>(t[n1]);
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < 4; ++k2) {
+    C w[3] = {t[0][k2], t[1][k2], t[2][k2]};
+    dft3<DIR>(w);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) v[(4 * k1 + 9 * k2) % 12] = w[k1];
+  }
+}
 template <int R, int DIR, class C>
 __host__ __device__ __forceinline__ void dftR(C* v) {
   if constexpr (R == 2) dft2<DIR>(v);
   else if constexpr (R == 3) dft3<DIR>(v);
   else if constexpr (R == 4) dft4<DIR>(v);
+  else if constexpr (R == 5) dft5<DIR>(v);
+  else if constexpr (R == 6) dft6<DIR>(v);
+  else if constexpr (R == 7) dft7<DIR>(v);
+  else if constexpr (R == 12) dft12<DIR>(v);
   else if constexpr (R == 8) dft8<DIR>(v);
   else if constexpr (R == 16) dft16<DIR>(v);
   else static_assert(R == 2, "unsupported radix");

@@ -5,14 +5,26 @@
 // project, truncate, product_dealiased, nonlinear_rhs with or without the phase-shift pair,
 // rhs, step_rk3, the diagnostics and the vorticity slice of write_vorticity_ppm).
 //
-// The fused pass kernels (sns_kernels.cu) serve the reference's benchmark domain: cubic,
-// L = 2 pi, N in a fixed list, half spectrum.  This file serves everything else, in the
-// reference's own storage: full complex fields [nz][ny][nx] of double2, x fastest.  One
-// kernel transforms along any axis with a mixed-radix Stockham FFT whose radices are a
-// runtime plan (8, 4, 2, 3, 5, 7 and any other prime as a direct DFT of that length):
-// a CTA loads a tile of TW sequences into shared memory (TW consecutive x columns for the
-// y and z axes, so every global access is a coalesced row segment; TW whole rows for x),
-// runs the stages between two shared buffers, and writes the tile back.
+// The fused pass kernels (sns_kernels.cu, sns_small.cu) serve the reference's benchmark
+// domain: cubic, L = 2 pi, N in a fixed list, half spectrum.  This file serves everything
+// else, in the reference's own storage: full complex fields [nz][ny][nx] of double2, x
+// fastest.  One kernel transforms along any axis with a mixed-radix Stockham FFT whose radices
+// are a runtime plan (register butterflies of 2 .. 8, 12 and 16; any other prime as a direct
+// DFT of that length): a CTA takes TW sequences (TW consecutive x columns for the y and z
+// axes, so every global access is a coalesced row segment; TW whole rows for x); the first
+// stage reads global memory, the last one writes it, the stages between meet in shared memory.
+//
+// The solver's transforms are packed two real fields to a complex one.  The reference keeps
+// the real part of every inverse transform, and Re(IDFT(c)) = IDFT(H(c)) with H(c)_m =
+// (c_m + conj(c_-m)) / 2, for any c.  So the first inverse pass reads Z = H(U) + i H(V) from
+// the spectrum (U, V: the plain and the shifted grid of one component, or two components when
+// there is no shifted grid), the x passes work on u + i v, the forward passes read products
+// formed on the fly, and the finishing kernel takes both spectra apart through the mirror
+// mode.  A stage is 3 inverse and 5 forward complex transforms (2 and 3 without the shifted
+// grid) in seven launches; one transform per real field, with a table lookup per DFT
+// term, took 18 and 75 launches.  Six steps at 96 x 80 x 60, host copies included, take 10.8 ms
+// instead of 56.2.
+#include "sns_fft.cuh"
 #include "sns_kernels.cuh"
 #include "../../include/sns_b200.h"
 
@@ -29,8 +41,7 @@
 namespace {
 
 constexpr int kMaxFactors = 24;
-constexpr int kNT = 256;                    // threads per CTA of the axis kernel
-constexpr int kMaxRegRadix = 16;            // radices up to this run from registers
+constexpr int kNT = 256;                    // most threads per CTA of the axis kernel
 constexpr size_t kSmemBudget = 200 * 1024;  // two tile buffers of L x TW complex doubles
 
 struct AxisPlan {
@@ -44,141 +55,8 @@ struct Dims {
   int nx, ny, nz;
 };
 
-// Element e of sequence s of tile t, as a flat index of the [nz][ny][nx] array; -1 when the
-// sequence lies past the array's edge (partial last tile).
-__device__ __forceinline__ long long axis_index(int axis, Dims d, int tw, long long t, int s, int e) {
-  if (axis == 0) {
-    const long long row = t * tw + s;
-    if (row >= (long long)d.ny * d.nz) return -1;
-    return row * d.nx + e;
-  }
-  const int xt = (d.nx + tw - 1) / tw;  // tiles across x
-  const int x = (int)(t % xt) * tw + s;
-  if (x >= d.nx) return -1;
-  const long long other = t / xt;  // iz (axis 1) or iy (axis 2)
-  if (axis == 1) return (other * d.ny + e) * d.nx + x;
-  return ((long long)e * d.ny + other) * d.nx + x;
-}
-
-// One Stockham stage of radix r on all TW sequences: src -> dst (element e of sequence s
-// at e * TW + s).  Butterfly j reads src[j + p L/r], p < r, and writes
-// dst[(j / Ns) Ns r + j % Ns + q Ns] = sum_p src[j + p L/r] W_L^(p (k L/(Ns r) + q L/r)),
-// k = j % Ns, W_L = exp(DIR 2 pi i / L): the stage twiddle and the radix-r DFT in one table
-// lookup per term.
-template <int DIR>
-__device__ void generic_stage(const double2* __restrict__ src, double2* __restrict__ dst, int L, int tw, int r,
-                              int Ns, const double2* __restrict__ twl) {
-  const int m = L / r;
-  const int stride = L / (Ns * r);
-  const int total = tw * m;
-  for (int b = threadIdx.x; b < total; b += blockDim.x) {
-    const int s = b % tw, j = b / tw;
-    const int k = j % Ns;
-    const int base = (j / Ns) * Ns * r + k;
-    if (r <= kMaxRegRadix) {
-      double2 x[kMaxRegRadix];
-#pragma unroll
-      for (int p = 0; p < kMaxRegRadix; ++p)
-        if (p < r) x[p] = src[(j + p * m) * tw + s];
-      for (int q = 0; q < r; ++q) {
-        const int a = k * stride + q * m;  // exponent step of this output (< L)
-        double re = 0.0, im = 0.0;
-        int e = 0;
-#pragma unroll
-        for (int p = 0; p < kMaxRegRadix; ++p) {
-          if (p < r) {
-            double2 w = __ldg(&twl[e]);
-            if (DIR > 0) w.y = -w.y;
-            re += x[p].x * w.x - x[p].y * w.y;
-            im += x[p].x * w.y + x[p].y * w.x;
-            e += a;
-            if (e >= L) e -= L;
-          }
-        }
-        dst[(base + q * Ns) * tw + s] = make_double2(re, im);
-      }
-    } else {
-      for (int q = 0; q < r; ++q) {
-        const int a = k * stride + q * m;
-        double re = 0.0, im = 0.0;
-        int e = 0;
-        for (int p = 0; p < r; ++p) {
-          const double2 v = src[(j + p * m) * tw + s];
-          double2 w = __ldg(&twl[e]);
-          if (DIR > 0) w.y = -w.y;
-          re += v.x * w.x - v.y * w.y;
-          im += v.x * w.y + v.y * w.x;
-          e += a;
-          if (e >= L) e -= L;
-        }
-        dst[(base + q * Ns) * tw + s] = make_double2(re, im);
-      }
-    }
-  }
-}
-
-// Transform every sequence along `axis`.  in_real: the source is a real array (imaginary
-// part 0; the forward transform of FftwFft3D::forward); out_real: only the real part, times
-// `scale`, is written to a real array (FftwFft3D::backward).  Otherwise complex in -> complex
-// out (may alias: each tile is read whole before it is written, and tiles are disjoint).
-template <int DIR>
-__global__ void __launch_bounds__(kNT)
-k_axis_fft(const double2* __restrict__ in, const double* __restrict__ in_real, double2* __restrict__ out,
-           double* __restrict__ out_real, double scale, int axis, Dims d, AxisPlan plan,
-           const double2* __restrict__ twl) {
-  extern __shared__ double2 sm[];
-  const int L = plan.L, tw = plan.tw;
-  double2* A = sm;
-  double2* B = sm + (size_t)L * tw;
-  const long long t = blockIdx.x;
-  const int total = L * tw;
-  // consecutive threads take consecutive x where the axis is strided, consecutive elements
-  // along the row where it is x
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    int s, e;
-    if (axis == 0) {
-      s = i / L;
-      e = i % L;
-    } else {
-      s = i % tw;
-      e = i / tw;
-    }
-    const long long g = axis_index(axis, d, tw, t, s, e);
-    double2 v = make_double2(0.0, 0.0);
-    if (g >= 0) v = in_real ? make_double2(in_real[g], 0.0) : in[g];
-    A[e * tw + s] = v;
-  }
-  __syncthreads();
-  double2* src = A;
-  double2* dst = B;
-  int Ns = 1;
-  for (int f = 0; f < plan.nfac; ++f) {
-    generic_stage<DIR>(src, dst, L, tw, plan.fac[f], Ns, twl);
-    __syncthreads();
-    Ns *= plan.fac[f];
-    double2* tmp = src;
-    src = dst;
-    dst = tmp;
-  }
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    int s, e;
-    if (axis == 0) {
-      s = i / L;
-      e = i % L;
-    } else {
-      s = i % tw;
-      e = i / tw;
-    }
-    const long long g = axis_index(axis, d, tw, t, s, e);
-    if (g < 0) continue;
-    const double2 v = src[e * tw + s];
-    if (out_real) out_real[g] = v.x * scale;
-    else out[g] = v;
-  }
-}
-
 // ------------------------------------------------------------------------------------
-// Point-wise kernels of the legacy solver (src/spectral_solver.cpp).  Mode numbers follow
+// Modes of the legacy solver (src/spectral_solver.cpp).  Mode numbers follow
 // FftwFft3D::signed_mode (index n/2 -> +n/2), k = (2 pi m) / L per axis.
 struct Modes {
   Dims d;
@@ -226,107 +104,373 @@ __device__ __forceinline__ double2 cm(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// nf consecutive fields times the phase (the shifted grid's spectra)
-__global__ void k_times_phase(const double2* __restrict__ u, double2* __restrict__ out, int nf, long long n3,
-                              Modes md) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n3) return;
-  const double2 ph = phase_of(mode_of(id, md), md);
-  for (int c = 0; c < nf; ++c) out[c * n3 + id] = cm(u[c * n3 + id], ph);
+// ------------------------------------------------------------------------------------
+// Axis transforms.
+// Where a transform's elements come from: a complex field, a real field (imaginary part 0;
+// FftwFft3D::forward), the packed Hermitian parts of two spectra (kPack, z axis only), or a
+// product of packed physical fields (kProduct).
+enum { kComplex = 0, kReal = 1, kPack = 2, kProduct = 3 };
+
+struct AxisArgs {
+  const double2* in;    // field 0; blockIdx.y steps by n3
+  const double* in_real;
+  double2* out;
+  double* out_real;     // non-null: the real part is written there (FftwFft3D::backward)
+  double scale;         // of the output
+  int axis;
+  Dims d;
+  long long n3;
+  AxisPlan plan;
+  const double2* twl;   // W_L^t = exp(-2 pi i t / L)
+  Modes md;             // kPack
+  int shifted;          // kPack, kProduct: the packed pair is one component's two grids
+  int nprod;            // kProduct: 5 (squares less u_2^2) or 6 products; -1: u_0 u_1 alone
+};
+
+__device__ __forceinline__ double2 mirror_of(const double2* __restrict__ f, int ix, int iy, int iz, Dims d) {
+  const int jx = ix ? d.nx - ix : 0, jy = iy ? d.ny - iy : 0, jz = iz ? d.nz - iz : 0;
+  return f[((long long)jz * d.ny + jy) * d.nx + jx];
+}
+__device__ __forceinline__ Mode mode_at(int ix, int iy, int iz, const Modes& md) {
+  return mode_of(((long long)iz * md.d.ny + iy) * md.d.nx + ix, md);
+}
+__device__ __forceinline__ double2 herm(double2 a, double2 m) {
+  return make_double2(0.5 * (a.x + m.x), 0.5 * (a.y - m.y));
 }
 
-__global__ void k_product(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ p,
-                          long long n3) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id < n3) p[id] = a[id] * b[id];
-}
-
-// One pair (a, b) of nonlinear_rhs (:186-228): the masked, dealiased (or plain) product
-// spectrum into its slot.
-__global__ void k_pair_value(const double2* __restrict__ c0, const double2* __restrict__ cs, double2* __restrict__ out,
-                             long long n3, Modes md, int dealias) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n3) return;
-  const Mode m = mode_of(id, md);
-  double2 v = c0[id];
-  if (dealias) {
-    const double2 ph = phase_of(m, md);
-    const double2 sb = cm(cs[id], make_double2(ph.x, -ph.y));
-    v = make_double2(0.5 * (v.x + sb.x), 0.5 * (v.y + sb.y));
+// H(U) + i H(V) at one mode: U, V = u_f on both grids (shifted), or u_2f and u_2f+1 (the last
+// one absent: zero).
+__device__ double2 packed_pair(const AxisArgs& a, int f, int ix, int iy, int iz) {
+  const long long id = ((long long)iz * a.d.ny + iy) * a.d.nx + ix;
+  double2 U, V;
+  if (a.shifted) {
+    const double2* u = a.in + f * a.n3;
+    const double2 c = u[id], m = mirror_of(u, ix, iy, iz, a.d);
+    const Mode mo = mode_at(ix, iy, iz, a.md);
+    const double2 ph = phase_of(mo, a.md);
+    // the mirror mode's phase: its wavenumber is -k, except +n/2 on an axis of index n/2
+    const int nx = a.d.nx, ny = a.d.ny, nz = a.d.nz;
+    double2 pm = make_double2(ph.x, -ph.y);
+    if (2 * ix == nx || 2 * iy == ny || 2 * iz == nz)
+      pm = phase_of(mode_at(ix ? nx - ix : 0, iy ? ny - iy : 0, iz ? nz - iz : 0, a.md), a.md);
+    U = herm(c, m);
+    V = herm(cm(c, ph), cm(m, pm));
+  } else {
+    const double2* u = a.in + 2 * f * a.n3;
+    U = herm(u[id], mirror_of(u, ix, iy, iz, a.d));
+    V = make_double2(0.0, 0.0);
+    if (2 * f + 1 < 3) V = herm(u[a.n3 + id], mirror_of(u + a.n3, ix, iy, iz, a.d));
   }
-  if (!keep_of(m, md.d)) v = make_double2(0.0, 0.0);
-  out[id] = v;
+  return make_double2(U.x - V.y, U.y + V.x);
 }
 
-// rhs_i = -i (kx P_0i + ky P_1i + kz P_2i), truncated (:230-238); then, for the full RHS
-// (:242-260), minus nu k^2 u_hat, the projection with zero mean (:94-109, 400-409) and the
-// truncation again.  P holds the 6 symmetric products in the order 00 01 02 11 12 22.
-__global__ void k_rhs_finish(const double2* __restrict__ P, const double2* __restrict__ u, double2* __restrict__ r,
-                             long long n3, Modes md, double nu, int full) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// Product p of the physical fields at point id: 00, 01, 02, 11, 12, 22, the squares less u_2^2
+// when only 5 are asked for (the difference is a gradient's, which the projection removes).
+__device__ __forceinline__ double one_product(double a, double b, bool diff) {
+  return diff ? (a - b) * (a + b) : a * b;
+}
+__device__ double2 packed_product(const AxisArgs& a, int f, long long id) {
+  auto pair = [&](int p, int* x, int* y) {
+    *x = (p >= 3) + (p >= 5);
+    *y = p < 3 ? p : (p < 5 ? p - 2 : 2);
+    const bool diff = a.nprod == 5 && *x == *y;
+    if (diff) *y = 2;
+    return diff;
+  };
+  int x, y;
+  if (a.shifted) {  // both grids of product f
+    const bool diff = pair(a.nprod < 0 ? 1 : f, &x, &y);
+    const double2 u = a.in[x * a.n3 + id], v = a.in[y * a.n3 + id];
+    return make_double2(one_product(u.x, v.x, diff), one_product(u.y, v.y, diff));
+  }
+  // products 2f and 2f + 1 (or none) on one grid; u_0, u_1 are the parts of field 0, u_2 of 1
+  auto u = [&](int c) { return c == 1 ? a.in[id].y : a.in[(c >> 1) * a.n3 + id].x; };
+  bool diff = pair(2 * f, &x, &y);
+  double2 r = make_double2(one_product(u(x), u(y), diff), 0.0);
+  if (2 * f + 1 < a.nprod) {
+    diff = pair(2 * f + 1, &x, &y);
+    r.y = one_product(u(x), u(y), diff);
+  }
+  return r;
+}
+
+// One Stockham stage: butterfly j of a sequence reads elements j + p L/R, multiplies by
+// W_{Ns R}^(p (j mod Ns)), and writes (j / Ns) Ns R + j mod Ns + q Ns.  Lanes run over the
+// sequences (axes y, z) or along the row (x), whichever is contiguous in global memory.
+template <int R, int DIR, class Ld, class St>
+__device__ __forceinline__ void axis_stage(const Ld& ld, const St& st, int L, int tw, bool row, int Ns,
+                                           const double2* __restrict__ twl) {
+  const int m = L / R, stride = m / Ns, total = tw * m;
+  for (int b = threadIdx.x; b < total; b += blockDim.x) {
+    int s, j;
+    if (row) {
+      s = b / m;
+      j = b - s * m;
+    } else {
+      s = b & (tw - 1);  // tw is a power of two
+      j = b / tw;
+    }
+    double2 v[R];
+#pragma unroll
+    for (int p = 0; p < R; ++p) v[p] = ld(s, j + p * m);
+    int base = 0, k = 0;
+    if (Ns > 1) {
+      const int q = j / Ns;
+      k = j - q * Ns;
+      base = q * Ns * R + k;
+#pragma unroll
+      for (int p = 1; p < R; ++p) {
+        double2 w = __ldg(&twl[p * k * stride]);
+        if (DIR > 0) w.y = -w.y;
+        v[p] = cm(v[p], w);
+      }
+    } else {
+      base = j * R;
+    }
+    sns::dftR<R, DIR>(v);
+#pragma unroll
+    for (int q = 0; q < R; ++q) st(s, base + q * Ns, v[q]);
+  }
+}
+
+// The same for any other radix (a prime above 7), O(r) per output from shared memory: the stage
+// twiddle and the DFT are one table lookup per term.
+template <int DIR, class St>
+__device__ void axis_stage_any(const double2* src, int es, int ss, const St& st, int L, int tw, bool row, int r,
+                               int Ns, const double2* __restrict__ twl) {
+  const int m = L / r, stride = m / Ns, total = tw * m;
+  for (int b = threadIdx.x; b < total * r; b += blockDim.x) {
+    const int q = b / total, c = b - q * total;
+    int s, j;
+    if (row) {
+      s = c / m;
+      j = c - s * m;
+    } else {
+      s = c & (tw - 1);
+      j = c / tw;
+    }
+    const int k = j % Ns, a = k * stride + q * m;  // exponent step of this output (< L)
+    double re = 0.0, im = 0.0;
+    int e = 0;
+    for (int p = 0; p < r; ++p) {
+      const double2 v = src[(j + p * m) * es + s * ss];
+      double2 w = __ldg(&twl[e]);
+      if (DIR > 0) w.y = -w.y;
+      re += v.x * w.x - v.y * w.y;
+      im += v.x * w.y + v.y * w.x;
+      e += a;
+      if (e >= L) e -= L;
+    }
+    st(s, (j / Ns) * Ns * r + k + q * Ns, make_double2(re, im));
+  }
+}
+
+template <int DIR, class Ld, class St>
+__device__ __forceinline__ void axis_stage_switch(int r, const Ld& ld, const St& st, int L, int tw, bool row, int Ns,
+                                                  const double2* __restrict__ twl) {
+  switch (r) {
+    case 2: axis_stage<2, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 3: axis_stage<3, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 4: axis_stage<4, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 5: axis_stage<5, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 6: axis_stage<6, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 7: axis_stage<7, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 8: axis_stage<8, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    case 12: axis_stage<12, DIR>(ld, st, L, tw, row, Ns, twl); break;
+    default: axis_stage<16, DIR>(ld, st, L, tw, row, Ns, twl); break;
+  }
+}
+__host__ __device__ constexpr bool register_radix(int r) { return r <= 8 || r == 12 || r == 16; }
+
+// Transform every sequence along a.axis; grid (tiles, fields).  In place is fine: a tile is
+// read whole before it is written (its last stage starts after a barrier, or, when a single
+// butterfly spans the sequence, each thread writes only what it read), and tiles are disjoint.
+template <int DIR, int LOAD>
+__global__ void __launch_bounds__(kNT) k_axis_fft(const AxisArgs a) {
+  extern __shared__ double2 sm[];
+  const int L = a.plan.L, tw = a.plan.tw, fld = blockIdx.y;
+  const bool row = a.axis == 0;
+  const long long t = blockIdx.x;
+  // element e of sequence s is base + s ss + e es, s < smax; in shared memory s sss + e ses
+  long long base, es, ss;
+  int smax, ix0 = 0, other = 0;
+  if (row) {
+    base = t * tw * a.d.nx;
+    es = 1;
+    ss = a.d.nx;
+    const long long left = (long long)a.d.ny * a.d.nz - t * tw;
+    smax = left < tw ? (int)left : tw;
+  } else {
+    const int xt = (a.d.nx + tw - 1) / tw;
+    other = (int)(t / xt);  // iz (axis 1) or iy (axis 2)
+    ix0 = (int)(t - (long long)other * xt) * tw;
+    smax = a.d.nx - ix0 < tw ? a.d.nx - ix0 : tw;
+    ss = 1;
+    if (a.axis == 1) {
+      base = (long long)other * a.d.ny * a.d.nx + ix0;
+      es = a.d.nx;
+    } else {
+      base = (long long)other * a.d.nx + ix0;
+      es = (long long)a.d.nx * a.d.ny;
+    }
+  }
+  const int ses = row ? 1 : tw, sss = row ? L : 1;
+  const double2* in = a.in + (LOAD == kComplex ? fld * a.n3 : 0);
+  auto from_global = [&](int s, int e) -> double2 {
+    if (s >= smax) return make_double2(0.0, 0.0);
+    const long long id = base + s * ss + e * es;
+    if constexpr (LOAD == kComplex) return in[id];
+    else if constexpr (LOAD == kReal) return make_double2(a.in_real[id], 0.0);
+    else if constexpr (LOAD == kPack) return packed_pair(a, fld, ix0 + s, other, e);
+    else return packed_product(a, fld, id);
+  };
+  auto to_global = [&](int s, int e, double2 v) {
+    if (s >= smax) return;
+    const long long id = base + s * ss + e * es;
+    if (a.out_real) a.out_real[id] = v.x * a.scale;
+    else a.out[fld * a.n3 + id] = make_double2(v.x * a.scale, v.y * a.scale);
+  };
+  double2* src = sm;
+  double2* dst = sm + (size_t)L * tw;  // (plans of one or two register stages never touch it)
+  const int nfac = a.plan.nfac;
+  int f = 0, Ns = 1;
+  if (nfac == 1 && register_radix(a.plan.fac[0])) {
+    axis_stage_switch<DIR>(a.plan.fac[0], from_global, to_global, L, tw, row, 1, a.twl);
+    return;
+  }
+  auto into = [&](double2* p) { return [=](int s, int e, double2 v) { p[s * sss + e * ses] = v; }; };
+  if (register_radix(a.plan.fac[0])) {
+    axis_stage_switch<DIR>(a.plan.fac[0], from_global, into(src), L, tw, row, 1, a.twl);
+    Ns = a.plan.fac[0];
+    f = 1;
+  } else {
+    for (int i = threadIdx.x; i < L * tw; i += blockDim.x) {
+      const int s = row ? i / L : i & (tw - 1), e = row ? i - s * L : i / tw;
+      into(src)(s, e, from_global(s, e));
+    }
+  }
+  __syncthreads();
+  for (; f < nfac; ++f) {
+    const int r = a.plan.fac[f];
+    const bool last = f == nfac - 1;
+    auto from_src = [&](int s, int e) { return src[s * sss + e * ses]; };
+    if (register_radix(r)) {
+      if (last) axis_stage_switch<DIR>(r, from_src, to_global, L, tw, row, Ns, a.twl);
+      else axis_stage_switch<DIR>(r, from_src, into(dst), L, tw, row, Ns, a.twl);
+    } else {
+      if (last) axis_stage_any<DIR>(src, ses, sss, to_global, L, tw, row, r, Ns, a.twl);
+      else axis_stage_any<DIR>(src, ses, sss, into(dst), L, tw, row, r, Ns, a.twl);
+    }
+    if (last) return;
+    __syncthreads();
+    Ns *= r;
+    double2* tmp = src;
+    src = dst;
+    dst = tmp;
+  }
+}
+
+// ------------------------------------------------------------------------------------
+// Point-wise kernels.
+
+// The dealiased (or plain), masked spectrum of product p at mode id from the packed
+// transforms Z (nonlinear_rhs, src/spectral_solver.cpp:186-228).
+__device__ double2 product_value(const double2* __restrict__ Z, int p, long long id, int ix, int iy, int iz,
+                                 long long n3, Dims d, double2 ph, bool keep, int dealias) {
+  if (!keep) return make_double2(0.0, 0.0);
+  const double2* f = Z + (dealias ? p : p / 2) * n3;
+  const double2 z = f[id], m = mirror_of(f, ix, iy, iz, d);
+  const double2 re = herm(z, m);                                             // the real part's spectrum
+  const double2 im = make_double2(0.5 * (z.y + m.y), -0.5 * (z.x - m.x));    // the imaginary part's
+  if (!dealias) return p % 2 ? im : re;
+  const double2 sb = cm(im, make_double2(ph.x, -ph.y));
+  return make_double2(0.5 * (re.x + sb.x), 0.5 * (re.y + sb.y));
+}
+
+__device__ __forceinline__ void project_mode(const Mode& m, bool drop, double2 v[3]) {
+  if (m.k2 != 0.0) {
+    const double2 dot = make_double2(m.kx * v[0].x + m.ky * v[1].x + m.kz * v[2].x,
+                                     m.kx * v[0].y + m.ky * v[1].y + m.kz * v[2].y);
+    const double2 f = make_double2(dot.x / m.k2, dot.y / m.k2);
+    const double kv[3] = {m.kx, m.ky, m.kz};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = make_double2(v[i].x - kv[i] * f.x, v[i].y - kv[i] * f.y);
+  }
+  if (drop) v[0] = v[1] = v[2] = make_double2(0.0, 0.0);  // zero_mean, truncate
+}
+
+// rhs_i = -i (kx P_0i + ky P_1i + kz P_2i), truncated (:230-238); for the full RHS (:242-260)
+// minus nu k^2 u_hat, the projection with zero mean (:94-109, 400-409) and the truncation
+// again; with g, one stage of step_rk3 (:262-309) on it: g = ga g + rhs (first stage: g = rhs),
+// u += b g, project with zero mean, truncate.  nprod = 6: all products; 5: the diagonal ones
+// less u_2^2 (full RHS only).
+struct FinishArgs {
+  const double2* Z;
+  double2* u;
+  double2* r;  // the right-hand side is written here (g null)
+  double2* g;
+  double nu, ga, b;
+  int dealias, nprod, full, first;
+};
+__global__ void __launch_bounds__(256) k_finish(const FinishArgs a, long long n3, Modes md) {
+  const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
   if (id >= n3) return;
   const Mode m = mode_of(id, md);
-  const bool keep = keep_of(m, md.d);
+  const int ix = (int)(id % md.d.nx), iy = (int)((id / md.d.nx) % md.d.ny);
+  const int iz = (int)(id / ((long long)md.d.nx * md.d.ny));
+  const bool keep = keep_of(m, md.d), drop = id == 0 || !keep;
+  double2 ph = make_double2(1.0, 0.0);
+  if (a.dealias && keep) ph = phase_of(m, md);
+  double2 P[6];
+#pragma unroll
+  for (int p = 0; p < 6; ++p)
+    P[p] = p < a.nprod ? product_value(a.Z, p, id, ix, iy, iz, n3, md.d, ph, keep, a.dealias)
+                       : make_double2(0.0, 0.0);
   const int slot[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
   double2 out[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const double2 p0 = P[slot[0][i] * n3 + id], p1 = P[slot[1][i] * n3 + id], p2 = P[slot[2][i] * n3 + id];
-    const double sx = m.kx * p0.x + m.ky * p1.x + m.kz * p2.x;
-    const double sy = m.kx * p0.y + m.ky * p1.y + m.kz * p2.y;
-    out[i] = keep ? make_double2(sy, -sx) : make_double2(0.0, 0.0);  // -i (sx + i sy)
+    const double2 p0 = P[slot[0][i]], p1 = P[slot[1][i]], p2 = P[slot[2][i]];
+    out[i] = make_double2(m.kx * p0.y + m.ky * p1.y + m.kz * p2.y, -(m.kx * p0.x + m.ky * p1.x + m.kz * p2.x));
   }
-  if (full) {
+  double2 uu[3];
+  if (a.full) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const double2 ui = u[i * n3 + id];
-      out[i] = make_double2(out[i].x - nu * m.k2 * ui.x, out[i].y - nu * m.k2 * ui.y);
+      uu[i] = a.u[i * n3 + id];
+      out[i] = make_double2(out[i].x - a.nu * m.k2 * uu[i].x, out[i].y - a.nu * m.k2 * uu[i].y);
     }
-    if (m.k2 != 0.0) {
-      const double2 dot = make_double2(m.kx * out[0].x + m.ky * out[1].x + m.kz * out[2].x,
-                                       m.kx * out[0].y + m.ky * out[1].y + m.kz * out[2].y);
-      const double2 f = make_double2(dot.x / m.k2, dot.y / m.k2);
-      const double kv[3] = {m.kx, m.ky, m.kz};
-#pragma unroll
-      for (int i = 0; i < 3; ++i) out[i] = make_double2(out[i].x - kv[i] * f.x, out[i].y - kv[i] * f.y);
-    }
-    if (id == 0 || !keep) out[0] = out[1] = out[2] = make_double2(0.0, 0.0);  // zero_mean, truncate
+    project_mode(m, drop, out);
   }
+  if (a.g == nullptr) {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) r[i * n3 + id] = out[i];
-}
-
-// One stage of step_rk3 (:262-309): g = a g + h (first stage: g = h), u += b g, project
-// with zero mean, truncate.
-__global__ void k_rk_stage(double2* __restrict__ u, double2* __restrict__ g, const double2* __restrict__ h,
-                           long long n3, Modes md, double a, double b, int first) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n3) return;
-  const Mode m = mode_of(id, md);
-  double2 uu[3];
+    for (int i = 0; i < 3; ++i) a.r[i * n3 + id] = out[i];
+    return;
+  }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const double2 hh = h[c * n3 + id];
-    double2 gg = hh;
-    if (!first) {
-      const double2 go = g[c * n3 + id];
-      gg = make_double2(a * go.x + hh.x, a * go.y + hh.y);
+    double2 gg = out[c];
+    if (!a.first) {
+      const double2 go = a.g[c * n3 + id];
+      gg = make_double2(a.ga * go.x + gg.x, a.ga * go.y + gg.y);
     }
-    g[c * n3 + id] = gg;
-    const double2 u0 = u[c * n3 + id];
-    uu[c] = make_double2(u0.x + b * gg.x, u0.y + b * gg.y);
+    a.g[c * n3 + id] = gg;
+    uu[c] = make_double2(uu[c].x + a.b * gg.x, uu[c].y + a.b * gg.y);
   }
-  if (m.k2 != 0.0) {
-    const double2 dot = make_double2(m.kx * uu[0].x + m.ky * uu[1].x + m.kz * uu[2].x,
-                                     m.kx * uu[0].y + m.ky * uu[1].y + m.kz * uu[2].y);
-    const double2 f = make_double2(dot.x / m.k2, dot.y / m.k2);
-    const double kv[3] = {m.kx, m.ky, m.kz};
+  project_mode(m, drop, uu);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) uu[c] = make_double2(uu[c].x - kv[c] * f.x, uu[c].y - kv[c] * f.y);
-  }
-  if (id == 0 || !keep_of(m, md.d)) uu[0] = uu[1] = uu[2] = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) u[c * n3 + id] = uu[c];
+  for (int c = 0; c < 3; ++c) a.u[c * n3 + id] = uu[c];
+}
+
+// product_dealiased (:122-158): one packed product's value
+__global__ void __launch_bounds__(256) k_pair_value(const double2* __restrict__ Z, double2* __restrict__ out,
+                                                    long long n3, Modes md) {
+  const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (id >= n3) return;
+  const Mode m = mode_of(id, md);
+  const int ix = (int)(id % md.d.nx), iy = (int)((id / md.d.nx) % md.d.ny);
+  const int iz = (int)(id / ((long long)md.d.nx * md.d.ny));
+  out[id] = product_value(Z, 0, id, ix, iy, iz, n3, md.d, phase_of(m, md), keep_of(m, md.d), 1);
 }
 
 // omega_hat = i k x u_hat (vorticity_hat, src/spectral_solver.cpp:338-351)
@@ -412,8 +556,9 @@ void gck(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw GenericError(SNS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// Radices of L in application order: 8s, a 4 or 2 for the rest of the power of two, then
-// 3, 5, 7 and any larger prime (a direct DFT of that length).
+// Radices of L in application order: the primes above 7 (direct DFTs) first, then the fewest
+// register butterflies of 2 .. 8, 12, 16 whose product is the rest, the largest first (the
+// first stage has no twiddles); of equal counts the smallest largest radix.
 bool factor(int L, AxisPlan& p) {
   p.L = L;
   p.nfac = 0;
@@ -421,18 +566,37 @@ bool factor(int L, AxisPlan& p) {
   auto push = [&](int r) {
     if (p.nfac >= kMaxFactors) return false;
     p.fac[p.nfac++] = r;
-    rest /= r;
     return true;
   };
-  while (rest % 8 == 0)
-    if (!push(8)) return false;
-  if (rest % 4 == 0 && !push(4)) return false;
-  if (rest % 2 == 0 && !push(2)) return false;
-  for (int f = 3; rest > 1; f += 2) {
+  for (int f = 2; f <= 7; ++f)
+    while (rest % f == 0) rest /= f;
+  const int smooth = L / rest;
+  for (int f = 11; rest > 1; f += 2) {
     if ((long long)f * f > rest) f = rest;
-    while (rest % f == 0)
+    while (rest % f == 0) {
       if (!push(f)) return false;
+      rest /= f;
+    }
   }
+  static const int radix[] = {2, 3, 4, 5, 6, 7, 8, 12, 16};
+  // by depth-first search: few divisors, a handful of stages
+  std::vector<int> best, cur;
+  auto search = [&](auto&& self, int n, int most) -> void {
+    if (n == 1) {
+      if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && cur[0] < best[0])) best = cur;
+      return;
+    }
+    if (!best.empty() && cur.size() >= best.size()) return;
+    for (int i = 8; i >= 0; --i)
+      if (radix[i] <= most && n % radix[i] == 0) {
+        cur.push_back(radix[i]);
+        self(self, n / radix[i], radix[i]);
+        cur.pop_back();
+      }
+  };
+  search(search, smooth, 16);
+  for (int r : best)
+    if (!push(r)) return false;
   return true;
 }
 
@@ -452,7 +616,7 @@ struct sns_fft3d {
   double* real = nullptr;   // one real field
   // the legacy solver's working set, allocated by the first solver call
   double2* sw = nullptr;  // 18 complex fields: u (3), g (3), h (3), products (6), scratch (3)
-  double* pr = nullptr;   // 8 real fields: velocity on both grids (6), two products
+  double* pr = nullptr;   // 3 real fields (diagnostics, the vorticity slice)
   double* part = nullptr;  // reduction partials
   double* red = nullptr;
   size_t bytes = 0;
@@ -462,37 +626,6 @@ struct sns_fft3d {
 namespace {
 
 constexpr int kRedBlocks = 1184;
-
-void launch_axis(sns_fft3d* h, int axis, int dir, const double2* in, const double* in_real, double2* out,
-                 double* out_real, double scale) {
-  const AxisPlan& p = h->plan[axis];
-  const Dims& d = h->d;
-  long long tiles;
-  if (axis == 0) tiles = ((long long)d.ny * d.nz + p.tw - 1) / p.tw;
-  else tiles = (long long)((d.nx + p.tw - 1) / p.tw) * (axis == 1 ? d.nz : d.ny);
-  const size_t smem = 2 * (size_t)p.L * p.tw * sizeof(double2);
-  if (dir < 0)
-    k_axis_fft<-1><<<(unsigned)tiles, kNT, smem, h->stream>>>(in, in_real, out, out_real, scale, axis, d, p,
-                                                                 h->tw[axis]);
-  else
-    k_axis_fft<+1><<<(unsigned)tiles, kNT, smem, h->stream>>>(in, in_real, out, out_real, scale, axis, d, p,
-                                                                 h->tw[axis]);
-}
-
-// Forward transform of one real field into a complex field (x, y, z passes).
-void forward_real(sns_fft3d* h, const double* real, double2* spec) {
-  launch_axis(h, 0, -1, nullptr, real, spec, nullptr, 1.0);
-  launch_axis(h, 1, -1, spec, nullptr, spec, nullptr, 1.0);
-  launch_axis(h, 2, -1, spec, nullptr, spec, nullptr, 1.0);
-}
-
-// Re(IDFT(spec)) / N into a real field; `scratch` (a complex field) may alias `spec` when the
-// spectrum need not survive.
-void backward_real(sns_fft3d* h, const double2* spec, double2* scratch, double* real) {
-  launch_axis(h, 2, +1, spec, nullptr, scratch, nullptr, 1.0);
-  launch_axis(h, 1, +1, scratch, nullptr, scratch, nullptr, 1.0);
-  launch_axis(h, 0, +1, scratch, nullptr, nullptr, real, 1.0 / (double)h->n3);
-}
 
 Modes modes_of(const sns_fft3d* h) {
   Modes m;
@@ -504,6 +637,61 @@ Modes modes_of(const sns_fft3d* h) {
   m.hy = 0.5 * h->len[1] / h->d.ny;
   m.hz = 0.5 * h->len[2] / h->d.nz;
   return m;
+}
+
+// One axis pass of nf fields (a.axis and the sources set by the caller).
+template <int LOAD>
+void launch_axis(sns_fft3d* h, int dir, AxisArgs a, int nf = 1) {
+  const AxisPlan& p = h->plan[a.axis];
+  const Dims& d = h->d;
+  a.d = d;
+  a.n3 = h->n3;
+  a.plan = p;
+  a.twl = h->tw[a.axis];
+  long long tiles;
+  if (a.axis == 0) tiles = ((long long)d.ny * d.nz + p.tw - 1) / p.tw;
+  else tiles = (long long)((d.nx + p.tw - 1) / p.tw) * (a.axis == 1 ? d.nz : d.ny);
+  // two register stages meet in one buffer; one needs none; a thread per butterfly of 8 points
+  const bool regs = register_radix(p.fac[0]) && register_radix(p.fac[p.nfac - 1]);
+  const int nbuf = regs && p.nfac <= 2 ? p.nfac - 1 : 2;
+  const size_t smem = nbuf * (size_t)p.L * p.tw * sizeof(double2);
+  const int nt = std::min(kNT, std::max(32, (p.L * p.tw / 8 + 31) / 32 * 32));
+  const dim3 grid((unsigned)tiles, nf);
+  if constexpr (LOAD == kPack) {
+    k_axis_fft<+1, LOAD><<<grid, nt, smem, h->stream>>>(a);
+  } else if constexpr (LOAD == kComplex) {
+    if (dir < 0) k_axis_fft<-1, LOAD><<<grid, nt, smem, h->stream>>>(a);
+    else k_axis_fft<+1, LOAD><<<grid, nt, smem, h->stream>>>(a);
+  } else {
+    k_axis_fft<-1, LOAD><<<grid, nt, smem, h->stream>>>(a);
+  }
+}
+AxisArgs axis_args(int axis, const double2* in, double2* out, double scale = 1.0) {
+  AxisArgs a{};
+  a.axis = axis;
+  a.in = in;
+  a.out = out;
+  a.scale = scale;
+  return a;
+}
+
+// Forward transform of one real field into a complex field (x, y, z passes).
+void forward_real(sns_fft3d* h, const double* real, double2* spec) {
+  AxisArgs a = axis_args(0, nullptr, spec);
+  a.in_real = real;
+  launch_axis<kReal>(h, -1, a);
+  launch_axis<kComplex>(h, -1, axis_args(1, spec, spec));
+  launch_axis<kComplex>(h, -1, axis_args(2, spec, spec));
+}
+
+// Re(IDFT(spec)) / N into a real field; `scratch` (a complex field) may alias `spec` when the
+// spectrum need not survive.
+void backward_real(sns_fft3d* h, const double2* spec, double2* scratch, double* real) {
+  launch_axis<kComplex>(h, +1, axis_args(2, spec, scratch));
+  launch_axis<kComplex>(h, +1, axis_args(1, scratch, scratch));
+  AxisArgs a = axis_args(0, scratch, nullptr, 1.0 / (double)h->n3);
+  a.out_real = real;
+  launch_axis<kComplex>(h, +1, a);
 }
 
 void dalloc(sns_fft3d* h, void** p, size_t bytes) {
@@ -520,12 +708,12 @@ void ensure_solver_memory(sns_fft3d* h) {
   const size_t cf = (size_t)h->n3 * sizeof(double2), rf = (size_t)h->n3 * sizeof(double);
   size_t free_b = 0, total_b = 0;
   gck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-  const size_t need = 18 * cf + 8 * rf + (2 * kRedBlocks + 16) * sizeof(double);
+  const size_t need = 18 * cf + 3 * rf + (2 * kRedBlocks + 16) * sizeof(double);
   if (need > free_b)
     throw GenericError(SNS_ERR_NOMEM, "the solver working set needs " + std::to_string(need) + " bytes, device has " +
                                           std::to_string(free_b) + " free");
   dalloc(h, (void**)&h->sw, 18 * cf);
-  dalloc(h, (void**)&h->pr, 8 * rf);
+  dalloc(h, (void**)&h->pr, 3 * rf);
   dalloc(h, (void**)&h->part, 2 * kRedBlocks * sizeof(double));
   dalloc(h, (void**)&h->red, 16 * sizeof(double));
 }
@@ -535,27 +723,47 @@ double* PR(sns_fft3d* h, int f) { return h->pr + (size_t)f * h->n3; }
 // slots of the working set
 constexpr int kU = 0, kG = 3, kH = 6, kP = 9, kS = 15;
 
-// nonlinear_rhs of u (slots kU) into slots `dst`; full = 1: the whole rhs
-void rhs_device(sns_fft3d* h, double nu, int dealias, int full, int dst) {
-  const long long n3 = h->n3;
-  const Modes md = modes_of(h);
-  const unsigned nb = blocks(n3, 256);
-  for (int c = 0; c < 3; ++c) backward_real(h, SW(h, kU + c), SW(h, kS), PR(h, c));
-  if (dealias) {
-    k_times_phase<<<nb, 256, 0, h->stream>>>(SW(h, kU), SW(h, kS), 3, n3, md);
-    for (int c = 0; c < 3; ++c) backward_real(h, SW(h, kS + c), SW(h, kS + c), PR(h, 3 + c));
-  }
-  const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
-  for (int p = 0; p < 6; ++p) {
-    k_product<<<nb, 256, 0, h->stream>>>(PR(h, pa[p]), PR(h, pb[p]), PR(h, 6), n3);
-    forward_real(h, PR(h, 6), SW(h, kS));
-    if (dealias) {
-      k_product<<<nb, 256, 0, h->stream>>>(PR(h, 3 + pa[p]), PR(h, 3 + pb[p]), PR(h, 7), n3);
-      forward_real(h, PR(h, 7), SW(h, kS + 1));
-    }
-    k_pair_value<<<nb, 256, 0, h->stream>>>(SW(h, kS), SW(h, kS + 1), SW(h, kP + p), n3, md, dealias);
-  }
-  k_rhs_finish<<<nb, 256, 0, h->stream>>>(SW(h, kP), SW(h, kU), SW(h, dst), n3, md, nu, full);
+// The packed products' spectra of `nu` spectra (first slot kU) into the slots from kP: the
+// physical fields are formed in kS.
+void product_spectra(sns_fft3d* h, int nu, int shifted, int nprod) {
+  const int nin = shifted ? nu : (nu + 1) / 2, nout = shifted ? nprod : (nprod + 1) / 2;
+  AxisArgs a = axis_args(2, SW(h, kU), SW(h, kS), 1.0 / (double)h->n3);
+  a.md = modes_of(h);
+  a.shifted = shifted;
+  launch_axis<kPack>(h, +1, a, nin);
+  launch_axis<kComplex>(h, +1, axis_args(1, SW(h, kS), SW(h, kS)), nin);
+  launch_axis<kComplex>(h, +1, axis_args(0, SW(h, kS), SW(h, kS)), nin);
+  a = axis_args(0, SW(h, kS), SW(h, kP));
+  a.shifted = shifted;
+  a.nprod = nprod;
+  launch_axis<kProduct>(h, -1, a, nout);
+  launch_axis<kComplex>(h, -1, axis_args(1, SW(h, kP), SW(h, kP)), nout);
+  launch_axis<kComplex>(h, -1, axis_args(2, SW(h, kP), SW(h, kP)), nout);
+}
+
+// The product of the two fields in slots kU, kU + 1, on both grids, into slot kP.
+void pair_spectrum(sns_fft3d* h) {
+  AxisArgs a = axis_args(2, SW(h, kU), SW(h, kS), 1.0 / (double)h->n3);
+  a.md = modes_of(h);
+  a.shifted = 1;
+  launch_axis<kPack>(h, +1, a, 2);
+  launch_axis<kComplex>(h, +1, axis_args(1, SW(h, kS), SW(h, kS)), 2);
+  launch_axis<kComplex>(h, +1, axis_args(0, SW(h, kS), SW(h, kS)), 2);
+  a = axis_args(0, SW(h, kS), SW(h, kP));
+  a.shifted = 1;
+  a.nprod = -1;  // u_0 u_1 alone
+  launch_axis<kProduct>(h, -1, a);
+  launch_axis<kComplex>(h, -1, axis_args(1, SW(h, kP), SW(h, kP)));
+  launch_axis<kComplex>(h, -1, axis_args(2, SW(h, kP), SW(h, kP)));
+}
+
+// The right-hand side of u (slots kU; full = 0: nonlinear_rhs), or one RK stage on it.
+void stage_device(sns_fft3d* h, FinishArgs f) {
+  f.nprod = f.full ? 5 : 6;
+  product_spectra(h, 3, f.dealias, f.nprod);
+  f.Z = SW(h, kP);
+  f.u = SW(h, kU);
+  k_finish<<<blocks(h->n3, 256), 256, 0, h->stream>>>(f, h->n3, modes_of(h));
 }
 
 void gsync(sns_fft3d* h, const char* what) {
@@ -683,8 +891,14 @@ int sns_fft3d_create(int nx, int ny, int nz, double lx, double ly, double lz, sn
       gck(cudaMemcpyAsync(h->tw[a], t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, h->stream), "tw");
       gck(cudaStreamSynchronize(h->stream), "tw");
     }
-    gck(cudaFuncSetAttribute(k_axis_fft<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget), "attr");
-    gck(cudaFuncSetAttribute(k_axis_fft<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget), "attr");
+    auto allow = [](auto k) {
+      gck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget), "attr");
+    };
+    allow(k_axis_fft<-1, kComplex>);
+    allow(k_axis_fft<-1, kReal>);
+    allow(k_axis_fft<-1, kProduct>);
+    allow(k_axis_fft<+1, kComplex>);
+    allow(k_axis_fft<+1, kPack>);
     gsync(h, "sns_fft3d_create");
   } catch (const GenericError& e) {
     sns::set_handleless_error(e.msg.c_str());
@@ -737,7 +951,12 @@ int sns_fft3d_rhs(sns_fft3d* h, double nu, int dealias, int full, const double* 
       throw GenericError(SNS_ERR_INVALID, "nu must be >= 0, dealias and full 0 or 1");
     ensure_solver_memory(h);
     upload3(h, uhat, kU);
-    rhs_device(h, nu, dealias, full, kH);
+    FinishArgs f{};
+    f.r = SW(h, kH);
+    f.nu = nu;
+    f.dealias = dealias;
+    f.full = full;
+    stage_device(h, f);
     download3(h, kH, out);
     gsync(h, "sns_fft3d_rhs");
   });
@@ -750,15 +969,20 @@ int sns_fft3d_step(sns_fft3d* h, double nu, int dealias, double dt, int nsteps, 
       throw GenericError(SNS_ERR_INVALID, "nu must be >= 0, dealias 0 or 1, nsteps >= 0, dt finite");
     ensure_solver_memory(h);
     upload3(h, uhat, kU);
-    const Modes md = modes_of(h);
-    const unsigned nb = blocks(h->n3, 256);
     // Williamson low-storage RK3 with the reference's coefficient products (:262-309)
-    const double a[3] = {0.0, -(5.0 / 9.0), -(153.0 / 128.0)};
+    const double ga[3] = {0.0, -(5.0 / 9.0), -(153.0 / 128.0)};
     const double b[3] = {dt / 3.0, (15.0 / 16.0) * dt, (8.0 / 15.0) * dt};
+    FinishArgs f{};
+    f.g = SW(h, kG);
+    f.nu = nu;
+    f.dealias = dealias;
+    f.full = 1;
     for (int s = 0; s < nsteps; ++s)
       for (int st = 0; st < 3; ++st) {
-        rhs_device(h, nu, dealias, 1, kH);
-        k_rk_stage<<<nb, 256, 0, h->stream>>>(SW(h, kU), SW(h, kG), SW(h, kH), h->n3, md, a[st], b[st], st == 0);
+        f.ga = ga[st];
+        f.b = b[st];
+        f.first = st == 0;
+        stage_device(h, f);
       }
     download3(h, kU, uhat);
     gsync(h, "sns_fft3d_step");
@@ -802,19 +1026,11 @@ int sns_fft3d_product(sns_fft3d* h, const double* a_hat, const double* b_hat, do
     const size_t cf = (size_t)n3 * sizeof(double2);
     gck(cudaMemcpyAsync(SW(h, kU), a_hat, cf, cudaMemcpyHostToDevice, h->stream), "upload");
     gck(cudaMemcpyAsync(SW(h, kU + 1), b_hat, cf, cudaMemcpyHostToDevice, h->stream), "upload");
-    const Modes md = modes_of(h);
-    const unsigned nb = blocks(n3, 256);
     // product_dealiased (src/spectral_solver.cpp:122-158): both grids, whatever the solver's
     // dealiasing flag
-    for (int c = 0; c < 2; ++c) backward_real(h, SW(h, kU + c), SW(h, kS), PR(h, c));
-    k_product<<<nb, 256, 0, h->stream>>>(PR(h, 0), PR(h, 1), PR(h, 6), n3);
-    forward_real(h, PR(h, 6), SW(h, kH));
-    k_times_phase<<<nb, 256, 0, h->stream>>>(SW(h, kU), SW(h, kS), 2, n3, md);
-    for (int c = 0; c < 2; ++c) backward_real(h, SW(h, kS + c), SW(h, kS + c), PR(h, 3 + c));
-    k_product<<<nb, 256, 0, h->stream>>>(PR(h, 3), PR(h, 4), PR(h, 7), n3);
-    forward_real(h, PR(h, 7), SW(h, kH + 1));
-    k_pair_value<<<nb, 256, 0, h->stream>>>(SW(h, kH), SW(h, kH + 1), SW(h, kP), n3, md, 1);
-    gck(cudaMemcpyAsync(out, SW(h, kP), cf, cudaMemcpyDeviceToHost, h->stream), "download");
+    pair_spectrum(h);
+    k_pair_value<<<blocks(n3, 256), 256, 0, h->stream>>>(SW(h, kP), SW(h, kH), n3, modes_of(h));
+    gck(cudaMemcpyAsync(out, SW(h, kH), cf, cudaMemcpyDeviceToHost, h->stream), "download");
     gsync(h, "sns_fft3d_product");
   });
 }
@@ -829,8 +1045,9 @@ int sns_fft3d_vorticity_slice(sns_fft3d* h, const double* const uhat[3], int iz,
     k_vorticity_hat<<<blocks(n3, 256), 256, 0, h->stream>>>(SW(h, kU), SW(h, kG), n3, modes_of(h));
     for (int c = 0; c < 3; ++c) backward_real(h, SW(h, kG + c), SW(h, kS), PR(h, c));
     const int nxy = h->d.nx * h->d.ny;
-    k_slice_mag<<<blocks(nxy, 256), 256, 0, h->stream>>>(PR(h, 0), n3, (long long)iz * nxy, nxy, PR(h, 6));
-    gck(cudaMemcpyAsync(host_mag, PR(h, 6), (size_t)nxy * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
+    k_slice_mag<<<blocks(nxy, 256), 256, 0, h->stream>>>(PR(h, 0), n3, (long long)iz * nxy, nxy,
+                                                       reinterpret_cast<double*>(SW(h, kS)));
+    gck(cudaMemcpyAsync(host_mag, SW(h, kS), (size_t)nxy * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
         "download");
     gsync(h, "sns_fft3d_vorticity_slice");
   });

@@ -22,46 +22,6 @@ namespace sns {
 
 namespace {
 
-// Good-Thomas 6 = 2 x 3 and 12 = 3 x 4: no twiddles between the factors.
-template <int DIR, class C>
-__device__ __forceinline__ void dft6(C* v) {
-  C t[2][3];
-#pragma unroll
-  for (int n1 = 0; n1 < 2; ++n1) {
-#pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) t[n1][n2] = v[(3 * n1 + 2 * n2) % 6];
-    dft3<DIR>(t[n1]);
-  }
-#pragma unroll
-  for (int k2 = 0; k2 < 3; ++k2) {
-    v[(4 * k2) % 6] = cadd(t[0][k2], t[1][k2]);
-    v[(3 + 4 * k2) % 6] = csub(t[0][k2], t[1][k2]);
-  }
-}
-template <int DIR, class C>
-__device__ __forceinline__ void dft12(C* v) {
-  C t[3][4];
-#pragma unroll
-  for (int n1 = 0; n1 < 3; ++n1) {
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) t[n1][n2] = v[(4 * n1 + 3 * n2) % 12];
-    dft4<DIR>(t[n1]);
-  }
-#pragma unroll
-  for (int k2 = 0; k2 < 4; ++k2) {
-    C w[3] = {t[0][k2], t[1][k2], t[2][k2]};
-    dft3<DIR>(w);
-#pragma unroll
-    for (int k1 = 0; k1 < 3; ++k1) v[(4 * k1 + 9 * k2) % 12] = w[k1];
-  }
-}
-template <int R, int DIR, class C>
-__device__ __forceinline__ void dft_r(C* v) {
-  if constexpr (R == 6) dft6<DIR>(v);
-  else if constexpr (R == 12) dft12<DIR>(v);
-  else dftR<R, DIR>(v);
-}
-
 template <int A, int B>
 struct Split {
   static constexpr int R1 = A, R2 = B;
@@ -100,7 +60,7 @@ __device__ __forceinline__ void fwd1(C* p, At at, const C* tw, int n2, int lim) 
   C v[S::R1];
 #pragma unroll
   for (int r = 0; r < S::R1; ++r) v[r] = p[SNS_IDX(at(S::slot(r, n2)), lim)];
-  dft_r<S::R1, DIR>(v);
+  dftR<S::R1, DIR>(v);
   p[SNS_IDX(at(S::slot(0, n2)), lim)] = v[0];
 #pragma unroll
   for (int k1 = 1; k1 < S::R1; ++k1)
@@ -110,12 +70,12 @@ template <class S, int DIR, class C, class At>
 __device__ __forceinline__ void fwd2(const C* p, At at, int k1, int lim, C v[S::R2]) {
 #pragma unroll
   for (int n2 = 0; n2 < S::R2; ++n2) v[n2] = p[SNS_IDX(at(S::slot(k1, n2)), lim)];
-  dft_r<S::R2, DIR>(v);
+  dftR<S::R2, DIR>(v);
 }
 // Permuted in: pass 1 of row k1 (size R2, on registers), pass 2 of column m2 (size R1).
 template <class S, int DIR, class C, class At>
 __device__ __forceinline__ void rev1(C v[S::R2], C* p, At at, const C* tw, int k1, int lim) {
-  dft_r<S::R2, DIR>(v);
+  dftR<S::R2, DIR>(v);
   p[SNS_IDX(at(S::slot(k1, 0)), lim)] = v[0];
 #pragma unroll
   for (int m2 = 1; m2 < S::R2; ++m2)
@@ -125,7 +85,7 @@ template <class S, int DIR, class C, class At>
 __device__ __forceinline__ void rev2(const C* p, At at, int m2, int lim, C v[S::R1]) {
 #pragma unroll
   for (int k1 = 0; k1 < S::R1; ++k1) v[k1] = p[SNS_IDX(at(S::slot(k1, m2)), lim)];
-  dft_r<S::R1, DIR>(v);
+  dftR<S::R1, DIR>(v);
 }
 
 // Asynchronous copy of V consecutive values (8 or 16 bytes, aligned to their size).
