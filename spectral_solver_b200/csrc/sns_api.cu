@@ -9,6 +9,7 @@
 //   tables: twiddles (N), phase exp(i*pi*(mx+my+mz)/N) for mx+my+mz in [-3N/2, 3N/2],
 //           reduction partials, the 12 Nyquist-plane sums.
 #include "sns_kernels.cuh"
+#include "sns_p5.cuh"
 #include "sns_small.cuh"
 #include "../../include/sns_b200.h"
 
@@ -110,7 +111,9 @@ struct sns_handle {
   int warm_steps = 0;        // steps taken launch by launch
   int tma_grid = 0;         // persistent CTAs of the TMA passes
   int x2_grid = 0;          // persistent CTAs of the two-stage x pass (0: generic x pass)
-  int p5_grid = 0;          // persistent CTAs of the fused forward-z + sweep pass (0: two kernels)
+  const sns::P5Ops* p5 = nullptr;  // the fused forward-z + sweep pass, where the size has it
+  int p5_grid = 0;          // its persistent CTAs (0: two kernels)
+  CUtensorMap map_p5_state{};      // the state fields, boxes of its state units
   void* tw2 = nullptr;      // W_N^(r*j), r < N/16, j < 16 (two-stage x pass)
   double* nyq_part = nullptr;  // [12][max(1, x2_grid)] Nyquist-plane partial sums
   CUtensorMap map_state_z{};  // state fields (u[3], g[3]), z-pencil boxes
@@ -292,14 +295,14 @@ EncodeTiled encode_fn() {
 }
 
 // Tensor map over `nf` consecutive half fields viewed as [field][z][y][2*pitch reals],
-// box = 128 bytes (16 doubles = 8 complex, or 32 floats = 16 complex) x up to 256 rows
+// box = 128 bytes (16 doubles = 8 complex, or 32 floats = 16 complex) x up to `rows` rows
 // along y (axis 1) or z (axis 2).
-CUtensorMap make_field_map(void* base, int nf, int axis, const sns::Geom& g, int cbytes) {
+CUtensorMap make_field_map(void* base, int nf, int axis, const sns::Geom& g, int cbytes, int rows = 256) {
   CUtensorMap m;
   const cuuint64_t row = (cuuint64_t)g.pitch * cbytes;
   cuuint64_t dims[4] = {(cuuint64_t)2 * g.pitch, (cuuint64_t)g.n, (cuuint64_t)g.n, (cuuint64_t)nf};
   cuuint64_t strides[3] = {row, row * g.n, (cuuint64_t)g.field * cbytes};
-  const cuuint32_t br = g.n < 256 ? (cuuint32_t)g.n : 256u;
+  const cuuint32_t br = (cuuint32_t)std::min(g.n, rows);
   cuuint32_t box[4] = {(cuuint32_t)(256 / cbytes), axis == 1 ? br : 1u, axis == 2 ? br : 1u, 1u};
   cuuint32_t es[4] = {1u, 1u, 1u, 1u};
   const CUtensorMapDataType dt = cbytes == 16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
@@ -504,8 +507,8 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   mark(pm, 6, st);
   const sns::SweepArgs a = stage_args(h, stage, dt, mode, u_src);
   if (fused)
-    o->p5(h->map_work_z, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->tw, h->phase, a, h->tiles_data(),
-          prune ? h->live : nullptr, prune ? h->nlive : 0, g, h->p5_grid, h->err_word, st);
+    h->p5->run(h->map_work_z, h->map_p5_state, f_src, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->tw, h->phase, a,
+               h->tiles_data(), prune ? h->live : nullptr, prune ? h->nlive : 0, g, h->p5_grid, h->err_word, st);
   else
     o->sweep(h->work, np, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->phase, a, g, st);
   mark(pm, 7, st);
@@ -775,7 +778,7 @@ int small_grid_cap(int n, int grid) { return n <= 128 ? std::min(grid, std::max(
 bool set_launch_shape(sns_handle* h, const int* cfg) {
   int nsm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return false;
-  const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->ops->p5_grid(nsm);
+  const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
   const int tma_max = h->ops->tma_blocks_per_sm();
   if (cfg[0] < nsm || cfg[0] > nsm * tma_max || (cfg[1] != 0 && cfg[1] != x2_full) ||
       (cfg[2] != 0 && cfg[2] != p5_full))
@@ -907,7 +910,11 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
     h->tma_grid = sns::small_grid_cap(n, nsm * ops->tma_blocks_per_sm());
     h->x2_grid = ops->xpass2_grid(nsm);
-    h->p5_grid = ops->p5_grid(nsm);
+    h->p5 = sns::p5_for(n, precision);
+    if (h->p5) {
+      h->p5->init();
+      h->p5_grid = h->p5->grid(nsm);
+    }
     if (small_rule(n)) {
       h->small = sns::small_for(n, precision);
       h->small->init();
@@ -940,6 +947,7 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
       ck(cudaStreamSynchronize(h->stream), "live");
     }
     h->map_state_z = make_field_map(h->state, 6, 2, h->g, h->cbytes);
+    if (h->p5) h->map_p5_state = make_field_map(h->state, 6, 2, h->g, h->cbytes, h->p5->chunk_rows);
     h->map_work_y = make_field_map(h->work, 12, 1, h->g, h->cbytes);
     h->map_work_z = make_field_map(h->work, 12, 2, h->g, h->cbytes);
     ck(cudaMemsetAsync(h->state, 0, 6 * fb, h->stream), "memset");
@@ -1069,7 +1077,7 @@ int sns_autotune(sns_handle* h, int trial_steps, const char* cache_path, int* ou
     const std::string key = dev + " " + std::to_string(h->n) + " " + std::to_string(h->precision);
     int nsm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
-    const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->ops->p5_grid(nsm);
+    const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
     const int tma_max = h->ops->tma_blocks_per_sm();
     auto apply = [&](int tma, int x2, int p5) {
       // only shapes this handle was built for: its Nyquist partial buffer is sized for x2_full

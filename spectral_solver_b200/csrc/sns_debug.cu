@@ -3,6 +3,7 @@
 // GPU: the wait that runs out is on a barrier that nothing will complete, with a short
 // poll limit, and the error word is written by the host.
 #include "sns_kernels.cuh"
+#include "sns_p5.cuh"
 #include "sns_small.cuh"
 #include "sns_tma.cuh"
 #include "../../include/sns_b200.h"
@@ -67,6 +68,7 @@ extern "C" int sns_debug_bounds(long long* count, int* line, long long* index) {
   long long r[3] = {0, 0, 0};
   int e = sns::bounds_record(r);
   if (e == 0 && r[0] == 0) e = sns::bounds_record_small(r);  // the small grids' kernels
+  if (e == 0 && r[0] == 0) e = sns::bounds_record_p5(r);     // the fused forward-z + sweep
   if (e != 0) {
     char buf[200];
     std::snprintf(buf, sizeof buf, "sns_debug_bounds: %s", cudaGetErrorString((cudaError_t)e));

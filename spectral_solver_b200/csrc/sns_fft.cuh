@@ -6,8 +6,8 @@
 // Govindaraju et al., SC'08): butterfly j of a sequence reads elements j + r*L/R,
 // multiplies by W_{Ns*R}^{r*(j mod Ns)}, runs an R-point DFT in registers and writes
 // elements (j/Ns)*Ns*R + (j mod Ns) + r*Ns.  Output comes out in natural order, so no
-// bit reversal pass is needed.  Radices 2, 3, 4 and 8 are written out as register
-// butterflies; each length has a compile-time plan.
+// bit reversal pass is needed.  Small radices are written out as register butterflies; each
+// length has a compile-time plan.
 //
 // Twiddles come from a per-CTA shared-memory table tw[t] = exp(-2*pi*i*t/L), t < L,
 // filled from a host-computed global table (no sin/cos on the device).
@@ -333,6 +333,30 @@ __host__ __device__ __forceinline__ void dftR(C* v) {
   else static_assert(R == 2, "unsupported radix");
 }
 
+// W_32^q = exp(-2*pi*i*q/32), q < 16, as the twiddle table holds it (exp(-2*pi*i*t/512) at
+// t = 16 q, rounded from long double; the FP32 form rounds these doubles), so the radix-32
+// combine of the two-stage x pass multiplies by immediates instead of loading them.
+__host__ __device__ constexpr double w32_cos(int q) {  // cos(pi q / 16), 0 <= q <= 8
+  return q == 0 ? 1.0 : q == 1 ? 0.98078528040323043 : q == 2 ? 0.92387953251128674 : q == 3 ? 0.83146961230254524
+       : q == 4 ? 0.70710678118654757 : q == 5 ? 0.55557023301960218 : q == 6 ? 0.38268343236508978
+       : q == 7 ? 0.19509032201612828 : 0.0;
+}
+template <class C>
+__device__ __forceinline__ C w32(int q) {  // 0 <= q < 16 (unrolled: folds to immediates)
+  const double re = q <= 8 ? w32_cos(q) : -w32_cos(16 - q);
+  const double im = q <= 8 ? -w32_cos(8 - q) : -w32_cos(q - 8);
+  return cmk((real_of<C>)re, (real_of<C>)im);
+}
+
+template <class C>
+__device__ __forceinline__ C shfl2(C v, int src) {
+  return cmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+template <class C>
+__device__ __forceinline__ C shfl2_xor(C v, int m) {
+  return cmk(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+
 // ------------------------------------------------------------------------------------
 // Plans: radices in application order.  Ns grows as the product of earlier radices.
 template <int... Rs>
@@ -525,79 +549,6 @@ __device__ __forceinline__ void tfft_run(const Src0& src0, C* W, const DstG& dst
 template <int L, int DIR, int NT, int TW, class Src0, class DstG, class C>
 __device__ __forceinline__ void tile_fft(const Src0& src0, C* W, const DstG& dstg, const C* tw, int tid) {
   tfft_run<L, DIR, NT, TW>(src0, W, dstg, tw, tid, typename Plan<L>::type{});
-}
-
-// ------------------------------------------------------------------------------------
-// Tile FFT whose last stage hands each butterfly's R outputs to sink(i, v) as soon as they
-// are computed (i = the thread's butterfly index; output r of butterfly i sits at column
-// b % TW and element (j/NS)*NS*R + j%NS + r*NS, b = tid + i*NT, j = b / TW), so only R
-// values are live at a time.  Requires every thread to own whole butterflies.
-template <class P>
-struct LastRadix;
-template <int R>
-struct LastRadix<Radices<R>> {
-  static constexpr int value = R;
-};
-template <int R0, int R1, int... Rs>
-struct LastRadix<Radices<R0, R1, Rs...>> {
-  static constexpr int value = LastRadix<Radices<R1, Rs...>>::value;
-};
-
-// Shape of the last stage of a TW-column tile FFT of length L on NT threads.
-template <int L, int NT, int TW>
-struct LastStage {
-  static constexpr int R = LastRadix<typename Plan<L>::type>::value;
-  static constexpr int NS = L / R;                        // Ns of the last stage
-  static constexpr int KB = (TW * (L / R) + NT - 1) / NT;  // butterflies per thread
-};
-
-template <int L, int DIR, int NT, int TW, int Ns, int R, class Src, class Sink, class C>
-__device__ __forceinline__ void tstage_sink(const Src& src, const C* tw, int tid, Sink& sink) {
-  constexpr int kBf = L / R;
-  constexpr int kTot = TW * kBf;
-  static_assert(kTot % NT == 0, "whole butterflies per thread");
-  constexpr int kBpt = kTot / NT;
-  constexpr int kTwStep = L / (Ns * R);
-#pragma unroll
-  for (int i = 0; i < kBpt; ++i) {
-    const int b = tid + i * NT;
-    const int s = b % TW, j = b / TW;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src(s, j + r * kBf);
-    if constexpr (Ns > 1) {
-      const int k = j % Ns;
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], stage_twiddle<DIR>(tw, r * k * kTwStep));
-    }
-    dftR<R, DIR>(v);
-    sink(i, v);
-  }
-}
-
-template <int L, int DIR, int NT, int TW, int Ns, bool FIRST, class Src0, class Sink, class C, int R, int... Rest>
-__device__ __forceinline__ void tfft_sink_rec(const Src0& src0, C* W, const C* tw, int tid, Sink& sink) {
-  using WL = WLoad<TW, C>;
-  using WS = WStore<TW, C>;
-  if constexpr (sizeof...(Rest) == 0) {
-    if constexpr (FIRST) tstage_sink<L, DIR, NT, TW, Ns, R>(src0, tw, tid, sink);
-    else tstage_sink<L, DIR, NT, TW, Ns, R>(WL{W, L * TW}, tw, tid, sink);
-  } else {
-    if constexpr (FIRST) tstage<L, DIR, NT, TW, Ns, R, true, false>(src0, WS{W, L * TW}, tw, tid);
-    else tstage<L, DIR, NT, TW, Ns, R, false, false>(WL{W, L * TW}, WS{W, L * TW}, tw, tid);
-    tfft_sink_rec<L, DIR, NT, TW, Ns * R, false, Src0, Sink, C, Rest...>(src0, W, tw, tid, sink);
-  }
-}
-
-template <int L, int DIR, int NT, int TW, class Src0, class Sink, class C, int... Rs>
-__device__ __forceinline__ void tfft_sink_run(const Src0& src0, C* W, const C* tw, int tid, Sink& sink,
-                                              Radices<Rs...>) {
-  tfft_sink_rec<L, DIR, NT, TW, 1, true, Src0, Sink, C, Rs...>(src0, W, tw, tid, sink);
-}
-
-template <int L, int DIR, int NT, int TW, class Src0, class Sink, class C>
-__device__ __forceinline__ void tile_fft_sink(const Src0& src0, C* W, const C* tw, int tid, Sink& sink) {
-  tfft_sink_run<L, DIR, NT, TW>(src0, W, tw, tid, sink, typename Plan<L>::type{});
 }
 
 }  // namespace sns

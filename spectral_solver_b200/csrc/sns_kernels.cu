@@ -440,30 +440,6 @@ struct XP {
 
 __device__ __forceinline__ int pp16(int e) { return e + (e >> 4); }
 
-// W_32^q = exp(-2*pi*i*q/32), q < 16, as the twiddle table holds it (exp(-2*pi*i*t/512) at
-// t = 16 q, rounded from long double; the FP32 form rounds these doubles), so the radix-32
-// combine of the two-stage x pass multiplies by immediates instead of loading them.
-__host__ __device__ constexpr double w32_cos(int q) {  // cos(pi q / 16), 0 <= q <= 8
-  return q == 0 ? 1.0 : q == 1 ? 0.98078528040323043 : q == 2 ? 0.92387953251128674 : q == 3 ? 0.83146961230254524
-       : q == 4 ? 0.70710678118654757 : q == 5 ? 0.55557023301960218 : q == 6 ? 0.38268343236508978
-       : q == 7 ? 0.19509032201612828 : 0.0;
-}
-template <class C>
-__device__ __forceinline__ C w32(int q) {  // 0 <= q < 16 (unrolled: folds to immediates)
-  const double re = q <= 8 ? w32_cos(q) : -w32_cos(16 - q);
-  const double im = q <= 8 ? -w32_cos(8 - q) : -w32_cos(q - 8);
-  return cmk((real_of<C>)re, (real_of<C>)im);
-}
-
-template <class C>
-__device__ __forceinline__ C shfl2(C v, int src) {
-  return cmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-template <class C>
-__device__ __forceinline__ C shfl2_xor(C v, int m) {
-  return cmk(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
-}
-
 template <int N, class C>
 __global__ void __launch_bounds__(XP<N, C>::NT, XP<N, C>::MINB)
 k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase,
@@ -1210,54 +1186,6 @@ k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
 
 
 
-// The self-conjugate mode (N/2, 0, 0) for the fused P5 path: one warp sums the x pass's
-// per-CTA plane sums in a fixed order and runs the sweep on that single mode (column N/2
-// of row 0, which no P5 tile touches).
-template <int N, class C>
-__global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restrict__ gbuf,
-                                                 C* __restrict__ rhs, const double* __restrict__ nyq_part,
-                                                 int nparts, const C* __restrict__ phase, SweepArgs a0, Geom g) {
-  const SweepArgs a = resolve_step(a0);
-  constexpr int NH = N / 2;
-  const int tid = threadIdx.x;
-  const bool load_g = a.stage > 0;
-  double part[10];
-#pragma unroll
-  for (int f = 0; f < 10; ++f) {
-    double acc = 0.0;
-    for (int i = tid; i < nparts; i += 32) acc += nyq_part[f * nparts + i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    part[f] = acc;
-  }
-  if (tid != 0) return;
-  ModeIn<C, 5> in;
-#pragma unroll
-  for (int p = 0; p < 5; ++p) {
-    in.p0[p] = cmk((real_of<C>)part[2 * p], real_of<C>(0));
-    in.ps[p] = cmk((real_of<C>)part[2 * p + 1], real_of<C>(0));
-  }
-  C uu[3], gg[3], rr[3];
-  CompWord lo[3] = {0, 0, 0};
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    uu[c] = u[(long long)c * g.field + NH];
-    gg[c] = load_g ? gbuf[(long long)c * g.field + NH] : czero<C>();
-    if (a.ulo) lo[c] = a.ulo[(long long)c * g.field + NH];
-  }
-  sweep_mode(in, NH, 0, 0, N, phase[NH + 3 * N / 2], uu, gg, load_g, rr, a, lo);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (a.mode != 0) {
-      rhs[(long long)c * g.field + NH] = rr[c];
-    } else {
-      u[(long long)c * g.field + NH] = uu[c];
-      gbuf[(long long)c * g.field + NH] = gg[c];
-      if (a.ulo) a.ulo[(long long)c * g.field + NH] = lo[c];
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------
 // Rotational form (selectable; the reference computes only the conservative form).
 // omega_hat = i k x u_hat on every stored mode (the wavenumbers of the stored modes, index
@@ -1419,234 +1347,6 @@ k_sweep_rot(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
     }
     update(NH, NH, 0, 0, A, B, phase[NH + 3 * N / 2]);
   }
-}
-
-// ------------------------------------------------------------------------------------
-// P5 fused (N = 128, 256, 512): forward z pass of the 10 product fields and the whole
-// k-space sweep in one persistent kernel, so the transformed products never return to HBM.
-// A tile is (TW columns mx, one my, all mz); its 10 field tiles arrive one after another
-// through TMA (double-buffered).  The z FFT leaves each thread 8 modes in registers:
-//   P0 field of pair p -> parked in tensor memory;
-//   Ps field of pair p -> combined with the parked P0 into the dealiased value, whose -i k
-//                          contributions accumulate into r_x, r_y, r_z in tensor memory, in
-//                          the reference's order (pairs 00 01 02 11 12, the squares less u_2^2);
-//   after the 10th      -> viscous term, Leray projection, RK3 update and projection of u.
-// Tensor memory per thread: 4 blocks of CW columns (P0, r_x, r_y, r_z).
-template <int N>
-constexpr uint32_t p5_cols() { return N == 512 ? 512u : (N == 256 ? 256u : 128u); }
-template <int N>
-constexpr int nt_p5() { return nt_tma<N>(); }
-
-template <int N, class C>
-__global__ void __launch_bounds__(nt_p5<N>(), tma_minb<N>())
-k_p5(const __grid_constant__ CUtensorMap map, C* __restrict__ u, C* __restrict__ gbuf,
-     C* __restrict__ rhs, const double* __restrict__ nyq_part, int nparts, const C* __restrict__ tw,
-     const C* __restrict__ phase, SweepArgs a0, int ncb, const int* __restrict__ live, int nlive, Geom g,
-     int* err) {
-  const SweepArgs a = resolve_step(a0);
-  constexpr int NT = nt_p5<N>();
-  constexpr int BR = box_rows<N>();
-  constexpr int NBOX = N / BR;
-  constexpr int NH = N / 2;
-  constexpr int TW = tile_cols<C>();
-  constexpr uint32_t kTileBytes = 128u * N;
-  constexpr uint32_t COLS = p5_cols<N>();
-  using RO = LastStage<N, NT, TW>;
-  constexpr int WPC = tmem_words<C>();  // tensor-memory words per complex value
-  constexpr int MPT = RO::KB * RO::R;    // modes per thread
-  constexpr int CW = WPC * MPT;          // tensor-memory words per field of modes
-  constexpr int kF = 10;                 // product fields: 5 products on two grids
-  static_assert(RO::R == 4 || RO::R == 8, "last radix moves through tensor memory");
-  static_assert((NT / 32 + 3) / 4 * 4 * CW <= (int)COLS, "tensor memory budget");
-  static_assert((TW * (N / RO::R)) % NT == 0, "every thread owns whole butterflies");
-  extern __shared__ unsigned char smraw[];
-  __shared__ int s_fail;
-  __shared__ uint32_t s_tmem;
-  const uint32_t pad = (128u - (smem_u32(smraw) & 127u)) & 127u;
-  C* in0 = reinterpret_cast<C*>(smraw + pad);
-  C* in1 = in0 + TW * N;
-  C* W = in1 + TW * N;
-  C* s_tw = W + TW * N;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_tw + N);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_mbar_init();
-    s_fail = 0;
-  }
-  if (warp == 0) {
-    tmem_alloc(&s_tmem, COLS);
-    tmem_relinquish();
-  }
-  __syncthreads();
-  const uint32_t tbase = s_tmem;
-  // this thread's lane and columns: P0 park [0, CW), r_x, r_y, r_z at CW * (1 + c)
-  const uint32_t tq = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * 4 * CW);
-  const bool load_g = a.stage > 0;
-
-  // tiles (cb, my), index my * ncb + cb (at most N x (N/16 + 1): 32-bit); with a live list
-  // only the listed ones
-  const long long ntiles = live ? (long long)nlive : (long long)ncb * N;
-  auto tile_of = [&](long long t, int& cb, int& my) {
-    const int idx = live ? __ldg(&live[SNS_IDX(t, nlive)]) : (int)t;
-    my = idx / ncb;
-    cb = idx - my * ncb;
-  };
-  const long long mytiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const long long nunits = kF * mytiles;
-  auto issue = [&](long long ul, int b) {
-    const long long t = blockIdx.x + (ul / kF) * gridDim.x;
-    const int f = (int)(ul % kF);
-    int cb, my;
-    tile_of(t, cb, my);
-    C* dst = b ? in1 : in0;
-    mbar_arrive_expect_tx(&bars[b], kTileBytes);
-#pragma unroll
-    for (int k = 0; k < NBOX; ++k) tma_load_4d(dst + k * BR * TW, &map, &bars[b], cb * 2 * TW, my, k * BR, f);
-  };
-  if (tid == 0) {
-    if (nunits > 0) issue(0, 0);
-    if (nunits > 1) issue(1, 1);
-  }
-  for (long long ul = 0; ul < nunits; ++ul) {
-    const int b = (int)(ul & 1);
-    const uint32_t parity = (uint32_t)(ul >> 1) & 1u;
-    if (tid == 0 && !mbar_wait_bounded(&bars[b], parity)) s_fail = 1;
-    __syncthreads();
-    if (s_fail) {
-      if (tid == 0) {
-        atomicExch(err, kErrTmaTimeout);
-        (void)mbar_wait_bounded(&bars[b ^ 1], (uint32_t)((ul + 1) >> 1) & 1u);
-      }
-      if (warp == 0) tmem_dealloc(tbase, COLS);
-      return;
-    }
-    (void)mbar_try_wait(&bars[b], parity);
-    const C* IN = b ? in1 : in0;
-    const long long t = blockIdx.x + (ul / kF) * gridDim.x;
-    const int f = (int)(ul % kF);
-    int cb, my;
-    tile_of(t, cb, my);
-    const int mx0 = cb * TW;
-    // Each radix butterfly of the last stage hands its R modes to the sink: column
-    // s = b % TW (b = tid + i*NT), z index (j/NS)*NS*R + j%NS + r*NS with j = b / TW; mode
-    // q = i*R + r of this thread owns tensor-memory columns [WPC*q, WPC*(q + 1)) of every block.
-    const int iy = signed_mode(my, N);
-    const int p = f >> 1;
-    const int ca = (p >= 3) + (p >= 5), cbp = p < 3 ? p : (p < 5 ? p - 2 : 2);
-    auto sink = [&](int i, C* v) {
-      constexpr int R = RO::R, NS = RO::NS;
-      const int bb = tid + i * NT, s_ = bb % TW, j = bb / TW;
-      const uint32_t col = (uint32_t)(WPC * R * i);
-      // tensor-memory columns of this thread's blocks stay inside the allocation
-      (void)SNS_IDX((warp >> 2) * 4 * CW + 4 * CW - 1, (long long)COLS);
-      (void)SNS_IDX(col + WPC * R - 1, (long long)CW);
-      if ((f & 1) == 0) {
-        tmem_st<R>(tq + col, v);  // park P0 of this pair
-        return;
-      }
-      const int ix = mx0 + s_;
-      int izs[R];
-      {
-        C p0[R];
-        tmem_ld<R>(tq + col, p0);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          izs[r] = signed_mode((j / NS) * NS * R + (j % NS) + r * NS, N);
-          const bool keep = 4LL * (ix * ix + iy * iy + izs[r] * izs[r]) <= (long long)N * N;
-          v[r] = pair_value(p0[r], v[r], __ldg(&phase[SNS_IDX(ix + iy + izs[r] + 3 * N / 2, 3 * N + 1)]), keep,
-                            a.dealias);
-        }
-      }
-      // r_a += -i k_b value; r_b += -i k_a value (a != b); the first touch starts the sum
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        if (side == 1 && ca == cbp) break;
-        const int dst = side == 0 ? ca : cbp, kc = side == 0 ? cbp : ca;
-        const bool first = side == 0 ? (p == 0) : (p == 1 || p == 2);  // r_x at 00, r_y at 01, r_z at 02
-        const uint32_t ta = tq + (uint32_t)(CW * (1 + dst)) + col;
-        C r[R];
-        if (!first) tmem_ld<R>(ta, r);
-#pragma unroll
-        for (int rr = 0; rr < R; ++rr) {
-          const int kk = kc == 0 ? ix : (kc == 1 ? iy : izs[rr]);
-          const C c = minus_i_k(v[rr], kk);
-          r[rr] = first ? c : cadd(r[rr], c);
-        }
-        tmem_st<R>(ta, r);
-      }
-    };
-    tile_fft_sink<N, -1, NT, TW>([&](int s_, int e_) { return IN[SNS_IDX(e_ * TW + s_, TW * N)]; }, W, s_tw, tid,
-                                 sink);
-    tmem_wait_st();
-    __syncthreads();  // IN[b] and W are free again
-    if (tid == 0 && ul + 2 < nunits) issue(ul + 2, b);
-    auto mode_s = [&](int q) { return (tid + (q / RO::R) * NT) % TW; };
-    auto mode_e = [&](int q) {
-      const int j = (tid + (q / RO::R) * NT) / TW, r = q % RO::R;
-      return (j / RO::NS) * RO::NS * RO::R + (j % RO::NS) + r * RO::NS;
-    };
-    if (f == kF - 1) {
-      // Two-deep software pipeline over this thread's modes: the u, g loads of mode q + 1
-      // are in flight while mode q is combined and stored (different modes, no aliasing).
-      C uu_n[3], gg_n[3];
-      CompWord lo_n[3] = {0, 0, 0};
-      auto load_mode = [&](int q, C* uu, C* gg, CompWord* lo) {
-        const long long idx = SNS_IDX(((long long)mode_e(q) * N + my) * g.pitch + mx0 + mode_s(q), g.field);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          uu[c] = u[(long long)c * g.field + idx];
-          gg[c] = load_g ? gbuf[(long long)c * g.field + idx] : czero<C>();
-          if (a.ulo) lo[c] = a.ulo[(long long)c * g.field + idx];
-        }
-      };
-      load_mode(0, uu_n, gg_n, lo_n);
-#pragma unroll 1
-      for (int q = 0; q < MPT; ++q) {
-        C uu[3], gg[3], rr[3];
-        CompWord lo[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          uu[c] = uu_n[c];
-          gg[c] = gg_n[c];
-          lo[c] = lo_n[c];
-        }
-        if (q + 1 < MPT) load_mode(q + 1, uu_n, gg_n, lo_n);
-        C r3[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r3[c] = tmem_ld1<C>(tq + CW * (1 + c) + WPC * q);
-        const int ix = mx0 + mode_s(q);
-        if (ix >= NH) continue;
-        const int ez = mode_e(q);
-        const int iz = signed_mode(ez, N);
-        const long long row = (long long)ez * N + my;
-        const long long idx = SNS_IDX(row * g.pitch + ix, g.field);
-        finish_mode(r3, ix, iy, iz, N, uu, gg, load_g, rr, a, lo);
-        const bool nyq_zero = ix == 0 && row != 0;  // plane mx = N/2 is zero off (N/2,0,0)
-        const long long inq = SNS_IDX(row * g.pitch + NH, g.field);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (a.mode != 0) {
-            rhs[(long long)c * g.field + idx] = rr[c];
-            if (nyq_zero) rhs[(long long)c * g.field + inq] = czero<C>();
-          } else {
-            u[(long long)c * g.field + idx] = uu[c];
-            gbuf[(long long)c * g.field + idx] = gg[c];
-            if (a.ulo) a.ulo[(long long)c * g.field + idx] = lo[c];
-            if (nyq_zero) {
-              u[(long long)c * g.field + inq] = czero<C>();
-              gbuf[(long long)c * g.field + inq] = czero<C>();
-              if (a.ulo) a.ulo[(long long)c * g.field + inq] = 0u;
-            }
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, COLS);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2084,41 +1784,6 @@ struct Launch {
                                                                   nyq_part, F(tw2), g, err);
     }
   }
-  static void p5(const CUtensorMap& map, void* u, void* gbuf, void* rhs, const double* nyq_part, int nparts,
-                 const void* tw, const void* phase, SweepArgs a, int ncb, const int* live, int nlive, Geom g,
-                 int grid, int* err, cudaStream_t st) {
-    if constexpr (N == 128 || N == 256 || N == 512) {
-      k_nyq_mode<N, C><<<1, 32, 0, st>>>(F(u), F(gbuf), F(rhs), nyq_part, nparts, F(phase), a, g);
-      k_p5<N, C><<<grid, nt_p5<N>(), tma_smem<N, C>(), st>>>(map, F(u), F(gbuf), F(rhs), nyq_part, nparts, F(tw),
-                                                              F(phase), a, ncb, live, nlive, g, err);
-    }
-  }
-  // Persistent grid of the fused P5 (0: this size runs forward z + sweep as two kernels).
-  // The runtime's occupancy query reports one CTA per SM for this tensor-memory kernel
-  // whatever its allocation, so residency is computed from the kernel's own limits: shared
-  // memory, registers, threads, and its tensor-memory columns (512 per SM).
-  static int p5_grid(int nsm) {
-    if constexpr (N == 128 || N == 256 || N == 512) {
-      int dev = 0, smem_sm = 0, smem_rsv = 0, regs_sm = 0, thr_sm = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-      cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-      cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-      cudaDeviceGetAttribute(&thr_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev);
-      cudaFuncAttributes fa{};
-      cudaFuncGetAttributes(&fa, k_p5<N, C>);
-      const long long smem_cta = (long long)tma_smem<N, C>() + fa.sharedSizeBytes + smem_rsv;
-      const long long regs_cta = (long long)((fa.numRegs + 7) / 8 * 8) * nt_p5<N>();
-      int nb = 512 / (int)p5_cols<N>();
-      if (smem_cta > 0) nb = (int)std::min<long long>(nb, smem_sm / smem_cta);
-      if (regs_cta > 0) nb = (int)std::min<long long>(nb, regs_sm / regs_cta);
-      nb = std::min(nb, thr_sm / nt_p5<N>());
-      return nsm * (nb < 1 ? 1 : nb);
-    } else {
-      (void)nsm;
-      return 0;
-    }
-  }
   // Persistent grid of the two-stage x pass (0: this size uses the generic x pass).
   static int xpass2_grid(int nsm) {
     if constexpr ((N == 128 || N == 256 || N == 512) && std::is_same_v<C, float2>) {
@@ -2217,7 +1882,6 @@ struct Launch {
       set_smem(k_xpass_w<N, true>, XW<N>::smem);
     }
     else if constexpr (N == 256 || N == 512) set_smem(k_xpass2<N, C>, XP<N, C>::smem);
-    if constexpr (N == 128 || N == 256 || N == 512) set_smem(k_p5<N, C>, tma_smem<N, C>());
     set_smem(k_yz_tma<N, 2, +1, 1, C>, tma_smem<N, C>());
     set_smem(k_yz_tma<N, 1, -1, 0, C>, tma_smem<N, C>());
     set_smem(k_yz_tma<N, 1, +1, 0, C>, tma_smem<N, C>());
@@ -2238,7 +1902,7 @@ struct Launch {
   static const Ops* table() {
     static const Ops ops = {N,  (int)sizeof(C), kT, init, zpass_inv_phase, ypass, zpass, xpass_products, nyq_reduce,
                             sweep, xpass_r2c, xpass_c2r, xpass_diag, yz_tma, tma_blocks_per_sm, xpass2, xpass2_grid,
-                            p5, p5_grid, omega_hat, xpass_rot, sweep_rot, xpass_diag2};
+                            omega_hat, xpass_rot, sweep_rot, xpass_diag2};
     return &ops;
   }
 };

@@ -62,22 +62,25 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
 // value never reaches the rounding boundary of hi: round-to-nearest(hi + lo) == hi), and a
 // decoded pair encodes back to the same pair, so states round-trip exactly through the host.
 // The precision kept is about ulp(hi)/255, 2^-32 relative, against 2^-24 for FP32 alone.
-// ulp(hi) = 2^(E - 150) and its inverse, E the biased exponent of hi (at least 1), built from
-// the exponent bits: no division anywhere in the encoding.
+// ulp(hi) = 2^(E - 150), E the biased exponent of hi (at least 1): the factors between a
+// remainder and its q are 255 and 1/255 with their exponent moved, one multiplication each way.
 __device__ __forceinline__ int comp_exp(float hi) {
   const int e = (int)((__float_as_uint(hi) >> 23) & 0xffu);
   return e > 0 ? e : 1;
 }
-__device__ __forceinline__ double pow2(int k) { return __longlong_as_double((long long)(k + 1023) << 52); }
+// c * 2^k for a normal c, by its exponent bits
+__device__ __forceinline__ double scaled(double c, int k) {
+  return __hiloint2double(__double2hiint(c) + (k << 20), __double2loint(c));
+}
 __device__ __forceinline__ double comp_part(float hi, int q) {
-  return (double)q * pow2(comp_exp(hi) - 150) * (1.0 / 255.0);
+  return (double)q * scaled(1.0 / 255.0, comp_exp(hi) - 150);
 }
 __device__ __forceinline__ int comp_q(double U, float hi) {
-  const double r = (U - (double)hi) * pow2(150 - comp_exp(hi)) * 255.0;  // U - hi exact; |r| <= 127.5
+  const double r = (U - (double)hi) * scaled(255.0, 150 - comp_exp(hi));  // U - hi exact; |r| <= 127.5
   // toward zero, after a nudge of 1e-6 away from it: a decoded remainder (an integer up to
   // FP64 round-off) comes back as the same integer, and the bounds 63.75 (hi a power of two,
   // U below it) and 127.5 are never crossed
-  return (int)trunc(r + copysign(1.0e-6, r));
+  return (int)(r + copysign(1.0e-6, r));
 }
 __device__ __forceinline__ double2 comp_decode(float2 hi, CompWord lo) {
   const int qr = (int)(int8_t)(lo & 0xffu), qi = (int)(int8_t)(lo >> 8);
@@ -136,6 +139,11 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
   const int m2 = ix * ix + iy * iy + iz * iz;
   const bool keep = 4LL * m2 <= (long long)n * n;
   const double k2 = (double)m2;
+  // the wavenumber in the form's precision (exact), and 1/k^2 formed once, in FP64
+  using RT = real_of<C>;
+  const RT kx = (RT)ix, ky = (RT)iy, kz = (RT)iz;
+  const double inv = 1.0 / k2;
+  const RT rinv = (RT)inv;
   if (a.mode == 2) {  // nonlinear term only: masked, neither viscous term nor projection
     rr[0] = r[0];
     rr[1] = r[1];
@@ -144,14 +152,14 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
   }
   if (!a.visc_if) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] = csub(r[c], cscale(uu[c], a.nu * k2));
+    for (int c = 0; c < 3; ++c) r[c] = csub(r[c], cscale(uu[c], (RT)(a.nu * k2)));
   }
   if (k2 > 0.0 && keep) {
-    const C dot = cadd(cadd(cscale(r[0], (double)ix), cscale(r[1], (double)iy)), cscale(r[2], (double)iz));
-    const C factor = cscale(dot, 1.0 / k2);
-    r[0] = csub(r[0], cscale(factor, (double)ix));
-    r[1] = csub(r[1], cscale(factor, (double)iy));
-    r[2] = csub(r[2], cscale(factor, (double)iz));
+    const C dot = cadd(cadd(cscale(r[0], kx), cscale(r[1], ky)), cscale(r[2], kz));
+    const C factor = cscale(dot, rinv);
+    r[0] = csub(r[0], cscale(factor, kx));
+    r[1] = csub(r[1], cscale(factor, ky));
+    r[2] = csub(r[2], cscale(factor, kz));
   } else {
     r[0] = r[1] = r[2] = czero<C>();
   }
@@ -181,10 +189,10 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
         }
       }
       if (k2 > 0.0 && keep) {
-        const double2 dot = make_double2((U[0].x * ix + U[1].x * iy) + U[2].x * iz,
-                                         (U[0].y * ix + U[1].y * iy) + U[2].y * iz);
-        const double2 factor = make_double2(dot.x * (1.0 / k2), dot.y * (1.0 / k2));
         const double kv[3] = {(double)ix, (double)iy, (double)iz};
+        const double2 dot = make_double2((U[0].x * kv[0] + U[1].x * kv[1]) + U[2].x * kv[2],
+                                         (U[0].y * kv[0] + U[1].y * kv[1]) + U[2].y * kv[2]);
+        const double2 factor = make_double2(dot.x * inv, dot.y * inv);
 #pragma unroll
         for (int c = 0; c < 3; ++c) uu[c] = comp_encode(make_double2(U[c].x - factor.x * kv[c],
                                                                      U[c].y - factor.y * kv[c]), &lo[c]);
@@ -213,11 +221,11 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
     }
   }
   if (k2 > 0.0 && keep) {
-    const C dot = cadd(cadd(cscale(uu[0], (double)ix), cscale(uu[1], (double)iy)), cscale(uu[2], (double)iz));
-    const C factor = cscale(dot, 1.0 / k2);
-    uu[0] = csub(uu[0], cscale(factor, (double)ix));
-    uu[1] = csub(uu[1], cscale(factor, (double)iy));
-    uu[2] = csub(uu[2], cscale(factor, (double)iz));
+    const C dot = cadd(cadd(cscale(uu[0], kx), cscale(uu[1], ky)), cscale(uu[2], kz));
+    const C factor = cscale(dot, rinv);
+    uu[0] = csub(uu[0], cscale(factor, kx));
+    uu[1] = csub(uu[1], cscale(factor, ky));
+    uu[2] = csub(uu[2], cscale(factor, kz));
   } else {
     uu[0] = uu[1] = uu[2] = czero<C>();
   }
