@@ -575,6 +575,121 @@ k_xsmall(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
   }
 }
 
+// ------------------------------------------------------------------------------------
+// Forward transform of one real field to the reference's full layout, two launches (FP64,
+// N <= 64): x and y on a whole z plane per CTA, then z with the mirror half written from the
+// same registers.
+template <int N>
+struct FT {
+  using S = XYSplit<N>;
+  using Z = ZSplit<N>;
+  static constexpr int NH = N / 2, NC = NH + 1;
+  static constexpr int NT = N <= 16 ? 64 : 256;
+  static constexpr int SEQ = NH * S::SLOTS;   // N / 2 packed row pairs
+  static constexpr int COL = S::SLOTS * NC;   // the plane's columns 0 .. N/2
+  static constexpr size_t smem_plane = (size_t)(N + SEQ + COL) * sizeof(double2);
+  static constexpr int TW = 4, NCB = (NC + TW - 1) / TW, NTZ = N <= 16 ? 32 : 64;
+  static constexpr size_t smem_z = (size_t)(N + Z::SLOTS * TW) * sizeof(double2);
+};
+
+// One z plane: real rows (two per complex sequence), x, the two rows' half spectra taken
+// apart, y; work rows (z, ky) of g.pitch values.  grid N.
+template <int N>
+__global__ void __launch_bounds__(FT<N>::NT)
+k_plane_r2c(const double* __restrict__ in, double2* __restrict__ work, const double2* __restrict__ tw, Geom g) {
+  using T = FT<N>;
+  using S = typename T::S;
+  constexpr int NT = T::NT, NH = T::NH, NC = T::NC, RP = S::SLOTS;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* const s_tw = reinterpret_cast<double2*>(smraw);
+  double2* const seq = s_tw + N;
+  double2* const col = seq + T::SEQ;
+  const int tid = threadIdx.x, z = blockIdx.x;
+  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  for (int e = tid; e < NH * N; e += NT) {
+    const int x = e % N, q = e / N;
+    const double* r = in + ((long long)z * N + 2 * q) * N + x;
+    seq[SNS_IDX(q * RP + S::natural(x), T::SEQ)] = make_double2(r[0], r[N]);
+  }
+  __syncthreads();
+  for (int b = tid; b < NH * S::R2; b += NT) {
+    const int n2 = b % S::R2, q = b / S::R2;
+    fwd1<S, -1>(seq, [&](int sl) { return q * RP + sl; }, s_tw, n2, T::SEQ);
+  }
+  __syncthreads();
+  for (int b = tid; b < NH * S::R1; b += NT) {
+    const int k1 = b % S::R1, q = b / S::R1;
+    auto at = [&](int sl) { return q * RP + sl; };
+    double2 v[S::R2];
+    fwd2<S, -1>(seq, at, k1, T::SEQ, v);
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) seq[SNS_IDX(at(S::slot(k1, k2)), T::SEQ)] = v[k2];
+  }
+  __syncthreads();
+  for (int e = tid; e < NH * NC; e += NT) {
+    const int k = e % NC, q = e / NC, m = k == 0 ? 0 : N - k;
+    const double2 Zk = seq[SNS_IDX(q * RP + S::slot(k % S::R1, k / S::R1), T::SEQ)];
+    const double2 Zm = seq[SNS_IDX(q * RP + S::slot(m % S::R1, m / S::R1), T::SEQ)];
+    col[SNS_IDX(S::natural(2 * q) * NC + k, T::COL)] = make_double2(0.5 * (Zk.x + Zm.x), 0.5 * (Zk.y - Zm.y));
+    col[SNS_IDX(S::natural(2 * q + 1) * NC + k, T::COL)] = make_double2(0.5 * (Zk.y + Zm.y), -0.5 * (Zk.x - Zm.x));
+  }
+  __syncthreads();
+  for (int b = tid; b < NC * S::R2; b += NT) {
+    const int c = b % NC, n2 = b / NC;
+    fwd1<S, -1>(col, [&](int sl) { return sl * NC + c; }, s_tw, n2, T::COL);
+  }
+  __syncthreads();
+  for (int b = tid; b < NC * S::R1; b += NT) {
+    const int c = b % NC, k1 = b / NC;
+    double2 v[S::R2];
+    fwd2<S, -1>(col, [&](int sl) { return sl * NC + c; }, k1, T::COL, v);
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2)
+      work[SNS_IDX(((long long)z * N + k1 + S::R1 * k2) * g.pitch + c, g.field)] = v[k2];
+  }
+}
+
+// z of TW columns at one my, out to the full layout [z][y][x]: mode m and, for 0 < mx < N/2, its
+// conjugate mirror.  grid (NCB, N).
+template <int N>
+__global__ void __launch_bounds__(FT<N>::NTZ)
+k_zfull(const double2* __restrict__ work, double2* __restrict__ full, const double2* __restrict__ tw, Geom g) {
+  using T = FT<N>;
+  using S = typename T::Z;
+  constexpr int NT = T::NTZ, TW = T::TW, LIM = S::SLOTS * TW;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* const s_tw = reinterpret_cast<double2*>(smraw);
+  double2* const buf = s_tw + N;
+  const int tid = threadIdx.x, mx0 = blockIdx.x * TW, my = blockIdx.y;
+  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  for (int e = tid; e < N * TW; e += NT) {  // (columns past N/2: the row's padding, never stored)
+    const int s = e % TW, row = e / TW;
+    copy_async<1>(buf + SNS_IDX(S::natural(row) * TW + s, LIM),
+                  work + SNS_IDX(((long long)row * N + my) * g.pitch + mx0 + s, g.field));
+  }
+  copies_wait();
+  __syncthreads();
+  for (int b = tid; b < TW * S::R2; b += NT) {
+    const int s = b % TW, n2 = b / TW;
+    fwd1<S, -1>(buf, [&](int q) { return q * TW + s; }, s_tw, n2, LIM);
+  }
+  __syncthreads();
+  for (int b = tid; b < TW * S::R1; b += NT) {
+    const int s = b % TW, k1 = b / TW, mx = mx0 + s;
+    double2 v[S::R2];
+    fwd2<S, -1>(buf, [&](int q) { return q * TW + s; }, k1, LIM, v);
+    if (mx > N / 2) continue;
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) {
+      const int z = k1 + S::R1 * k2;
+      full[SNS_IDX(((long long)z * N + my) * N + mx, (long long)N * N * N)] = v[k2];
+      if (mx > 0 && mx < N / 2)
+        full[SNS_IDX(((long long)(z ? N - z : 0) * N + (my ? N - my : 0)) * N + N - mx, (long long)N * N * N)] =
+            cconj(v[k2]);
+    }
+  }
+}
+
 template <class K>
 void allow_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -594,6 +709,19 @@ struct Small {
     allow_smem(k_xsmall<N, C, true>, XT<N, C>::smem);
     allow_smem(k_zphase<N, C>, Z::smem_phase);
     allow_smem(k_zsweep<N, C>, Z::smem_sweep);
+  }
+  static void forward_init() {
+    if constexpr (N <= 64) {
+      allow_smem(k_plane_r2c<N>, FT<N>::smem_plane);
+      allow_smem(k_zfull<N>, FT<N>::smem_z);
+    }
+  }
+  static void forward(const double* phys, void* work, void* full, const void* tw, Geom g, cudaStream_t st) {
+    if constexpr (N <= 64 && sizeof(C) == 16) {
+      using T = FT<N>;
+      k_plane_r2c<N><<<N, T::NT, T::smem_plane, st>>>(phys, F(work), F(tw), g);
+      k_zfull<N><<<dim3(T::NCB, N), T::NTZ, T::smem_z, st>>>(F(work), F(full), F(tw), g);
+    }
   }
   static void zphase(const void* u, void* work, const void* phase, const void* tw, double scale, int clean, Geom g,
                      cudaStream_t st) {
@@ -620,7 +748,9 @@ struct Small {
                                                                   F(phase), F(tw), a, prune, emit, scale, g);
   }
   static const SmallOps* table() {
-    static const SmallOps ops = {XT<N, C>::GRID, init, zphase, yinv, xpass, yfwd, zsweep};
+    static const SmallOps ops = {XT<N, C>::GRID, init, zphase, yinv, xpass, yfwd, zsweep,
+                                 N <= 64 && sizeof(C) == 16 ? forward_init : nullptr,
+                                 N <= 64 && sizeof(C) == 16 ? forward : nullptr};
     return &ops;
   }
 };

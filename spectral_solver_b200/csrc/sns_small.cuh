@@ -25,6 +25,10 @@ struct SmallOps {
   // next stage's zphase
   void (*zsweep)(void* work, void* u, void* gbuf, void* rhs, const double* part, int nparts, const void* phase,
                  const void* tw, SweepArgs a, int prune, int emit, double scale, Geom g, cudaStream_t st);
+  // FP64, N <= 64 (null otherwise): forward transform of a real field [z][y][x] to the full
+  // complex layout through one half field of scratch; forward_init once per device before it
+  void (*forward_init)();
+  void (*forward)(const double* phys, void* work, void* full, const void* tw, Geom g, cudaStream_t st);
 };
 
 // nullptr for sizes without these kernels
