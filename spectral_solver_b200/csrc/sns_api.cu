@@ -434,20 +434,22 @@ void run_stage_small(sns_handle* h, char* u_src, char* g_buf, int stage, double 
   cudaStream_t st = h->stream;
   const int clean = mode == 0 && sphere_known(h, stage) ? 1 : 0;
   const int emit = mode == 0 && stage < 2 ? 1 : 0;
+  const int rot = h->form;
   mark(pm, 0, st);
-  if (!h->z_ready) o->zphase(u_src, h->work, h->phase, h->tw, h->inv_size(), clean, h->g, st);
+  if (!h->z_ready) o->zphase(u_src, h->work, h->phase, h->tw, h->inv_size(), clean, rot, h->g, st);
   mark(pm, 1, st);
-  if (!h->y_ready) o->yinv(h->work, h->tw, 2, clean, h->g, st);
+  if (!h->y_ready) o->yinv(h->work, h->tw, rot ? 4 : 2, clean, h->g, st);
   mark(pm, 2, st);
-  o->xpass(h->work, u_src, h->phase, h->tw, h->inv_size(), h->nyq_part, 0, h->g, st);
+  if (rot) o->xrot(h->work, u_src, h->phase, h->tw, h->inv_size(), h->nyq_part, h->g, st);
+  else o->xpass(h->work, u_src, h->phase, h->tw, h->inv_size(), h->nyq_part, 0, h->g, st);
   mark(pm, 3, st);
   mark(pm, 4, st);
-  o->yfwd(h->work, h->tw, h->g, st);
+  o->yfwd(h->work, h->tw, rot, h->g, st);
   mark(pm, 5, st);
   mark(pm, 6, st);
   h->y_ready = false;
-  o->zsweep(h->work, u_src, g_buf, rhs_out, h->nyq_part, o->nparts, h->phase, h->tw, stage_args(h, stage, dt, mode, u_src), clean,
-            emit, h->inv_size(), h->g, st);
+  o->zsweep(h->work, u_src, g_buf, rhs_out, h->nyq_part, rot ? o->rparts : o->nparts, h->phase, h->tw,
+            stage_args(h, stage, dt, mode, u_src), clean, emit, rot, h->inv_size(), h->g, st);
   mark(pm, 7, st);
   h->z_ready = emit != 0;
 }
@@ -457,6 +459,12 @@ void run_stage_small(sns_handle* h, char* u_src, char* g_buf, int stage, double 
 // gradient's difference that the projection removes), mode 2 on all 6, as separate kernels.
 void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, int mode, char* rhs_out,
                PassMarks* pm = nullptr) {
+  // (the rotational form has one nonlinear term for every mode)
+  if (h->small && h->nyq_clean && (h->form == 1 || mode != 2)) {
+    run_stage_small(h, u_src, g_buf, stage, dt, mode, rhs_out, pm);
+    return;
+  }
+  h->z_ready = h->y_ready = false;
   if (h->form == 1) {
     run_stage_rot(h, u_src, g_buf, stage, dt, mode, rhs_out, pm);
     return;
@@ -467,11 +475,6 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   const int tiles_in = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   const int f_src = (int)((size_t)(u_src - h->state) / h->fbytes);  // u (0) or the g slot (3)
   const int np = mode == 2 ? 6 : 5;
-  if (h->small && np == 5 && h->nyq_clean) {
-    run_stage_small(h, u_src, g_buf, stage, dt, mode, rhs_out, pm);
-    return;
-  }
-  h->z_ready = false;
   const bool fused = h->p5_grid > 0 && np == 5;
   // Sphere pruning (RK update with the fused P5 only).  A column-block tile (my, cb) outside
   // the disk 4 ((cb * TW)^2 + my^2) <= N^2 holds only modes outside the sphere: u is zero
@@ -646,7 +649,7 @@ int velocity_partials(sns_handle* h, bool both) {
   const sns::Geom& g = h->g;
   if (h->small && h->nyq_clean) {
     const int clean = sphere_known(h, 0) ? 1 : 0;
-    h->small->zphase(h->u(), h->work, h->phase, h->tw, h->inv_size(), clean, g, h->stream);
+    h->small->zphase(h->u(), h->work, h->phase, h->tw, h->inv_size(), clean, 0, g, h->stream);
     h->small->yinv(h->work, h->tw, both ? 2 : 1, clean, g, h->stream);
     h->small->xpass(h->work, h->u(), h->phase, h->tw, h->inv_size(), h->partials, 1, g, h->stream);
     h->y_ready = both;
@@ -919,7 +922,7 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
       h->small = sns::small_for(n, precision);
       h->small->init();
     }
-    const int nparts = std::max(std::max(1, h->x2_grid), h->small ? h->small->nparts : 1);
+    const int nparts = std::max(std::max(1, h->x2_grid), h->small ? std::max(h->small->nparts, h->small->rparts) : 1);
     alloc((void**)&h->nyq_part, (size_t)12 * nparts * sizeof(double));
     alloc((void**)&h->tw2, (size_t)n * h->cbytes);
     {

@@ -117,8 +117,7 @@ struct ZT {
   static constexpr int NT = N <= 32 ? 160 : (N <= 64 ? 320 : 256);
   static constexpr int MINB = NT == 256 ? 2 : (NT == 320 ? 2 : 1);
   static constexpr int FP = S::SLOTS * TW;  // one field's tile
-  static constexpr size_t smem_sweep = (size_t)(N + 10 * FP) * sizeof(C);
-  static constexpr size_t smem_phase = (size_t)(N + 6 * FP) * sizeof(C);
+  static constexpr size_t smem(int fields) { return (size_t)(N + fields * FP) * sizeof(C); }
   static constexpr int MODES = (N * TW + NT - 1) / NT;  // per thread in the sweep
 };
 
@@ -133,14 +132,29 @@ __device__ __forceinline__ void both_grids(C u, int mx, int iy, int iz, const C*
             : cmul(*U, __ldg(&phase[SNS_IDX(mx + signed_mode(iy, N) + signed_mode(iz, N) + 3 * N / 2, 3 * N + 1)]));
 }
 
-// Inverse z of u on both grids: work fields 2c, 2c + 1.  grid (NCB, N).
-template <int N, class C>
+// Vorticity i k x u_hat at one mode (index N/2 -> wavenumber +N/2).
+template <class C>
+__device__ __forceinline__ void vorticity(const C u[3], int ix, int iy, int iz, C w[3]) {
+  using RT = real_of<C>;
+  const RT kx = (RT)ix, ky = (RT)iy, kz = (RT)iz;
+  const C a = cmk(ky * u[2].x - kz * u[1].x, ky * u[2].y - kz * u[1].y);
+  const C b = cmk(kz * u[0].x - kx * u[2].x, kz * u[0].y - kx * u[2].y);
+  const C c = cmk(kx * u[1].x - ky * u[0].x, kx * u[1].y - ky * u[0].y);
+  w[0] = cmk(-a.y, a.x);
+  w[1] = cmk(-b.y, b.x);
+  w[2] = cmk(-c.y, c.x);
+}
+
+// Inverse z of u on both grids: work fields 2c, 2c + 1; ROT (the rotational form): of the
+// vorticity too, fields 6 + 2c, 7 + 2c.  grid (NCB, N).
+template <int N, class C, bool ROT>
 __global__ void __launch_bounds__(ZT<N, C>::NT)
 k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ phase, const C* __restrict__ tw,
          double scale, int clean, Geom g) {
   using Z = ZT<N, C>;
   using S = typename Z::S;
-  constexpr int TW = Z::TW, NT = Z::NT, FP = Z::FP, LIM = 6 * FP, NH = Z::NH;
+  constexpr int NQ = ROT ? 12 : 6;  // sequences per column
+  constexpr int TW = Z::TW, NT = Z::NT, FP = Z::FP, LIM = NQ * FP, NH = Z::NH;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* const s_tw = reinterpret_cast<C*>(smraw);
   C* const buf = s_tw + N;
@@ -148,24 +162,44 @@ k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ ph
   if (clean && dead_pencil<N>(mx0, signed_mode(my, N))) return;  // never read (k_ysmall)
   const real_of<C> sc = (real_of<C>)scale;
   for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
-  for (int e = tid; e < 3 * N * TW; e += NT) {
-    const int s = e % TW, row = (e / TW) % N, c = e / (TW * N);
-    const int mx = mx0 + s;
-    C U = czero<C>(), V = czero<C>();
-    if (mx < NH)
-      both_grids<N>(u[SNS_IDX(c * g.field + ((long long)row * N + my) * g.pitch + mx, 3 * g.field)], mx, my, row,
-                    phase, sc, &U, &V);
-    const int at = S::natural(row) * TW + s;
-    buf[SNS_IDX(2 * c * FP + at, LIM)] = U;
-    buf[SNS_IDX((2 * c + 1) * FP + at, LIM)] = V;
+  if constexpr (ROT) {
+    for (int e = tid; e < N * TW; e += NT) {
+      const int s = e % TW, row = e / TW, mx = mx0 + s, at = S::natural(row) * TW + s;
+      C f[6] = {};
+      if (mx < NH) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          f[c] = u[SNS_IDX(c * g.field + ((long long)row * N + my) * g.pitch + mx, 3 * g.field)];
+        vorticity(f, mx, signed_mode(my, N), signed_mode(row, N), f + 3);
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        C U = czero<C>(), V = czero<C>();
+        if (mx < NH) both_grids<N>(f[q], mx, my, row, phase, sc, &U, &V);
+        buf[SNS_IDX(2 * q * FP + at, LIM)] = U;
+        buf[SNS_IDX((2 * q + 1) * FP + at, LIM)] = V;
+      }
+    }
+  } else {
+    for (int e = tid; e < 3 * N * TW; e += NT) {
+      const int s = e % TW, row = (e / TW) % N, c = e / (TW * N);
+      const int mx = mx0 + s;
+      C U = czero<C>(), V = czero<C>();
+      if (mx < NH)
+        both_grids<N>(u[SNS_IDX(c * g.field + ((long long)row * N + my) * g.pitch + mx, 3 * g.field)], mx, my, row,
+                      phase, sc, &U, &V);
+      const int at = S::natural(row) * TW + s;
+      buf[SNS_IDX(2 * c * FP + at, LIM)] = U;
+      buf[SNS_IDX((2 * c + 1) * FP + at, LIM)] = V;
+    }
   }
   __syncthreads();
-  for (int b = tid; b < 6 * TW * S::R2; b += NT) {
+  for (int b = tid; b < NQ * TW * S::R2; b += NT) {
     const int s = b % TW, n2 = (b / TW) % S::R2, f = b / (TW * S::R2);
     fwd1<S, +1>(buf, [&](int q) { return f * FP + q * TW + s; }, s_tw, n2, LIM);
   }
   __syncthreads();
-  for (int b = tid; b < 6 * TW * S::R1; b += NT) {
+  for (int b = tid; b < NQ * TW * S::R1; b += NT) {
     const int s = b % TW, k1 = (b / TW) % S::R1, f = b / (TW * S::R1);
     C v[S::R2];
     fwd2<S, +1>(buf, [&](int q) { return f * FP + q * TW + s; }, k1, LIM, v);
@@ -177,16 +211,18 @@ k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ ph
   }
 }
 
-// Forward z of the 10 product fields, the sweep, and (emit) the next stage's k_zphase on the
-// updated u.  The state's loads are in flight while the fields are transformed.  grid (NCB, N).
-template <int N, class C>
+// Forward z of the 10 product fields (ROT: the 6 of u x omega on both grids), the sweep, and
+// (emit) the next stage's k_zphase on the updated u.  The state's loads are in flight while the
+// fields are transformed.  grid (NCB, N).
+template <int N, class C, bool ROT>
 __global__ void __launch_bounds__(ZT<N, C>::NT, ZT<N, C>::MINB)
 k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __restrict__ rhs,
          const double* __restrict__ nyq_part, int nparts, const C* __restrict__ phase, const C* __restrict__ tw,
          SweepArgs a0, int prune, int emit, double scale, Geom g) {
   using Z = ZT<N, C>;
   using S = typename Z::S;
-  constexpr int TW = Z::TW, NT = Z::NT, FP = Z::FP, LIM = 10 * FP, NH = Z::NH, MODES = Z::MODES;
+  constexpr int NI = ROT ? 6 : 10, NQ = ROT ? 12 : 6;  // fields in, sequences out
+  constexpr int TW = Z::TW, NT = Z::NT, FP = Z::FP, LIM = (ROT ? 12 : 10) * FP, NH = Z::NH, MODES = Z::MODES;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* const s_tw = reinterpret_cast<C*>(smraw);
   C* const buf = s_tw + N;
@@ -198,7 +234,7 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
   const bool load_g = a.stage > 0;
 
   constexpr int VL = 16 / (int)sizeof(C);  // (a row's padding past N/2 is 128-byte aligned: inside the field)
-  for (int e = tid; e < 10 * N * (TW / VL); e += NT) {
+  for (int e = tid; e < NI * N * (TW / VL); e += NT) {
     const int s = e % (TW / VL) * VL, row = (e / (TW / VL)) % N, f = e / (TW / VL * N);
     copy_async<VL>(buf + SNS_IDX(f * FP + S::natural(row) * TW + s, LIM - VL + 1),
                    work + SNS_IDX(f * g.field + ((long long)row * N + my) * g.pitch + mx0 + s, 12 * g.field));
@@ -226,14 +262,26 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
       lo[i][c] = on && a.ulo ? a.ulo[SNS_IDX(c * g.field + idx, 3 * g.field)] : 0;
     }
   }
+  // r from the products' (or u x omega's) spectra on both grids, then the mode's update
+  auto one_mode = [&](const auto& in, int ix, int iy_, int iz, C ph, C* un, C* gn, C* rr, CompWord* ln) {
+    if constexpr (ROT) {
+      const bool keep = 4LL * (ix * ix + iy_ * iy_ + iz * iz) <= (long long)N * N;
+      C r[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) r[c] = pair_value(in.p0[c], in.ps[c], ph, keep, a.dealias);
+      finish_mode(r, ix, iy_, iz, N, un, gn, load_g, rr, a, ln);
+    } else {
+      sweep_mode(in, ix, iy_, iz, N, ph, un, gn, load_g, rr, a, ln);
+    }
+  };
   copies_wait();
   __syncthreads();
-  for (int b = tid; b < 10 * TW * S::R2; b += NT) {
+  for (int b = tid; b < NI * TW * S::R2; b += NT) {
     const int s = b % TW, n2 = (b / TW) % S::R2, f = b / (TW * S::R2);
     fwd1<S, -1>(buf, [&](int q) { return f * FP + q * TW + s; }, s_tw, n2, LIM);
   }
   __syncthreads();
-  for (int b = tid; b < 10 * TW * S::R1; b += NT) {
+  for (int b = tid; b < NI * TW * S::R1; b += NT) {
     const int s = b % TW, k1 = (b / TW) % S::R1, f = b / (TW * S::R1);
     auto at = [&](int q) { return f * FP + q * TW + s; };
     C v[S::R2];
@@ -249,17 +297,16 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
     const bool on = mode(i, &s, &sl, &ez);
     if (tid + i * NT >= N * TW) continue;
     const int at = sl * TW + s, ix = mx0 + s, iz = signed_mode(ez, N);
-    C U[3], V[3];
     if (on) {
-      ModeIn<C, 5> in;
+      constexpr int NV = NI / 2;
+      ModeIn<C, NV> in;
 #pragma unroll
-      for (int p = 0; p < 5; ++p) {
+      for (int p = 0; p < NV; ++p) {
         in.p0[p] = buf[SNS_IDX(2 * p * FP + at, LIM)];
         in.ps[p] = buf[SNS_IDX((2 * p + 1) * FP + at, LIM)];
       }
       C rr[3];
-      sweep_mode(in, ix, iy, iz, N, __ldg(&phase[SNS_IDX(ix + iy + iz + 3 * N / 2, 3 * N + 1)]), uu[i], gg[i], load_g,
-                 rr, a, lo[i]);
+      one_mode(in, ix, iy, iz, __ldg(&phase[SNS_IDX(ix + iy + iz + 3 * N / 2, 3 * N + 1)]), uu[i], gg[i], rr, lo[i]);
       const long long row = (long long)ez * N + my, idx = row * g.pitch + ix, inq = row * g.pitch + NH;
       const bool nyq_zero = ix == 0 && row != 0;  // the plane mx = N/2 is zero off (N/2,0,0)
 #pragma unroll
@@ -279,13 +326,19 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
         }
       }
     }
-    if (emit) {  // this thread's slots of fields 0..5: nobody else reads them any more
+    if (emit) {  // this thread's slots: nobody else reads them any more
+      C f[NQ / 2] = {};
+      if (on) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        U[c] = V[c] = czero<C>();
-        if (on) both_grids<N>(uu[i][c], ix, my, ez, phase, (real_of<C>)scale, &U[c], &V[c]);
-        buf[SNS_IDX(2 * c * FP + at, LIM)] = U[c];
-        buf[SNS_IDX((2 * c + 1) * FP + at, LIM)] = V[c];
+        for (int c = 0; c < 3; ++c) f[c] = uu[i][c];
+        if constexpr (ROT) vorticity(f, ix, iy, iz, f + 3);
+      }
+#pragma unroll
+      for (int q = 0; q < NQ / 2; ++q) {
+        C U = czero<C>(), V = czero<C>();
+        if (on) both_grids<N>(f[q], ix, my, ez, phase, (real_of<C>)scale, &U, &V);
+        buf[SNS_IDX(2 * q * FP + at, LIM)] = U;
+        buf[SNS_IDX((2 * q + 1) * FP + at, LIM)] = V;
       }
     }
   }
@@ -293,8 +346,8 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
   if (mx0 == 0 && my == 0) {
     // the self-conjugate mode (N/2, 0, 0): a warp per field sums the x pass's per-CTA plane
     // sums (lane-strided, then a fixed shuffle tree)
-    __shared__ double s_part[10];
-    for (int f = tid / 32; f < 10; f += NT / 32) {
+    __shared__ double s_part[NI];
+    for (int f = tid / 32; f < NI; f += NT / 32) {
       double acc = 0.0;
 #pragma unroll 8
       for (int i = tid % 32; i < nparts; i += 32) acc += nyq_part[f * nparts + i];
@@ -304,9 +357,9 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
     }
     __syncthreads();
     if (tid == 0) {
-      ModeIn<C, 5> in;
+      ModeIn<C, NI / 2> in;
 #pragma unroll
-      for (int p = 0; p < 5; ++p) {
+      for (int p = 0; p < NI / 2; ++p) {
         in.p0[p] = cmk((real_of<C>)s_part[2 * p], real_of<C>(0));
         in.ps[p] = cmk((real_of<C>)s_part[2 * p + 1], real_of<C>(0));
       }
@@ -318,7 +371,7 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
         gn[c] = load_g ? gbuf[c * g.field + NH] : czero<C>();
         if (a.ulo) ln[c] = a.ulo[c * g.field + NH];
       }
-      sweep_mode(in, NH, 0, 0, N, phase[NH + 3 * N / 2], un, gn, load_g, rr, a, ln);
+      one_mode(in, NH, 0, 0, phase[NH + 3 * N / 2], un, gn, rr, ln);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         if (a.mode != 0) {
@@ -334,7 +387,7 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
   if (!emit) return;
 
   __syncthreads();
-  for (int b = tid; b < 6 * TW * S::R1; b += NT) {
+  for (int b = tid; b < NQ * TW * S::R1; b += NT) {
     const int s = b % TW, k1 = (b / TW) % S::R1, f = b / (TW * S::R1);
     auto at = [&](int q) { return f * FP + q * TW + s; };
     C v[S::R2];
@@ -343,7 +396,7 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
     rev1<S, +1>(v, buf, at, s_tw, k1, LIM);
   }
   __syncthreads();
-  for (int b = tid; b < 6 * TW * S::R2; b += NT) {
+  for (int b = tid; b < NQ * TW * S::R2; b += NT) {
     const int s = b % TW, m2 = (b / TW) % S::R2, f = b / (TW * S::R2);
     C v[S::R1];
     rev2<S, +1>(buf, [&](int q) { return f * FP + q * TW + s; }, m2, LIM, v);
@@ -359,22 +412,22 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
 // y pass, in place: F fields per CTA (first + 2 i: the fields of one grid), tiles as the z
 // kernels'.  Inverse: pencils outside the sphere are zero when `clean`; forward: they are not
 // stored (the sweep drops them whatever they hold).  grid (NCB, N [z], groups).
-template <int N, class C, int DIR>
+template <int N, class C, int DIR, int NF>
 struct YT {
   using S = ZSplit<N>;
   static constexpr int NH = N / 2;
   static constexpr int TW = (int)(64 / sizeof(C));
   static constexpr int NCB = (NH + TW - 1) / TW;
-  static constexpr int F = DIR > 0 ? 3 : 5;
+  static constexpr int F = NF;
   static constexpr int NT = N <= 32 ? 64 : 160;
   static constexpr int FP = S::SLOTS * TW;
   static constexpr size_t smem = (size_t)(N + F * FP) * sizeof(C);
 };
 
-template <int N, class C, int DIR>
-__global__ void __launch_bounds__(YT<N, C, DIR>::NT)
+template <int N, class C, int DIR, int NF>
+__global__ void __launch_bounds__(YT<N, C, DIR, NF>::NT)
 k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
-  using Y = YT<N, C, DIR>;
+  using Y = YT<N, C, DIR, NF>;
   using S = typename Y::S;
   constexpr int TW = Y::TW, NT = Y::NT, FP = Y::FP, F = Y::F, LIM = F * FP, NH = Y::NH, VL = 16 / (int)sizeof(C);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -382,7 +435,9 @@ k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
   C* const buf = s_tw + N;
   const int tid = threadIdx.x, mx0 = blockIdx.x * TW;
   const long long plane = (long long)blockIdx.y * N;
-  C* const fld = work + (long long)blockIdx.z * g.field;  // fields blockIdx.z + 2 i
+  // groups 0, 1: fields 0, 2, .. and 1, 3, ..; groups 2, 3 (the rotational form's vorticity):
+  // fields 6, 8, 10 and 7, 9, 11
+  C* const fld = work + (long long)(blockIdx.z < 2 ? blockIdx.z : blockIdx.z + 4) * g.field;
   for (int e = tid; e < F * N * (TW / VL); e += NT) {
     const int s = e % (TW / VL) * VL, row = (e / (TW / VL)) % N, f = e / (TW / VL * N);
     C* dst = buf + SNS_IDX(f * FP + S::natural(row) * TW + s, LIM - VL + 1);
@@ -575,6 +630,127 @@ k_xsmall(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
   }
 }
 
+// x pass of the rotational form, in place: u x omega on both grids.  Six packed sequences a row
+// are too many for a thread's registers, so the cross product runs point by point in shared
+// memory between the two transforms.  Inputs: fields 2c, 2c + 1 (u_c), 6 + 2c, 7 + 2c (omega_c);
+// outputs: fields 2c, 2c + 1.  `part`: [6][grid] Nyquist-plane sums.
+template <int N, class C>
+struct XR {
+  using S = ZSplit<N>;
+  static constexpr int NH = N / 2;
+  static constexpr int NT = N <= 32 ? 64 : 128;
+  static constexpr int RB = N <= 32 ? 8 : 4;
+  static constexpr int RP = S::SLOTS;
+  static constexpr int GRID = N * N / RB;
+  static constexpr size_t smem = (size_t)(N + 6 * RB * RP) * sizeof(C);
+  static_assert(N * N % RB == 0, "whole row groups");
+};
+
+template <int N, class C>
+__global__ void __launch_bounds__(XR<N, C>::NT)
+k_xrot(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase, const C* __restrict__ tw,
+       double scale, double* __restrict__ part, Geom g) {
+  using X = XR<N, C>;
+  using S = typename X::S;
+  using RT = real_of<C>;
+  constexpr int NH = X::NH, RB = X::RB, NT = X::NT, RP = X::RP, LIM = 6 * RB * RP;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* const s_tw = reinterpret_cast<C*>(smraw);
+  C* const buf = s_tw + N;
+  const int tid = threadIdx.x;
+  const long long row0 = (long long)blockIdx.x * RB;
+  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+#pragma unroll 4
+  for (int e = tid; e < 6 * RB * NH; e += NT) {
+    const int k = e % NH, q = e / NH, r = q % RB, c = q / RB;  // c: u_0 u_1 u_2 omega_0 omega_1 omega_2
+    const long long at = (row0 + r) * g.pitch + k;
+    const C U = work[SNS_IDX(2 * c * g.field + at, 12 * g.field)];
+    const C V = work[SNS_IDX((2 * c + 1) * g.field + at, 12 * g.field)];
+    C zk, zm;
+    if (k == 0) {  // as k_xsmall; the vorticity of the mode (N/2, 0, 0) from u's
+      C un[6];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) un[i] = unyq[SNS_IDX(i * g.field + NH, 3 * g.field)];
+      vorticity(un, NH, 0, 0, un + 3);
+      C A = un[0];
+#pragma unroll
+      for (int i = 1; i < 6; ++i) A = c == i ? un[i] : A;
+      A = cscale(A, (RT)scale);
+      const C B = cmul(A, phase[NH + 3 * N / 2]);
+      zk = cmk(U.x, V.x);
+      zm = cmk(A.x, B.x);
+    } else {
+      zk = cmk(U.x - V.y, U.y + V.x);
+      zm = cmk(U.x + V.y, V.x - U.y);
+    }
+    buf[SNS_IDX(q * RP + S::natural(k), LIM)] = zk;
+    buf[SNS_IDX(q * RP + S::natural(k == 0 ? NH : N - k), LIM)] = zm;
+  }
+  __syncthreads();
+  for (int b = tid; b < 6 * RB * S::R2; b += NT) {
+    const int n2 = b % S::R2, q = b / S::R2;
+    fwd1<S, +1>(buf, [&](int sl) { return q * RP + sl; }, s_tw, n2, LIM);
+  }
+  __syncthreads();
+  for (int b = tid; b < 6 * RB * S::R1; b += NT) {
+    const int k1 = b % S::R1, q = b / S::R1;
+    auto at = [&](int sl) { return q * RP + sl; };
+    C v[S::R2];
+    fwd2<S, +1>(buf, at, k1, LIM, v);
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) buf[SNS_IDX(at(S::slot(k1, k2)), LIM)] = v[k2];
+  }
+  __syncthreads();
+  for (int e = tid; e < RB * N; e += NT) {
+    const int at = (e / N) * RP + S::natural(e % N);
+    C f[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) f[c] = buf[SNS_IDX(c * RB * RP + at, LIM)];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int a = (c + 1) % 3, b = (c + 2) % 3;
+      buf[SNS_IDX(c * RB * RP + at, LIM)] = cmk(f[a].x * f[3 + b].x - f[b].x * f[3 + a].x,
+                                                f[a].y * f[3 + b].y - f[b].y * f[3 + a].y);
+    }
+  }
+  __syncthreads();
+  for (int b = tid; b < 3 * RB * S::R1; b += NT) {
+    const int k1 = b % S::R1, q = b / S::R1;
+    auto at = [&](int sl) { return q * RP + sl; };
+    C v[S::R2];
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) v[k2] = buf[SNS_IDX(at(S::slot(k1, k2)), LIM)];
+    rev1<S, -1>(v, buf, at, s_tw, k1, LIM);
+  }
+  __syncthreads();
+  for (int b = tid; b < 3 * RB * S::R2; b += NT) {
+    const int m2 = b % S::R2, q = b / S::R2;
+    auto at = [&](int sl) { return q * RP + sl; };
+    C v[S::R1];
+    rev2<S, -1>(buf, at, m2, LIM, v);
+#pragma unroll
+    for (int m1 = 0; m1 < S::R1; ++m1) buf[SNS_IDX(at(S::slot(m1, m2)), LIM)] = v[m1];
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int e = tid; e < 3 * RB * NH; e += NT) {
+    const int k = e % NH, q = e / NH, r = q % RB, c = q / RB;
+    const C Zk = buf[SNS_IDX(q * RP + S::natural(k), LIM)];
+    const C Zm = buf[SNS_IDX(q * RP + S::natural(k == 0 ? 0 : N - k), LIM)];
+    const long long at = 2 * c * g.field + (row0 + r) * g.pitch + k;
+    work[SNS_IDX(at, 12 * g.field)] = cmk(RT(0.5) * (Zk.x + Zm.x), RT(0.5) * (Zk.y - Zm.y));
+    work[SNS_IDX(at + g.field, 12 * g.field)] = cmk(RT(0.5) * (Zk.y + Zm.y), RT(-0.5) * (Zk.x - Zm.x));
+  }
+  if (tid < 6) {
+    double s = 0.0;
+    for (int r = 0; r < RB; ++r) {
+      const C X_ = buf[SNS_IDX(((tid >> 1) * RB + r) * RP + S::natural(NH), LIM)];
+      s += (tid & 1) ? X_.y : X_.x;
+    }
+    part[tid * gridDim.x + blockIdx.x] = s;
+  }
+}
+
 // ------------------------------------------------------------------------------------
 // Forward transform of one real field to the reference's full layout, two launches (FP64,
 // N <= 64): x and y on a whole z plane per CTA, then z with the mirror half written from the
@@ -703,12 +879,16 @@ struct Small {
   static C* F(void* p) { return static_cast<C*>(p); }
   static const C* F(const void* p) { return static_cast<const C*>(p); }
   static void init() {
-    allow_smem(k_ysmall<N, C, +1>, YT<N, C, +1>::smem);
-    allow_smem(k_ysmall<N, C, -1>, YT<N, C, -1>::smem);
+    allow_smem(k_ysmall<N, C, +1, 3>, YT<N, C, +1, 3>::smem);
+    allow_smem(k_ysmall<N, C, -1, 5>, YT<N, C, -1, 5>::smem);
+    allow_smem(k_ysmall<N, C, -1, 3>, YT<N, C, -1, 3>::smem);
+    allow_smem(k_xrot<N, C>, XR<N, C>::smem);
     allow_smem(k_xsmall<N, C, false>, XT<N, C>::smem);
     allow_smem(k_xsmall<N, C, true>, XT<N, C>::smem);
-    allow_smem(k_zphase<N, C>, Z::smem_phase);
-    allow_smem(k_zsweep<N, C>, Z::smem_sweep);
+    allow_smem(k_zphase<N, C, false>, Z::smem(6));
+    allow_smem(k_zphase<N, C, true>, Z::smem(12));
+    allow_smem(k_zsweep<N, C, false>, Z::smem(10));
+    allow_smem(k_zsweep<N, C, true>, Z::smem(12));
   }
   static void forward_init() {
     if constexpr (N <= 64) {
@@ -723,17 +903,25 @@ struct Small {
       k_zfull<N><<<dim3(T::NCB, N), T::NTZ, T::smem_z, st>>>(F(work), F(full), F(tw), g);
     }
   }
-  static void zphase(const void* u, void* work, const void* phase, const void* tw, double scale, int clean, Geom g,
-                     cudaStream_t st) {
-    k_zphase<N, C><<<dim3(Z::NCB, N), Z::NT, Z::smem_phase, st>>>(F(u), F(work), F(phase), F(tw), scale, clean, g);
+  static void zphase(const void* u, void* work, const void* phase, const void* tw, double scale, int clean, int rot,
+                     Geom g, cudaStream_t st) {
+    auto k = rot ? k_zphase<N, C, true> : k_zphase<N, C, false>;
+    k<<<dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 6), st>>>(F(u), F(work), F(phase), F(tw), scale, clean, g);
   }
-  static void yinv(void* work, const void* tw, int grids, int clean, Geom g, cudaStream_t st) {
-    using Y = YT<N, C, +1>;
-    k_ysmall<N, C, +1><<<dim3(Y::NCB, N, grids), Y::NT, Y::smem, st>>>(F(work), F(tw), clean, g);
+  static void yinv(void* work, const void* tw, int groups, int clean, Geom g, cudaStream_t st) {
+    using Y = YT<N, C, +1, 3>;
+    k_ysmall<N, C, +1, 3><<<dim3(Y::NCB, N, groups), Y::NT, Y::smem, st>>>(F(work), F(tw), clean, g);
   }
-  static void yfwd(void* work, const void* tw, Geom g, cudaStream_t st) {
-    using Y = YT<N, C, -1>;
-    k_ysmall<N, C, -1><<<dim3(Y::NCB, N, 2), Y::NT, Y::smem, st>>>(F(work), F(tw), 0, g);
+  static void yfwd(void* work, const void* tw, int rot, Geom g, cudaStream_t st) {
+    using Y5 = YT<N, C, -1, 5>;
+    using Y3 = YT<N, C, -1, 3>;
+    if (rot) k_ysmall<N, C, -1, 3><<<dim3(Y3::NCB, N, 2), Y3::NT, Y3::smem, st>>>(F(work), F(tw), 0, g);
+    else k_ysmall<N, C, -1, 5><<<dim3(Y5::NCB, N, 2), Y5::NT, Y5::smem, st>>>(F(work), F(tw), 0, g);
+  }
+  static void xrot(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part, Geom g,
+                   cudaStream_t st) {
+    using X = XR<N, C>;
+    k_xrot<N, C><<<X::GRID, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), F(tw), scale, part, g);
   }
   static void xpass(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part,
                     int diag, Geom g, cudaStream_t st) {
@@ -743,12 +931,14 @@ struct Small {
     else k_xsmall<N, C, false><<<X::GRID, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), F(tw), scale, part, g);
   }
   static void zsweep(void* work, void* u, void* gbuf, void* rhs, const double* part, int nparts, const void* phase,
-                     const void* tw, SweepArgs a, int prune, int emit, double scale, Geom g, cudaStream_t st) {
-    k_zsweep<N, C><<<dim3(Z::NCB, N), Z::NT, Z::smem_sweep, st>>>(F(work), F(u), F(gbuf), F(rhs), part, nparts,
-                                                                  F(phase), F(tw), a, prune, emit, scale, g);
+                     const void* tw, SweepArgs a, int prune, int emit, int rot, double scale, Geom g,
+                     cudaStream_t st) {
+    auto k = rot ? k_zsweep<N, C, true> : k_zsweep<N, C, false>;
+    k<<<dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 10), st>>>(F(work), F(u), F(gbuf), F(rhs), part, nparts, F(phase),
+                                                              F(tw), a, prune, emit, scale, g);
   }
   static const SmallOps* table() {
-    static const SmallOps ops = {XT<N, C>::GRID, init, zphase, yinv, xpass, yfwd, zsweep,
+    static const SmallOps ops = {XT<N, C>::GRID, XR<N, C>::GRID, init, zphase, yinv, xpass, xrot, yfwd, zsweep,
                                  N <= 64 && sizeof(C) == 16 ? forward_init : nullptr,
                                  N <= 64 && sizeof(C) == 16 ? forward : nullptr};
     return &ops;
