@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -43,6 +44,58 @@ void ck(cudaError_t e, const char* what) {
 }
 
 thread_local std::string g_create_error;
+
+// Mapped pinned words of the handles (reduction results and the error word): pinning memory
+// costs a millisecond or two where the process has little of it, as much as the rest of a
+// small handle's creation, so slots are cut from pinned chunks that handles share and give
+// back.  One chunk stays for the next handle; further ones are freed when every slot is back.
+class WordPool {
+ public:
+  static constexpr size_t kSlot = 256, kSlots = 64;  // 16 KiB a chunk
+  void* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!chunks_.empty() && taken_ == 0) {
+      // a device reset in between takes pinned memory with it
+      cudaPointerAttributes a{};
+      if (cudaPointerGetAttributes(&a, chunks_[0]) != cudaSuccess || a.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        chunks_.clear();
+        free_.clear();
+      }
+    }
+    if (free_.empty()) {
+      void* c = nullptr;
+      ck(cudaHostAlloc(&c, kSlot * kSlots, cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+      chunks_.push_back(c);
+      for (size_t i = 0; i < kSlots; ++i) free_.push_back(static_cast<char*>(c) + i * kSlot);
+    }
+    void* p = free_.back();
+    free_.pop_back();
+    ++taken_;
+    std::memset(p, 0, kSlot);
+    return p;
+  }
+  void give(void* p) {
+    std::lock_guard<std::mutex> lock(mu_);
+    free_.push_back(p);
+    if (--taken_ == 0 && chunks_.size() > 1) {
+      for (size_t i = 1; i < chunks_.size(); ++i) cudaFreeHost(chunks_[i]);
+      chunks_.resize(1);
+      free_.clear();
+      for (size_t i = 0; i < kSlots; ++i) free_.push_back(static_cast<char*>(chunks_[0]) + i * kSlot);
+    }
+  }
+
+ private:
+  std::mutex mu_;
+  std::vector<void*> chunks_, free_;
+  size_t taken_ = 0;
+};
+
+WordPool& word_pool() {
+  static WordPool* pool = new WordPool;  // outlives every handle, static ones included
+  return *pool;
+}
 
 }  // namespace
 
@@ -732,7 +785,7 @@ void release(sns_handle* h) {
   cudaFree(h->tw);
   cudaFree(h->phase);
   cudaFree(h->partials);
-  if (h->red_host) cudaFreeHost(h->red_host);
+  if (h->red_host) word_pool().give(h->red_host);
   cudaFree(h->clock);
   cudaFree(h->tw2);
   cudaFree(h->nyq_part);
@@ -902,8 +955,8 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
     alloc((void**)&h->tw, (size_t)n * h->cbytes);
     alloc((void**)&h->phase, (size_t)(3 * n + 1) * h->cbytes);
     alloc((void**)&h->partials, h->partial_count * sizeof(double));
-    ck(cudaHostAlloc((void**)&h->red_host, 17 * sizeof(double), cudaHostAllocMapped), "cudaHostAlloc");
-    std::memset(h->red_host, 0, 17 * sizeof(double));
+    static_assert(17 * sizeof(double) <= WordPool::kSlot, "a handle's words fit a slot");
+    h->red_host = static_cast<double*>(word_pool().take());
     ck(cudaHostGetDevicePointer((void**)&h->red, h->red_host, 0), "cudaHostGetDevicePointer");
     h->err_word = reinterpret_cast<int*>(h->red + 16);
     alloc((void**)&h->clock, sns::kClockWords * sizeof(double));
