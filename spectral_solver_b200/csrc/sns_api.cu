@@ -11,6 +11,7 @@
 #include "sns_kernels.cuh"
 #include "sns_p5.cuh"
 #include "sns_small.cuh"
+#include "sns_stream.cuh"
 #include "../../include/sns_b200.h"
 
 #include <cuda.h>
@@ -167,6 +168,8 @@ struct sns_handle {
   const sns::P5Ops* p5 = nullptr;  // the fused forward-z + sweep pass, where the size has it
   int p5_grid = 0;          // its persistent CTAs (0: two kernels)
   CUtensorMap map_p5_state{};      // the state fields, boxes of its state units
+  const sns::StreamOps* stream_ops = nullptr;  // the y and z passes of large grids (else k_yz_tma)
+  CUtensorMap map_work_y_part{};   // work fields, y-pencil boxes of its partial loads
   void* tw2 = nullptr;      // W_N^(r*j), r < N/16, j < 16 (two-stage x pass)
   double* nyq_part = nullptr;  // [12][max(1, x2_grid)] Nyquist-plane partial sums
   CUtensorMap map_state_z{};  // state fields (u[3], g[3]), z-pencil boxes
@@ -378,6 +381,24 @@ sns::TmaArgs tma_args(sns_handle* h, int f_in0, int nf, int ncb, void* out, int 
   return a;
 }
 
+// One y (axis 1) or z (axis 2) pass; variant 1: the inverse z pass with the phase shift.
+// `clean` (large grids): the fields are zero outside the sphere's disk of pencils, or will be read
+// as zeros there: the inverse z passes skip those tiles, the inverse y pass does not read them.
+void yz_pass(sns_handle* h, const CUtensorMap& map, int axis, int dir, int variant, sns::TmaArgs a,
+             bool clean = false) {
+  if (h->stream_ops && (h->stream_ops->forward_y || axis != 1 || dir > 0)) {
+    const bool part = clean && axis == 1 && dir > 0;
+    if (clean && axis == 2 && dir > 0) {
+      a.live = h->live;
+      a.nlive = h->nlive;
+    }
+    h->stream_ops->run(part ? h->map_work_y_part : map, axis, dir, variant, part ? 1 : 0, a, h->tw, h->phase, h->g,
+                       h->tma_grid, h->stream);
+  } else {
+    h->ops->yz_tma(map, axis, dir, variant, a, h->tw, h->phase, h->g, h->tma_grid, h->stream);
+  }
+}
+
 void check_inject(sns_handle* h) {
   if (h->fail_after > 0) {
     if (--h->fail_after == 0) throw SnsError(SNS_ERR_INJECTED, "failure injected by sns_debug_fail_after");
@@ -438,6 +459,13 @@ sns::SweepArgs stage_args(const sns_handle* h, int stage, double dt, int mode, c
   return a;
 }
 
+// Is u known to be zero outside the sphere when this stage runs?  Stages 1 and 2 rely on stage
+// 0's sweep, stage 0 on the handle's flag, and not inside a batch's or server's graph capture,
+// where the graph may later be replayed on a new state.
+bool sphere_known(const sns_handle* h, int stage) {
+  return h->prune && (stage > 0 || (h->sphere_clean && (h->own_capture || !capturing(h->stream))));
+}
+
 // One stage in the rotational form: omega_hat, inverse z (+ phase) of u and omega, inverse y
 // of the 12 fields, the u x omega x pass, forward y and z of the 6 products, the sweep.
 void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, int mode, char* rhs_out,
@@ -447,35 +475,24 @@ void run_stage_rot(sns_handle* h, char* u_src, char* g_buf, int stage, double dt
   cudaStream_t st = h->stream;
   const int tiles_in = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   const int f_src = (int)((size_t)(u_src - h->state) / h->fbytes);
+  const bool clean = mode == 0 && h->nyq_clean && h->nlive > 0 && sphere_known(h, stage);
   mark(pm, 0, st);
   o->omega_hat(u_src, h->xf, g, st);
-  o->yz_tma(h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), h->tw, h->phase, g,
-            h->tma_grid, st);
-  o->yz_tma(h->map_x_z, 2, +1, 1, tma_args(h, 0, 3, tiles_in, h->work, 6, h->inv_size()), h->tw, h->phase, g,
-            h->tma_grid, st);
+  yz_pass(h, h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), clean);
+  yz_pass(h, h->map_x_z, 2, +1, 1, tma_args(h, 0, 3, tiles_in, h->work, 6, h->inv_size()), clean);
   mark(pm, 1, st);
-  o->yz_tma(h->map_work_y, 1, +1, 0, tma_args(h, 0, 12, tiles_in, h->work, 0, 1.0), h->tw, h->phase, g, h->tma_grid,
-            st);
+  yz_pass(h, h->map_work_y, 1, +1, 0, tma_args(h, 0, 12, tiles_in, h->work, 0, 1.0), clean);
   mark(pm, 2, st);
   o->xpass_rot(h->work, u_src, h->xf, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->tw, g, st);
   mark(pm, 3, st);
   o->nyq_reduce(h->work, 6, h->nyq_part, g, st);
   mark(pm, 4, st);
-  o->yz_tma(h->map_work_y, 1, -1, 0, tma_args(h, 0, 6, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
-            h->tma_grid, st);
+  yz_pass(h, h->map_work_y, 1, -1, 0, tma_args(h, 0, 6, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 5, st);
-  o->yz_tma(h->map_work_z, 2, -1, 0, tma_args(h, 0, 6, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
-            h->tma_grid, st);
+  yz_pass(h, h->map_work_z, 2, -1, 0, tma_args(h, 0, 6, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 6, st);
   o->sweep_rot(h->work, u_src, g_buf, rhs_out, h->nyq_part, h->phase, stage_args(h, stage, dt, mode, u_src), g, st);
   mark(pm, 7, st);
-}
-
-// Is u known to be zero outside the sphere when this stage runs?  Stages 1 and 2 rely on stage
-// 0's sweep, stage 0 on the handle's flag, and not inside a batch's or server's graph capture,
-// where the graph may later be replayed on a new state.
-bool sphere_known(const sns_handle* h, int stage) {
-  return h->prune && (stage > 0 || (h->sphere_clean && (h->own_capture || !capturing(h->stream))));
 }
 
 // The same stage on a small grid: the inverse z and y transforms of u (unless the previous
@@ -534,13 +551,13 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   // there before the stage (sphere_known) and the stage leaves it zero.  So P5 neither loads,
   // transforms nor sweeps these tiles (their forward-z inputs are never needed); every other
   // value is computed as without pruning.
-  const bool prune = fused && mode == 0 && h->nyq_clean && h->nlive > 0 && sphere_known(h, stage);
+  // The inverse passes of large grids use the same knowledge (yz_pass).
+  const bool clean = mode == 0 && h->nyq_clean && h->nlive > 0 && sphere_known(h, stage);
+  const bool prune = fused && clean;
   mark(pm, 0, st);
-  o->yz_tma(h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), h->tw, h->phase,
-            g, h->tma_grid, st);
+  yz_pass(h, h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), clean);
   mark(pm, 1, st);
-  o->yz_tma(h->map_work_y, 1, +1, 0, tma_args(h, 0, 6, tiles_in, h->work, 0, 1.0), h->tw, h->phase, g, h->tma_grid,
-            st);
+  yz_pass(h, h->map_work_y, 1, +1, 0, tma_args(h, 0, 6, tiles_in, h->work, 0, 1.0), clean);
   mark(pm, 2, st);
   int nparts = 1;
   if (h->x2_grid > 0 && np == 5) {
@@ -554,12 +571,10 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
     o->nyq_reduce(h->work, 2 * np, h->nyq_part, g, st);
   }
   mark(pm, 4, st);
-  o->yz_tma(h->map_work_y, 1, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
-            h->tma_grid, st);
+  yz_pass(h, h->map_work_y, 1, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 5, st);
   if (!fused)
-    o->yz_tma(h->map_work_z, 2, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0), h->tw, h->phase, g,
-              h->tma_grid, st);
+    yz_pass(h, h->map_work_z, 2, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 6, st);
   const sns::SweepArgs a = stage_args(h, stage, dt, mode, u_src);
   if (fused)
@@ -709,10 +724,9 @@ int velocity_partials(sns_handle* h, bool both) {
     return h->small->nparts;
   }
   const int tiles = h->nyq_clean ? h->tiles_data() : h->tiles_all();
-  o->yz_tma(h->map_state_z, 2, +1, 0, tma_args(h, 0, 3, tiles, h->work, 0, h->inv_size()), h->tw, h->phase, g,
-            h->tma_grid, h->stream);
-  o->yz_tma(h->map_work_y, 1, +1, 0, tma_args(h, 0, 3, tiles, h->work, 0, 1.0), h->tw, h->phase, g, h->tma_grid,
-            h->stream);
+  const bool clean = h->nyq_clean && h->nlive > 0 && sphere_known(h, 0);
+  yz_pass(h, h->map_state_z, 2, +1, 0, tma_args(h, 0, 3, tiles, h->work, 0, h->inv_size()), clean);
+  yz_pass(h, h->map_work_y, 1, +1, 0, tma_args(h, 0, 3, tiles, h->work, 0, 1.0), clean);
   return o->xpass_diag2(h->work, h->u(), h->inv_size(), h->nyq_clean ? 1 : 0, h->partials, h->tw, h->tw2, g,
                         h->x2_grid, h->err_word, h->stream);
 }
@@ -776,6 +790,11 @@ int guarded(sns_handle* h, F&& f) {
   }
 }
 
+// Resident CTAs per SM of the y and z passes.
+int yz_blocks_per_sm(const sns_handle* h) {
+  return h->stream_ops ? h->stream_ops->blocks_per_sm() : h->ops->tma_blocks_per_sm();
+}
+
 void release(sns_handle* h) {
   if (h == nullptr) return;
   cudaSetDevice(h->device);
@@ -835,7 +854,7 @@ bool set_launch_shape(sns_handle* h, const int* cfg) {
   int nsm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return false;
   const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
-  const int tma_max = h->ops->tma_blocks_per_sm();
+  const int tma_max = yz_blocks_per_sm(h);
   if (cfg[0] < nsm || cfg[0] > nsm * tma_max || (cfg[1] != 0 && cfg[1] != x2_full) ||
       (cfg[2] != 0 && cfg[2] != p5_full))
     return false;
@@ -964,7 +983,9 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
     ck(cudaMemsetAsync(h->clock, 0, sns::kClockWords * sizeof(double), h->stream), "memset");
     int nsm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
-    h->tma_grid = sns::small_grid_cap(n, nsm * ops->tma_blocks_per_sm());
+    h->stream_ops = sns::stream_for(n, precision);
+    if (h->stream_ops) h->stream_ops->init();
+    h->tma_grid = sns::small_grid_cap(n, nsm * yz_blocks_per_sm(h));
     h->x2_grid = ops->xpass2_grid(nsm);
     h->p5 = sns::p5_for(n, precision);
     if (h->p5) {
@@ -1003,6 +1024,8 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
       ck(cudaStreamSynchronize(h->stream), "live");
     }
     h->map_state_z = make_field_map(h->state, 6, 2, h->g, h->cbytes);
+    if (h->stream_ops)
+      h->map_work_y_part = make_field_map(h->work, 12, 1, h->g, h->cbytes, h->stream_ops->part_rows);
     if (h->p5) h->map_p5_state = make_field_map(h->state, 6, 2, h->g, h->cbytes, h->p5->chunk_rows);
     h->map_work_y = make_field_map(h->work, 12, 1, h->g, h->cbytes);
     h->map_work_z = make_field_map(h->work, 12, 2, h->g, h->cbytes);
@@ -1134,7 +1157,7 @@ int sns_autotune(sns_handle* h, int trial_steps, const char* cache_path, int* ou
     int nsm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
     const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
-    const int tma_max = h->ops->tma_blocks_per_sm();
+    const int tma_max = yz_blocks_per_sm(h);
     auto apply = [&](int tma, int x2, int p5) {
       // only shapes this handle was built for: its Nyquist partial buffer is sized for x2_full
       if (tma < nsm || tma > nsm * tma_max || (x2 != 0 && x2 != x2_full) || (p5 != 0 && p5 != p5_full))

@@ -5,6 +5,7 @@
 #include "sns_kernels.cuh"
 #include "sns_p5.cuh"
 #include "sns_small.cuh"
+#include "sns_stream.cuh"
 #include "sns_tma.cuh"
 #include "../../include/sns_b200.h"
 
@@ -69,6 +70,7 @@ extern "C" int sns_debug_bounds(long long* count, int* line, long long* index) {
   int e = sns::bounds_record(r);
   if (e == 0 && r[0] == 0) e = sns::bounds_record_small(r);  // the small grids' kernels
   if (e == 0 && r[0] == 0) e = sns::bounds_record_p5(r);     // the fused forward-z + sweep
+  if (e == 0 && r[0] == 0) e = sns::bounds_record_stream(r); // the large grids' y and z passes
   if (e != 0) {
     char buf[200];
     std::snprintf(buf, sizeof buf, "sns_debug_bounds: %s", cudaGetErrorString((cudaError_t)e));

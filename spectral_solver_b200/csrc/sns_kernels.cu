@@ -1847,10 +1847,13 @@ struct Launch {
                          const void* tw, Geom g, cudaStream_t st) {
     k_xpass_diag<N, C><<<N * N, nt_x<N>(), x_smem(2), st>>>(F(work), F(unyq), scale, nyq_scalar, partials, F(tw), g);
   }
+  // N >= 256: only the forward y pass (the others are sns_stream.cu's)
+  static constexpr bool kAllYz = N <= 128;
   template <int AXIS, int DIR, int VARIANT>
   static void yz_tma_launch(const CUtensorMap& map, TmaArgs a, const void* tw, const void* phase, Geom g, int grid,
                             cudaStream_t st) {
-    k_yz_tma<N, AXIS, DIR, VARIANT, C><<<grid, nt_tma<N>(), tma_smem<N, C>(), st>>>(map, a, F(tw), F(phase), g);
+    if constexpr (kAllYz || (AXIS == 1 && DIR < 0))
+      k_yz_tma<N, AXIS, DIR, VARIANT, C><<<grid, nt_tma<N>(), tma_smem<N, C>(), st>>>(map, a, F(tw), F(phase), g);
   }
   static void yz_tma(const CUtensorMap& map, int axis, int dir, int variant, TmaArgs a, const void* tw,
                      const void* phase, Geom g, int grid, cudaStream_t st) {
@@ -1868,11 +1871,13 @@ struct Launch {
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, nt_tma<N>(), tma_smem<N, C>());
       lo = nb < lo ? nb : lo;
     };
-    occ(k_yz_tma<N, 2, +1, 1, C>);
     occ(k_yz_tma<N, 1, -1, 0, C>);
-    occ(k_yz_tma<N, 1, +1, 0, C>);
-    occ(k_yz_tma<N, 2, -1, 0, C>);
-    occ(k_yz_tma<N, 2, +1, 0, C>);
+    if constexpr (kAllYz) {
+      occ(k_yz_tma<N, 2, +1, 1, C>);
+      occ(k_yz_tma<N, 1, +1, 0, C>);
+      occ(k_yz_tma<N, 2, -1, 0, C>);
+      occ(k_yz_tma<N, 2, +1, 0, C>);
+    }
     return lo > 0 && lo < (1 << 30) ? lo : 1;
   }
   // Opt every kernel of this size into its dynamic shared memory (once per process).
@@ -1882,11 +1887,13 @@ struct Launch {
       set_smem(k_xpass_w<N, true>, XW<N>::smem);
     }
     else if constexpr (N == 256 || N == 512) set_smem(k_xpass2<N, C>, XP<N, C>::smem);
-    set_smem(k_yz_tma<N, 2, +1, 1, C>, tma_smem<N, C>());
     set_smem(k_yz_tma<N, 1, -1, 0, C>, tma_smem<N, C>());
-    set_smem(k_yz_tma<N, 1, +1, 0, C>, tma_smem<N, C>());
-    set_smem(k_yz_tma<N, 2, -1, 0, C>, tma_smem<N, C>());
-    set_smem(k_yz_tma<N, 2, +1, 0, C>, tma_smem<N, C>());
+    if constexpr (kAllYz) {
+      set_smem(k_yz_tma<N, 2, +1, 1, C>, tma_smem<N, C>());
+      set_smem(k_yz_tma<N, 1, +1, 0, C>, tma_smem<N, C>());
+      set_smem(k_yz_tma<N, 2, -1, 0, C>, tma_smem<N, C>());
+      set_smem(k_yz_tma<N, 2, +1, 0, C>, tma_smem<N, C>());
+    }
     set_smem(k_zpass_inv_phase<N, C>, yz_smem());
     set_smem(k_ypass<N, -1, C>, yz_smem());
     set_smem(k_ypass<N, +1, C>, yz_smem());

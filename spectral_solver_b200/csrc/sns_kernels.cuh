@@ -68,6 +68,9 @@ struct TmaArgs {
   int f_out0;     // first output field (phase variant: 2 outputs per input field)
   double scale;   // applied to every element on load
   int* err;       // device error word (bounded-wait timeout)
+  // large grids: the (c, column block) tiles of each field to run, as c * ncb + cb (null: all)
+  const int* live;
+  int nlive;
 };
 
 // Launch table for one (grid size, precision).  Field and table pointers are complex

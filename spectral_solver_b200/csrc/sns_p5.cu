@@ -23,7 +23,7 @@
 // bandwidth on the bytes it moves), FP32 instruction issue (61 % of the cycles, 860 instructions
 // a mode of which 320 are FP32 arithmetic).  Before (three-stage transforms with five
 // barriers a field, the sweep reading u and g itself, a phase product per pair), per stage:
-// 256^3 0.58 -> 0.47 ms FP64, 0.35 -> 0.32 FP32; 512^3 5.39 -> 3.96 FP64, 2.82 -> 2.56 FP32.
+// 256^3 0.58 -> 0.45 ms FP64, 0.35 -> 0.32 FP32; 512^3 5.39 -> 3.92 FP64, 2.82 -> 2.56 FP32.
 #include "sns_p5.cuh"
 #include "sns_sweep.cuh"
 #include "sns_tma.cuh"
@@ -105,6 +105,10 @@ struct P5 {
   static constexpr int BR = N < 256 ? N : 256;
   static constexpr size_t smem = (size_t)(SLOTS * TILE + N) * sizeof(C) + 128 + SLOTS * sizeof(uint64_t);
   static constexpr int MINB = N >= 512 ? 1 : 2;
+  // a unit's values are in registers before they are worked on; with two CTAs an SM the slot is
+  // refilled then and no barrier ends a unit (256^3 FP64 465 -> 450 us), with one CTA the
+  // refill waits for the unit's end (512^3 FP32 2.60 -> 2.56 ms)
+  static constexpr bool EARLY = MINB == 2;
   static_assert(NT == TW * R2 && (NT / 32 + 3) / 4 * 3 * CW <= 512, "one butterfly per thread");
   static_assert(6 * H * CR * TW <= TILE, "a state unit fits a slot");
 };
@@ -220,6 +224,16 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
           lo_n[j][c] = a.ulo[SNS_IDX(c * g.field + ((long long)mode_e(QC * c0 + j) * N + my) * g.pitch + ix,
                                      3 * g.field)];
     };
+    auto release = [&] {  // true: a wait ran out
+      fence_proxy_async_smem();
+      if (__syncthreads_or(late)) return fail = true;
+      if (tid == 0) issue();
+      if (++b == SLOTS) {
+        b = 0;
+        parity ^= 1u;
+      }
+      return false;
+    };
     if (k < kF) {
       C v[M];
 #pragma unroll
@@ -234,6 +248,7 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = S[SNS_IDX((k1 * R2 + H * i + h) * TW + s, TILE)];
+      if constexpr (P::EARLY) (void)release();  // (the vote above was this unit's)
       dft16<-1>(v);
       if constexpr (P::PAIR) {
         if (h) {
@@ -303,6 +318,21 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
 #pragma unroll
         for (int c = 0; c < 3; ++c) lo[j][c] = lo_n[j][c];
       if (a.ulo && c0 + 1 < P::NCH) load_lo(c0 + 1);
+      auto u_of = [&](int j, int c) { return S[SNS_IDX(((c * H + h) * CR + k1 + 16 * j) * TW + s, TILE)]; };
+      auto g_of = [&](int j, int c) {
+        return load_g ? S[SNS_IDX((((c + 3) * H + h) * CR + k1 + 16 * j) * TW + s, TILE)] : czero<C>();
+      };
+      [[maybe_unused]] C us[QC][3], gs[QC][3];
+      if constexpr (P::EARLY) {
+#pragma unroll
+        for (int j = 0; j < QC; ++j)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            us[j][c] = u_of(j, c);
+            gs[j][c] = g_of(j, c);
+          }
+        if (release()) break;
+      }
 #pragma unroll 1
       for (int j = 0; j < QC; ++j) {
         const int q = QC * c0 + j, ez = mode_e(q), iz = signed_mode(ez, N);
@@ -312,13 +342,17 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
         const C ph = ph_of(iz);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const int row = k1 + 16 * j;
-          uu[c] = S[SNS_IDX(((c * H + h) * CR + row) * TW + s, TILE)];
-          gg[c] = load_g ? S[SNS_IDX((((c + 3) * H + h) * CR + row) * TW + s, TILE)] : czero<C>();
+          if constexpr (P::EARLY) {
+            uu[c] = j == 0 ? us[0][c] : us[QC - 1][c];
+            gg[c] = j == 0 ? gs[0][c] : gs[QC - 1][c];
+          } else {
+            uu[c] = u_of(j, c);
+            gg[c] = g_of(j, c);
+          }
           r3[c] = cscale(cmulc(tmem_ld1<C>(tq + CW * c + WPC * q), ph), RT(0.5));
           l3[c] = j == 0 ? lo[0][c] : lo[QC - 1][c];
         }
-        static_assert(QC == 2, "l3 picks one of two");
+        static_assert(QC == 2, "one of two is picked");
         finish_mode(r3, ix, iy, iz, N, uu, gg, load_g, rr, a, l3);
         if (ix < NH) {
           const long long row = (long long)ez * N + my;
@@ -343,15 +377,8 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
         }
       }
     }
-    fence_proxy_async_smem();  // this slot's accesses come before the copy that refills it
-    if (__syncthreads_or(late)) {
-      fail = true;
-      break;
-    }
-    if (tid == 0) issue();
-    if (++b == SLOTS) {
-      b = 0;
-      parity ^= 1u;
+    if constexpr (!P::EARLY) {
+      if (release()) break;
     }
   }
   }
