@@ -98,6 +98,13 @@ __device__ __forceinline__ void copy_async(C* dst, const C* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
+// Programmatic dependent launch between this file's kernels: a kernel may be scheduled while
+// the one before it on the stream finishes.  It waits for that one's end (and with it every
+// earlier one's) before it touches anything but constants, and lets its own successor be
+// scheduled when its last pass begins.
+__device__ __forceinline__ void predecessor_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Is the pencil (mx, my) wholly outside the sphere |k| <= N/2?
@@ -162,6 +169,7 @@ k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ ph
   if (clean && dead_pencil<N>(mx0, signed_mode(my, N))) return;  // never read (k_ysmall)
   const real_of<C> sc = (real_of<C>)scale;
   for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  predecessor_wait();
   if constexpr (ROT) {
     for (int e = tid; e < N * TW; e += NT) {
       const int s = e % TW, row = e / TW, mx = mx0 + s, at = S::natural(row) * TW + s;
@@ -199,6 +207,7 @@ k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ ph
     fwd1<S, +1>(buf, [&](int q) { return f * FP + q * TW + s; }, s_tw, n2, LIM);
   }
   __syncthreads();
+  successor_start();
   for (int b = tid; b < NQ * TW * S::R1; b += NT) {
     const int s = b % TW, k1 = (b / TW) % S::R1, f = b / (TW * S::R1);
     C v[S::R2];
@@ -230,6 +239,8 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
   const int iy = signed_mode(my, N);
   // u is zero in such a tile before the stage and stays zero; its products are never needed
   if (prune && dead_pencil<N>(mx0, iy)) return;
+  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  predecessor_wait();
   const SweepArgs a = resolve_step(a0);
   const bool load_g = a.stage > 0;
 
@@ -239,7 +250,6 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
     copy_async<VL>(buf + SNS_IDX(f * FP + S::natural(row) * TW + s, LIM - VL + 1),
                    work + SNS_IDX(f * g.field + ((long long)row * N + my) * g.pitch + mx0 + s, 12 * g.field));
   }
-  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
   // mode i of this thread: column s, slot (k1, k2), iz index k1 + R1 k2
   auto mode = [&](int i, int* s, int* sl, int* ez) {
     const int m = tid + i * NT, q = m / TW;
@@ -384,6 +394,7 @@ k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __res
       }
     }
   }
+  successor_start();
   if (!emit) return;
 
   __syncthreads();
@@ -438,6 +449,8 @@ k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
   // groups 0, 1: fields 0, 2, .. and 1, 3, ..; groups 2, 3 (the rotational form's vorticity):
   // fields 6, 8, 10 and 7, 9, 11
   C* const fld = work + (long long)(blockIdx.z < 2 ? blockIdx.z : blockIdx.z + 4) * g.field;
+  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  predecessor_wait();
   for (int e = tid; e < F * N * (TW / VL); e += NT) {
     const int s = e % (TW / VL) * VL, row = (e / (TW / VL)) % N, f = e / (TW / VL * N);
     C* dst = buf + SNS_IDX(f * FP + S::natural(row) * TW + s, LIM - VL + 1);
@@ -447,7 +460,6 @@ k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
       copy_async<VL>(dst, fld + SNS_IDX(2 * f * g.field + (plane + row) * g.pitch + mx0 + s, 11 * g.field));
     }
   }
-  for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
   copies_wait();
   __syncthreads();
   for (int b = tid; b < F * TW * S::R2; b += NT) {
@@ -455,6 +467,7 @@ k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
     fwd1<S, DIR>(buf, [&](int q) { return f * FP + q * TW + s; }, s_tw, n2, LIM);
   }
   __syncthreads();
+  successor_start();
   for (int b = tid; b < F * TW * S::R1; b += NT) {
     const int s = b % TW, k1 = (b / TW) % S::R1, f = b / (TW * S::R1);
     C v[S::R2];
@@ -504,6 +517,7 @@ k_xsmall(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
   const int tid = threadIdx.x;
   const long long row0 = (long long)blockIdx.x * RB;
   for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  predecessor_wait();
   constexpr int ITEMS = NC * RB * NH;
 #pragma unroll 4
   for (int e = tid; e < ITEMS; e += NT) {
@@ -607,6 +621,7 @@ k_xsmall(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
       for (int m1 = 0; m1 < S::R1; ++m1) buf[SNS_IDX(at(S::slot(m1, m2)), LIM)] = v[m1];
     }
     __syncthreads();
+    successor_start();
 #pragma unroll 4
     for (int e = tid; e < 5 * RB * NH; e += NT) {
       const int k = e % NH, q = e / NH, rr = q % RB, p = q / RB;
@@ -660,6 +675,7 @@ k_xrot(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ p
   const int tid = threadIdx.x;
   const long long row0 = (long long)blockIdx.x * RB;
   for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
+  predecessor_wait();
 #pragma unroll 4
   for (int e = tid; e < 6 * RB * NH; e += NT) {
     const int k = e % NH, q = e / NH, r = q % RB, c = q / RB;  // c: u_0 u_1 u_2 omega_0 omega_1 omega_2
@@ -732,6 +748,7 @@ k_xrot(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ p
     for (int m1 = 0; m1 < S::R1; ++m1) buf[SNS_IDX(at(S::slot(m1, m2)), LIM)] = v[m1];
   }
   __syncthreads();
+  successor_start();
 #pragma unroll 4
   for (int e = tid; e < 3 * RB * NH; e += NT) {
     const int k = e % NH, q = e / NH, r = q % RB, c = q / RB;
@@ -866,6 +883,21 @@ k_zfull(const double2* __restrict__ work, double2* __restrict__ full, const doub
   }
 }
 
+template <class... P, class... A>
+void launch(void (*kernel)(P...), dim3 grid, int nt, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(nt);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // (the callers check cudaGetLastError)
+}
+
 template <class K>
 void allow_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -906,36 +938,35 @@ struct Small {
   static void zphase(const void* u, void* work, const void* phase, const void* tw, double scale, int clean, int rot,
                      Geom g, cudaStream_t st) {
     auto k = rot ? k_zphase<N, C, true> : k_zphase<N, C, false>;
-    k<<<dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 6), st>>>(F(u), F(work), F(phase), F(tw), scale, clean, g);
+    launch(k, dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 6), st, F(u), F(work), F(phase), F(tw), scale, clean, g);
   }
   static void yinv(void* work, const void* tw, int groups, int clean, Geom g, cudaStream_t st) {
     using Y = YT<N, C, +1, 3>;
-    k_ysmall<N, C, +1, 3><<<dim3(Y::NCB, N, groups), Y::NT, Y::smem, st>>>(F(work), F(tw), clean, g);
+    launch(k_ysmall<N, C, +1, 3>, dim3(Y::NCB, N, groups), Y::NT, Y::smem, st, F(work), F(tw), clean, g);
   }
   static void yfwd(void* work, const void* tw, int rot, Geom g, cudaStream_t st) {
     using Y5 = YT<N, C, -1, 5>;
     using Y3 = YT<N, C, -1, 3>;
-    if (rot) k_ysmall<N, C, -1, 3><<<dim3(Y3::NCB, N, 2), Y3::NT, Y3::smem, st>>>(F(work), F(tw), 0, g);
-    else k_ysmall<N, C, -1, 5><<<dim3(Y5::NCB, N, 2), Y5::NT, Y5::smem, st>>>(F(work), F(tw), 0, g);
+    if (rot) launch(k_ysmall<N, C, -1, 3>, dim3(Y3::NCB, N, 2), Y3::NT, Y3::smem, st, F(work), F(tw), 0, g);
+    else launch(k_ysmall<N, C, -1, 5>, dim3(Y5::NCB, N, 2), Y5::NT, Y5::smem, st, F(work), F(tw), 0, g);
   }
   static void xrot(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part, Geom g,
                    cudaStream_t st) {
     using X = XR<N, C>;
-    k_xrot<N, C><<<X::GRID, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), F(tw), scale, part, g);
+    launch(k_xrot<N, C>, X::GRID, X::NT, X::smem, st, F(work), F(unyq), F(phase), F(tw), scale, part, g);
   }
   static void xpass(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part,
                     int diag, Geom g, cudaStream_t st) {
     using X = XT<N, C>;
-    if (diag)
-      k_xsmall<N, C, true><<<X::GRID, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), F(tw), scale, part, g);
-    else k_xsmall<N, C, false><<<X::GRID, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), F(tw), scale, part, g);
+    launch(diag ? k_xsmall<N, C, true> : k_xsmall<N, C, false>, X::GRID, X::NT, X::smem, st, F(work), F(unyq),
+           F(phase), F(tw), scale, part, g);
   }
   static void zsweep(void* work, void* u, void* gbuf, void* rhs, const double* part, int nparts, const void* phase,
                      const void* tw, SweepArgs a, int prune, int emit, int rot, double scale, Geom g,
                      cudaStream_t st) {
     auto k = rot ? k_zsweep<N, C, true> : k_zsweep<N, C, false>;
-    k<<<dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 10), st>>>(F(work), F(u), F(gbuf), F(rhs), part, nparts, F(phase),
-                                                              F(tw), a, prune, emit, scale, g);
+    launch(k, dim3(Z::NCB, N), Z::NT, Z::smem(rot ? 12 : 10), st, F(work), F(u), F(gbuf), F(rhs), part, nparts,
+           F(phase), F(tw), a, prune, emit, scale, g);
   }
   static const SmallOps* table() {
     static const SmallOps ops = {XT<N, C>::GRID, XR<N, C>::GRID, init, zphase, yinv, xpass, xrot, yfwd, zsweep,
