@@ -490,6 +490,14 @@ k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
 // x, the two grids' half spectra unpacked on the way out.  `part`: [10][grid] Nyquist-plane sums.
 // DIAG: the physical velocity's energy and vmax^2 instead: u_c on the unshifted grid (fields 0,
 // 2, 4), packed u_0 + i u_1 and u_2; one (sum |u|^2 / 2, max |u|^2) pair per CTA in `part`.
+// Pitch of a row in shared memory: R2 modulo a wavefront's 16 complex floats (8 complex doubles),
+// so that lanes that run over R2 columns and then over rows meet no bank twice.  At 96^3 FP64 the
+// padding would cost a resident CTA; its rows stay packed.
+template <int N, class C, class S>
+constexpr int row_stride() {
+  return N == 96 && sizeof(C) == 16 ? S::SLOTS : S::SLOTS + (16 + S::R2 % 16 - S::SLOTS % 16) % 16;
+}
+
 template <int N, class C>
 struct XT {
   using S = XYSplit<N>;
@@ -497,7 +505,7 @@ struct XT {
   static constexpr int NT = N <= 32 ? 64 : 128;
   // rows per CTA: a thread per (row, k1), a power of two that divides N^2
   static constexpr int RB = NT / S::R1 >= 32 ? 32 : (NT / S::R1 >= 16 ? 16 : (NT / S::R1 >= 8 ? 8 : 4));
-  static constexpr int RP = S::SLOTS;
+  static constexpr int RP = row_stride<N, C, S>();
   static constexpr int GRID = N * N / RB;
   static constexpr size_t smem = (size_t)(N + 5 * RB * RP) * sizeof(C);
   static_assert(N * N % RB == 0 && RB * S::R1 <= NT, "whole row groups");
@@ -655,7 +663,7 @@ struct XR {
   static constexpr int NH = N / 2;
   static constexpr int NT = N <= 32 ? 64 : 128;
   static constexpr int RB = N <= 32 ? 8 : 4;
-  static constexpr int RP = S::SLOTS;
+  static constexpr int RP = row_stride<N, C, S>();
   static constexpr int GRID = N * N / RB;
   static constexpr size_t smem = (size_t)(N + 6 * RB * RP) * sizeof(C);
   static_assert(N * N % RB == 0, "whole row groups");
