@@ -386,7 +386,7 @@ sns::TmaArgs tma_args(sns_handle* h, int f_in0, int nf, int ncb, void* out, int 
 // as zeros there: the inverse z passes skip those tiles, the inverse y pass does not read them.
 void yz_pass(sns_handle* h, const CUtensorMap& map, int axis, int dir, int variant, sns::TmaArgs a,
              bool clean = false) {
-  if (h->stream_ops && (h->stream_ops->forward_y || axis != 1 || dir > 0)) {
+  if (h->stream_ops && (axis != 1 || dir > 0)) {
     const bool part = clean && axis == 1 && dir > 0;
     if (clean && axis == 2 && dir > 0) {
       a.live = h->live;

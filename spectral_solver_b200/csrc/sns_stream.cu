@@ -1,4 +1,4 @@
-// y and z passes of the large grids (N = 256, 512), persistent and TMA-fed.  A tile is 128 bytes
+// z and inverse y passes of the large grids (N = 256, 512), persistent and TMA-fed.  A tile is 128 bytes
 // of columns (TW = 8 complex doubles or 16 complex floats) x the N elements of the axis; tiles
 // land in a ring of shared-memory slots (no multicast) while the ones before are transformed
 // in place: N = 16 * R2, a 16-point butterfly per thread, one barrier, an R2-point one (N = 512:
@@ -7,17 +7,18 @@
 // read, two transforms (the shifted grid's through a work buffer beside the ring), two outputs.
 //
 // The truncation sphere saves traffic, bit for bit: pencils (mx, my) outside the disk
-// 4 (mx^2 + my^2) <= N^2 hold nothing but modes that every stage zeroes.  Forward y does not
-// store them; with u known zero there (`clean`) variant 1 skips their tiles and inverse y reads
-// them as zeros, and does not load the row blocks that hold nothing else.
+// 4 (mx^2 + my^2) <= N^2 hold nothing but modes that every stage zeroes.  With u known zero
+// there, variant 1 skips their tiles and inverse y reads them as zeros, and does not load the
+// row blocks that hold nothing else.
 //
-// What bounds it: memory (256^3: 4.9 TB/s moved).  Per stage, three radix stages through a work
-// buffer with five barriers a tile on all pencils (k_yz_tma) -> here:
-//   variant 1  256^3 FP64 250 -> 202 us, FP32 126 -> 109; 512^3 FP64 2.26 -> 1.57 ms, FP32 1.02 -> 0.84
+// What bounds it: memory (512^3 FP32: variant 1 4.8, inverse y 5.9 TB/s moved).  Per stage, three
+// radix stages through a work buffer with five barriers a tile on all pencils (k_yz_tma) -> here:
+//   variant 1  256^3 FP64 250 -> 202 us, FP32 126 -> 109; 512^3 FP64 2.26 -> 1.57 ms, FP32 1.02 -> 0.87
 //   inverse y  256^3 FP64 298 -> 318 us, FP32 158 -> 159; 512^3 FP64 2.31 -> 1.95 ms, FP32 1.01 -> 1.02
 // (inverse y must read the skipped pencils as zeros, so it goes with variant 1 at every size).
-// Forward y gains at 512^3 FP64 only (3.84 -> 3.65 ms; FP32 1.72 -> 1.84, 256^3 512 -> 525 us and
-// 266 -> 273): the others keep k_yz_tma, whose two butterflies per thread hide more latency.
+// Forward y keeps k_yz_tma, whose two butterflies per thread hide more latency: here, with the
+// pencils outside not stored, 512^3 FP64 3.5 .. 3.9 ms (3.8), FP32 1.84 (1.72), 256^3 525 us (512)
+// and 273 (266).
 #include "sns_stream.cuh"
 #include "sns_sweep.cuh"
 #include "sns_tma.cuh"
@@ -89,6 +90,7 @@ k_stream(const __grid_constant__ CUtensorMap map, TmaArgs a, const C* __restrict
   constexpr int NT = Y::NT, TW = Y::TW, R2 = Y::R2, TILE = Y::TILE, SLOTS = Y::SLOTS, PART = Y::PART;
   constexpr int BR = PARTS ? PART : (N < 256 ? N : 256);
   static_assert(!PARTS || (AXIS == 1 && DIR > 0), "partial loads belong to the inverse y pass");
+  static_assert(AXIS == 2 || DIR > 0, "forward y is k_yz_tma's");
   extern __shared__ unsigned char smraw[];
   const uint32_t pad = (128u - (smem_u32(smraw) & 127u)) & 127u;
   C* const ring = reinterpret_cast<C*>(smraw + pad);
@@ -233,19 +235,8 @@ k_stream(const __grid_constant__ CUtensorMap map, TmaArgs a, const C* __restrict
     // outputs are stored, which then overlap the next tile's first pass
     if constexpr (Y::EARLY) release();
     pass2<DIR, Y>(h, v);
-    if constexpr (AXIS == 1 && DIR < 0) {
-      // pencils outside the disk are never used; element k1 + 16 q + 256 h, |my| as above
-      const int m = s_disk[SNS_IDX(mx, N / 2 + 1)];
-      const int lim = Y::PAIR && h ? m + k1 - 256 : m - k1, hi = m + k1 - N;
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const bool in = Y::PAIR ? lim >= (h ? -16 * q : 16 * q) : (q < 8 ? lim >= 16 * q : hi >= -16 * q);
-        if (in) out[SNS_IDX(at + q * step, g.field)] = v[q];
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 16; ++q) out[SNS_IDX(at + q * step, g.field)] = v[q];
-    }
+    for (int q = 0; q < 16; ++q) out[SNS_IDX(at + q * step, g.field)] = v[q];
     if constexpr (VARIANT == 1) {
       if constexpr (!Y::EARLY) pass2_load<Y>(W, s, k1, h, w);
       pass2<DIR, Y>(h, w);
@@ -281,7 +272,6 @@ struct LaunchStream {
     prepare<2, +1, 1, false>();
     prepare<1, +1, 0, true>();
     prepare<1, +1, 0, false>();
-    if constexpr (kForwardY) prepare<1, -1, 0, false>();
     prepare<2, +1, 0, false>();
     prepare<2, -1, 0, false>();
   }
@@ -294,7 +284,6 @@ struct LaunchStream {
     occ(k_stream<N, 2, +1, 1, false, C>, YZ<N, C, 1>::NT, YZ<N, C, 1>::smem);
     occ(k_stream<N, 1, +1, 0, true, C>, Y0::NT, Y0::smem);
     occ(k_stream<N, 1, +1, 0, false, C>, Y0::NT, Y0::smem);
-    if constexpr (kForwardY) occ(k_stream<N, 1, -1, 0, false, C>, Y0::NT, Y0::smem);
     occ(k_stream<N, 2, +1, 0, false, C>, Y0::NT, Y0::smem);
     occ(k_stream<N, 2, -1, 0, false, C>, Y0::NT, Y0::smem);
     return lo > 0 && lo < (1 << 30) ? lo : 1;
@@ -306,22 +295,16 @@ struct LaunchStream {
     k_stream<N, AXIS, DIR, VARIANT, PARTS, C><<<grid, Y::NT, Y::smem, st>>>(map, a, static_cast<const C*>(tw),
                                                                             static_cast<const C*>(phase), g);
   }
-  static constexpr bool kForwardY = N == 512 && sizeof(C) == 16;
-  static void forward_y(const CUtensorMap& map, TmaArgs a, const void* tw, const void* phase, Geom g, int grid,
-                        cudaStream_t st) {
-    if constexpr (kForwardY) go<1, -1, 0, false>(map, a, tw, phase, g, grid, st);
-  }
   static void run(const CUtensorMap& map, int axis, int dir, int variant, int part, TmaArgs a, const void* tw,
                   const void* phase, Geom g, int grid, cudaStream_t st) {
     if (variant == 1) go<2, +1, 1, false>(map, a, tw, phase, g, grid, st);
-    else if (axis == 1 && dir < 0) forward_y(map, a, tw, phase, g, grid, st);
     else if (axis == 1 && part) go<1, +1, 0, true>(map, a, tw, phase, g, grid, st);
     else if (axis == 1) go<1, +1, 0, false>(map, a, tw, phase, g, grid, st);
     else if (dir < 0) go<2, -1, 0, false>(map, a, tw, phase, g, grid, st);
     else go<2, +1, 0, false>(map, a, tw, phase, g, grid, st);
   }
   static const StreamOps* table() {
-    static const StreamOps ops = {init, blocks_per_sm, run, YZ<N, C, 0>::PART, kForwardY};
+    static const StreamOps ops = {init, blocks_per_sm, run, YZ<N, C, 0>::PART};
     return &ops;
   }
 };

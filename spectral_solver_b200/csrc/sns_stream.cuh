@@ -1,4 +1,4 @@
-// Launch table of the large grids' y and z passes (sns_stream.cu).
+// Launch table of the large grids' z and inverse y passes (sns_stream.cu).
 #pragma once
 
 #include "sns_kernels.cuh"
@@ -9,12 +9,11 @@ namespace sns {
 struct StreamOps {
   void (*init)();               // kernel attributes; call once per device before the first launch
   int (*blocks_per_sm)();       // resident CTAs
-  // as Ops::yz_tma; `part` (inverse y with a.clean): the map's boxes have part_rows rows, and
+  // as Ops::yz_tma, which keeps the forward y pass; `part` (inverse y with a.clean): the map's boxes have part_rows rows, and
   // those without a row inside the sphere are not loaded
   void (*run)(const CUtensorMap& map, int axis, int dir, int variant, int part, TmaArgs a, const void* tw,
               const void* phase, Geom g, int grid, cudaStream_t st);
   int part_rows;
-  bool forward_y;  // it serves the forward y pass too (else Ops::yz_tma does)
 };
 
 // nullptr for sizes whose passes run k_yz_tma
