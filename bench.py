@@ -39,11 +39,14 @@ RE = 1600.0
 DT = 1e-3
 
 # Algorithmic bytes per launch of each pass, in units of S = N^3 * 8 B (one FP64 real field
-# or one half-spectrum complex field): every field read or written once.  At N = 128, 256,
-# 512 the forward z pass and the sweep are one fused kernel ("p5_sweep": 12 product fields
-# + u + g in, u + g out; g is not read in the first stage, hence 23 on average).
-PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 18, "p3_nyq": 0,
-                "p4_yfwd": 24, "p5_zfwd": 24, "p5_sweep": 23}
+# or one half-spectrum complex field): every field read or written once.  The five products of
+# the projected term are 10 fields.  At N = 256 and 512 the forward z pass and the sweep are one
+# fused kernel ("p5_sweep": 10 product fields + u + g in, u + g out; g is not read in the first
+# stage, hence 21 on average).
+PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 16, "p3_nyq": 0,
+                "p4_yfwd": 20, "p5_zfwd": 20, "p5_sweep": 21}
+# The fixed byte model of the roofline figure (all six products, nothing pruned): S per step.
+MODEL_BYTES_S = 261
 
 
 def live_fraction(n, w):
@@ -59,30 +62,32 @@ def live_fraction(n, w):
 
 
 def pruned_pass_bytes(n, w):
-    """Per-launch bytes (units of S) that the sphere-pruned step moves: the fused forward z +
-    sweep loads, transforms and sweeps only the live tiles.  Reported beside the canonical
-    model (PASS_BYTES_S, 261 per step), which stays the roofline's algorithmic figure."""
+    """Per-launch bytes (units of S) that the sphere-pruned step moves: the inverse z pass and
+    the fused forward z + sweep run only the live tiles, and inverse y reads only the row
+    blocks that hold some.  Reported beside the fixed model (MODEL_BYTES_S per step)."""
     L = live_fraction(n, w)
     b = dict(PASS_BYTES_S)
-    b["p5_sweep"] = 23 * L
+    b["p1_zinv_phase"] = 9 * L
+    b["p2_yinv"] = 6 + 6 * L
+    b["p5_sweep"] = 21 * L
     return b, L
 
 
 def step_bytes_s(L):
-    """Bytes per RK3 step in units of S: 3 x (P1 9, P2 12, P3 18, P4 24, P5 24L), which is 261
-    without pruning (L = 1)."""
-    return 189 + 72 * L
+    """Bytes per RK3 step in units of S: 3 x (P1 9 L, P2 6 + 6 L, P3 16, P4 20, P5 21 L)."""
+    return 126 + 108 * L
 # kernels per RK3 stage at N = 512: P1, P2, P3, P4, the (N/2,0,0) mode, fused P5
 LAUNCHES_PER_STEP = 3 * 6
 # DRAM traffic per launch per grid point (dram__bytes_read.sum + dram__bytes_write.sum).  The
-# x pass and the fused P5 were captured on the 512^3 bench workload itself (one-pass metrics;
-# profiles/taylor_green_512_dram_traffic.txt; P5 with the sphere pruning); the other passes
-# come from single-launch captures at 256^3 (profiles/k_*_256_fp64.txt), scaled by N^3.
-TRAFFIC_PER_POINT = {"p5_sweep": (16.716e9 + 5.166e9) / 512 ** 3, "p3_xpass": (6.696e9 + 12.928e9) / 512 ** 3,
-                     "p4_yfwd": 3.268e9 / 256 ** 3, "p1_zinv_phase": 1.166e9 / 256 ** 3,
-                     "p2_yinv": 1.582e9 / 256 ** 3}
+# passes were captured on the 512^3 bench workload itself (profiles/taylor_green_512_dram_traffic.txt;
+# forward y of the FP64 form at 256^3, scaled by N^3).
+TRAFFIC_PER_POINT = {"p1_zinv_phase": (2.736e9 + 5.090e9) / 512 ** 3, "p2_yinv": (5.925e9 + 6.381e9) / 512 ** 3,
+                     "p3_xpass": (6.679e9 + 10.759e9) / 512 ** 3, "p4_yfwd": (1.420e9 + 1.280e9) / 256 ** 3,
+                     "p5_sweep": (12.266e9 + 5.155e9) / 512 ** 3}
 # The same for the FP32 precision form.
-TRAFFIC_PER_POINT_FP32 = {"p3_xpass": (3.485e9 + 6.485e9) / 512 ** 3, "p5_sweep": (9.059e9 + 2.983e9) / 512 ** 3}
+TRAFFIC_PER_POINT_FP32 = {"p1_zinv_phase": (1.379e9 + 2.557e9) / 512 ** 3, "p2_yinv": (2.972e9 + 3.158e9) / 512 ** 3,
+                          "p3_xpass": (3.464e9 + 5.391e9) / 512 ** 3, "p4_yfwd": (5.656e9 + 5.307e9) / 512 ** 3,
+                          "p5_sweep": (6.355e9 + 2.968e9) / 512 ** 3}
 
 
 def load_peaks():
@@ -331,8 +336,8 @@ def measure_form(args, n, precision, local, pg):
     prof = s.profile_passes(DT, 1)
     w = 8 if precision == 0 else 4
     S = n ** 3 * w
-    # roofline.achieved and the model fraction use the canonical per-pass bytes (261 N^3 w per
-    # step, fixed); the sphere-pruned bytes that the fused P5 actually moves are reported beside
+    # roofline.achieved uses the per-pass algorithmic bytes, the model fraction the fixed model
+    # (261 N^3 w per step); the bytes that the sphere-pruned passes move are reported beside
     pass_bytes, L = pruned_pass_bytes(n, w)
     top = max(prof, key=prof.get)
     achieved = PASS_BYTES_S[top] * S / (prof[top] / 1e3) / 1e9
@@ -345,7 +350,7 @@ def measure_form(args, n, precision, local, pg):
             "pruned_bytes_per_launch": pass_bytes[top] * S}
     return s, {"value": value, "ms_per_step": ms_max / args.steps, "clocks": clocks, "roofline": roof,
                "passes_ms_per_stage": prof, "live_tile_fraction": L,
-               "model_roofline_frac": value / (peak / (261 * w)),
+               "model_roofline_frac": value / (peak / (MODEL_BYTES_S * w)),
                "pruned_bytes_per_point_step": step_bytes_s(L) * w,
                "pruned_model_roofline_frac": value / (peak / (step_bytes_s(L) * w)),
                "steps_done": args.warmup + args.steps + 1}

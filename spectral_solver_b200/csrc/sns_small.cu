@@ -101,7 +101,9 @@ __device__ __forceinline__ void copy_async(C* dst, const C* src) {
 // Programmatic dependent launch between this file's kernels: a kernel may be scheduled while
 // the one before it on the stream finishes.  It waits for that one's end (and with it every
 // earlier one's) before it touches anything but constants, and lets its own successor be
-// scheduled when its last pass begins.
+// scheduled when its last pass begins.  The kernels' data pointers are not __restrict__: a load
+// through a restrict pointer may be moved above the wait, whatever the wait clobbers (only the
+// tables, written once at a handle's creation, stay restrict).
 __device__ __forceinline__ void predecessor_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -156,7 +158,7 @@ __device__ __forceinline__ void vorticity(const C u[3], int ix, int iy, int iz, 
 // vorticity too, fields 6 + 2c, 7 + 2c.  grid (NCB, N).
 template <int N, class C, bool ROT>
 __global__ void __launch_bounds__(ZT<N, C>::NT)
-k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ phase, const C* __restrict__ tw,
+k_zphase(const C* u, C* work, const C* __restrict__ phase, const C* __restrict__ tw,
          double scale, int clean, Geom g) {
   using Z = ZT<N, C>;
   using S = typename Z::S;
@@ -225,8 +227,8 @@ k_zphase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ ph
 // fields are transformed.  grid (NCB, N).
 template <int N, class C, bool ROT>
 __global__ void __launch_bounds__(ZT<N, C>::NT, ZT<N, C>::MINB)
-k_zsweep(C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf, C* __restrict__ rhs,
-         const double* __restrict__ nyq_part, int nparts, const C* __restrict__ phase, const C* __restrict__ tw,
+k_zsweep(C* work, C* u, C* gbuf, C* rhs,
+         const double* nyq_part, int nparts, const C* __restrict__ phase, const C* __restrict__ tw,
          SweepArgs a0, int prune, int emit, double scale, Geom g) {
   using Z = ZT<N, C>;
   using S = typename Z::S;
@@ -437,7 +439,7 @@ struct YT {
 
 template <int N, class C, int DIR, int NF>
 __global__ void __launch_bounds__(YT<N, C, DIR, NF>::NT)
-k_ysmall(C* __restrict__ work, const C* __restrict__ tw, int clean, Geom g) {
+k_ysmall(C* work, const C* __restrict__ tw, int clean, Geom g) {
   using Y = YT<N, C, DIR, NF>;
   using S = typename Y::S;
   constexpr int TW = Y::TW, NT = Y::NT, FP = Y::FP, F = Y::F, LIM = F * FP, NH = Y::NH, VL = 16 / (int)sizeof(C);
@@ -513,8 +515,8 @@ struct XT {
 
 template <int N, class C, bool DIAG>
 __global__ void __launch_bounds__(XT<N, C>::NT)
-k_xsmall(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase, const C* __restrict__ tw,
-         double scale, double* __restrict__ part, Geom g) {
+k_xsmall(C* work, const C* unyq, const C* __restrict__ phase, const C* __restrict__ tw,
+         double scale, double* part, Geom g) {
   using X = XT<N, C>;
   using S = typename X::S;
   using RT = real_of<C>;
@@ -671,8 +673,8 @@ struct XR {
 
 template <int N, class C>
 __global__ void __launch_bounds__(XR<N, C>::NT)
-k_xrot(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase, const C* __restrict__ tw,
-       double scale, double* __restrict__ part, Geom g) {
+k_xrot(C* work, const C* unyq, const C* __restrict__ phase, const C* __restrict__ tw,
+       double scale, double* part, Geom g) {
   using X = XR<N, C>;
   using S = typename X::S;
   using RT = real_of<C>;
