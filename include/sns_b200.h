@@ -139,10 +139,9 @@ int sns_set_viscosity(sns_handle* h, double nu);
 enum { SNS_FORM_CONSERVATIVE = 0, SNS_FORM_ROTATIONAL = 1 };
 int sns_set_nonlinear_form(sns_handle* h, int form);
 
-/* Sphere pruning of the RK update (on by default; grids with the fused forward-z + sweep
- * pass, N = 128, 256, 512).  The column-block tiles (my, mx block) of the z pencils that hold
- * only modes outside the sphere |k| <= N/2 are zero in the state and zeroed by every stage,
- * so the fused pass skips them: no load, no transform, no sweep (about a fifth of its tiles).
+/* Sphere pruning of the RK update (on by default).  The z pencils (mx, my) that hold only modes
+ * outside the sphere |k| <= N/2 are zero in the state and zeroed by every stage, so the passes
+ * skip the tiles that consist of them: no load, no transform, no sweep (about a fifth).
  * The results are bitwise those of the full computation; enabled = 0 runs every tile. */
 int sns_set_sphere_pruning(sns_handle* h, int enabled);
 

@@ -767,6 +767,7 @@ void initial_field(sns_handle* h, uint64_t seed, double pert_amp, int pert_kmax)
   ck(cudaMemsetAsync(h->work, 0, 12 * fb, h->stream), "memset");
   h->nyq_clean = true;
   h->sphere_clean = true;  // project_truncate zeroed every mode outside the sphere
+  h->z_ready = h->y_ready = false;
 }
 
 template <class F>
@@ -1318,6 +1319,7 @@ int sns_set_state(sns_handle* h, const double* const uhat_full[3]) {
     }
     h->nyq_clean = !dirty;
     h->sphere_clean = false;
+    h->z_ready = h->y_ready = false;
   });
 }
 
