@@ -45,7 +45,10 @@ DT = 1e-3
 # stage, hence 21 on average).
 PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 16, "p3_nyq": 0,
                 "p4_yfwd": 20, "p5_zfwd": 20, "p5_sweep": 21}
-# The fixed byte model of the roofline figure (all six products, nothing pruned): S per step.
+# The fixed byte model of the roofline figure: the same passes with all six products (12 fields).
+MODEL_PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 18, "p3_nyq": 0,
+                      "p4_yfwd": 24, "p5_zfwd": 24, "p5_sweep": 23}
+# S per step of that model, nothing pruned (step_bytes_s(1)).
 MODEL_BYTES_S = 261
 
 
@@ -62,9 +65,24 @@ def live_fraction(n, w):
 
 
 def pruned_pass_bytes(n, w):
-    """Per-launch bytes (units of S) that the sphere-pruned step moves: the inverse z pass and
-    the fused forward z + sweep run only the live tiles, and inverse y reads only the row
-    blocks that hold some.  Reported beside the fixed model (MODEL_BYTES_S per step)."""
+    """Per-launch bytes (units of S) of the fixed six-product model with only the fused forward
+    z + sweep pruned to its live tiles, and the live fraction."""
+    L = live_fraction(n, w)
+    b = dict(MODEL_PASS_BYTES_S)
+    b["p5_sweep"] = 23 * L
+    return b, L
+
+
+def step_bytes_s(L):
+    """Bytes per RK3 step of the fixed six-product model in units of S: 3 x (P1 9, P2 12, P3 18,
+    P4 24, P5 24L), which is 261 without pruning (L = 1)."""
+    return 189 + 72 * L
+
+
+def moved_pass_bytes(n, w):
+    """Per-launch bytes (units of S) that the step moves: five products, the inverse z pass and
+    the fused forward z + sweep on the live tiles only, inverse y reading only the row blocks
+    that hold some.  Reported beside the fixed model (MODEL_BYTES_S per step)."""
     L = live_fraction(n, w)
     b = dict(PASS_BYTES_S)
     b["p1_zinv_phase"] = 9 * L
@@ -73,8 +91,8 @@ def pruned_pass_bytes(n, w):
     return b, L
 
 
-def step_bytes_s(L):
-    """Bytes per RK3 step in units of S: 3 x (P1 9 L, P2 6 + 6 L, P3 16, P4 20, P5 21 L)."""
+def moved_step_bytes_s(L):
+    """Bytes moved per RK3 step in units of S: 3 x (P1 9L, P2 6 + 6L, P3 16, P4 20, P5 21L)."""
     return 126 + 108 * L
 # kernels per RK3 stage at N = 512: P1, P2, P3, P4, the (N/2,0,0) mode, fused P5
 LAUNCHES_PER_STEP = 3 * 6
@@ -338,7 +356,7 @@ def measure_form(args, n, precision, local, pg):
     S = n ** 3 * w
     # roofline.achieved uses the per-pass algorithmic bytes, the model fraction the fixed model
     # (261 N^3 w per step); the bytes that the sphere-pruned passes move are reported beside
-    pass_bytes, L = pruned_pass_bytes(n, w)
+    pass_bytes, L = moved_pass_bytes(n, w)
     top = max(prof, key=prof.get)
     achieved = PASS_BYTES_S[top] * S / (prof[top] / 1e3) / 1e9
     peak, peak_kind = load_peaks()
@@ -351,8 +369,8 @@ def measure_form(args, n, precision, local, pg):
     return s, {"value": value, "ms_per_step": ms_max / args.steps, "clocks": clocks, "roofline": roof,
                "passes_ms_per_stage": prof, "live_tile_fraction": L,
                "model_roofline_frac": value / (peak / (MODEL_BYTES_S * w)),
-               "pruned_bytes_per_point_step": step_bytes_s(L) * w,
-               "pruned_model_roofline_frac": value / (peak / (step_bytes_s(L) * w)),
+               "pruned_bytes_per_point_step": moved_step_bytes_s(L) * w,
+               "pruned_model_roofline_frac": value / (peak / (moved_step_bytes_s(L) * w)),
                "steps_done": args.warmup + args.steps + 1}
 
 

@@ -213,9 +213,9 @@ struct sns_handle {
 
 namespace {
 
-// Grids whose stage runs on the kernels of sns_small.cu.  At 128^3 they take 0.55 ms a step
-// (FP32; 0.60 on the streaming passes) and 1.00 ms (FP64; 1.30), at 96^3 0.28 (0.44) and 0.45
-// (0.75), at 64^3 0.12 (0.21) and 0.15 (0.30); at 256^3 a z tile of the ten product fields
+// Grids whose stage runs on the kernels of sns_small.cu.  At 128^3 they take 0.51 ms a step
+// (FP32; 0.60 on the streaming passes) and 0.98 ms (FP64; 1.30), at 96^3 0.24 (0.44) and 0.42
+// (0.75), at 64^3 0.086 (0.21) and 0.112 (0.30); at 256^3 a z tile of the ten product fields
 // takes a whole SM's shared memory.
 bool small_rule(int n) { return n <= 128; }
 
