@@ -16,7 +16,7 @@ struct BoundsRecord {
   long long index;
   int line;
 };
-// one record per translation unit; the pass kernels and sns_debug_bounds share sns_kernels.cu's
+// one record per translation unit; sns_debug_bounds reads each of them and adds up the counts
 static __device__ BoundsRecord g_bounds;
 __device__ __forceinline__ long long bounds_checked(long long i, long long n, int line) {
   if (i >= 0 && i < n) return i;
