@@ -16,7 +16,7 @@ struct BoundsRecord {
   long long index;
   int line;
 };
-// one record per translation unit; sns_debug_bounds reads each of them and adds up the counts
+// one record per translation unit; sns_debug_bounds returns the first one that holds an entry
 static __device__ BoundsRecord g_bounds;
 __device__ __forceinline__ long long bounds_checked(long long i, long long n, int line) {
   if (i >= 0 && i < n) return i;
