@@ -188,7 +188,7 @@ struct sns_handle {
   // inside the sphere |k| <= N/2 (4 ((cb * TW)^2 + my^2) <= N^2, ncb = tiles_data()); the
   // others hold only modes that every RK stage zeroes.  sphere_clean: u is known to be exactly
   // zero outside the sphere (after creation and after any RK stage that ran, not one only
-  // captured into a graph; false after the state is set).
+  // captured into a graph or on a clock that may have stopped; false after the state is set).
   int* live = nullptr;
   int nlive = 0;
   bool sphere_clean = false;
@@ -586,12 +586,13 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
 }
 
 void step_once(sns_handle* h, double dt) {
-  const bool deferred = capturing(h->stream);  // a captured graph runs later, on whatever state
+  // a captured graph runs later, on whatever state; a step on a stopped clock changes nothing
+  const bool unknown = capturing(h->stream) || h->step_src == h->clock;
   for (int s = 0; s < 3; ++s) {
     run_stage(h, h->u(), h->gb(), s, dt, 0, nullptr);
     h->nyq_clean = true;  // the sweep zeroes the plane mx = N/2 off (N/2,0,0)
     // and every mode outside the sphere, once the stage has run
-    if (!deferred) h->sphere_clean = true;
+    if (!unknown) h->sphere_clean = true;
   }
 }
 
@@ -654,6 +655,14 @@ bool replay_step(sns_handle* h, bool on_clock) {
   return true;
 }
 
+// Steps that the device clock has taken since it was set.
+double clock_steps(sns_handle* h) {
+  double n = 0.0;
+  ck(cudaMemcpyAsync(&n, h->clock + sns::kClockSteps, sizeof n, cudaMemcpyDeviceToHost, h->stream), "clock");
+  sync(h, "clock");
+  return n;
+}
+
 // nsteps fixed steps of size dt, or (on_clock) adaptive steps on the device clock.
 void take_steps(sns_handle* h, double dt, int nsteps, bool on_clock) {
   for (int s = 0; s < nsteps; ++s) {
@@ -665,8 +674,16 @@ void take_steps(sns_handle* h, double dt, int nsteps, bool on_clock) {
       }
       if (replay_step(h, on_clock)) continue;
     }
-    if (on_clock) step_on_clock(h);
-    else step_once(h, dt);
+    if (on_clock && !h->sphere_clean) {
+      // a state from outside: it is clean once the clock has moved (a stopped one leaves it as it is)
+      const double before = clock_steps(h);
+      step_on_clock(h);
+      h->sphere_clean = clock_steps(h) > before;
+    } else if (on_clock) {
+      step_on_clock(h);
+    } else {
+      step_once(h, dt);
+    }
     h->warm_steps++;
   }
 }
