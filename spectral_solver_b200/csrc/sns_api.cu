@@ -587,13 +587,15 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
 
 void step_once(sns_handle* h, double dt) {
   // a captured graph runs later, on whatever state; a step on a stopped clock changes nothing
-  const bool unknown = capturing(h->stream) || h->step_src == h->clock;
+  const bool on_clock = h->step_src == h->clock, unknown = capturing(h->stream) || on_clock;
+  const bool nyq = h->nyq_clean;
   for (int s = 0; s < 3; ++s) {
     run_stage(h, h->u(), h->gb(), s, dt, 0, nullptr);
     h->nyq_clean = true;  // the sweep zeroes the plane mx = N/2 off (N/2,0,0)
     // and every mode outside the sphere, once the stage has run
     if (!unknown) h->sphere_clean = true;
   }
+  if (on_clock) h->nyq_clean = nyq;
 }
 
 int velocity_partials(sns_handle* h, bool both = false);
@@ -674,11 +676,11 @@ void take_steps(sns_handle* h, double dt, int nsteps, bool on_clock) {
       }
       if (replay_step(h, on_clock)) continue;
     }
-    if (on_clock && !h->sphere_clean) {
+    if (on_clock && !(h->sphere_clean && h->nyq_clean)) {
       // a state from outside: it is clean once the clock has moved (a stopped one leaves it as it is)
       const double before = clock_steps(h);
       step_on_clock(h);
-      h->sphere_clean = clock_steps(h) > before;
+      if (clock_steps(h) > before) h->sphere_clean = h->nyq_clean = true;
     } else if (on_clock) {
       step_on_clock(h);
     } else {

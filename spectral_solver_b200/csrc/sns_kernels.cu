@@ -1125,7 +1125,7 @@ k_sweep(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
     }
     // The plane mx = N/2 is outside the sphere except at (N/2,0,0): the reference's
     // masked RHS, g and projected u are zero there.  Row 0 is written below.
-    if (mx == 0 && row != 0) {
+    if (mx == 0 && row != 0 && !a.frozen) {
       const long long inq = row * g.pitch + NH;
       const C zero = czero<C>();
 #pragma unroll
@@ -1324,7 +1324,7 @@ k_sweep_rot(const C* __restrict__ work, C* __restrict__ u, C* __restrict__ gbuf,
       B[c] = work[(long long)(2 * c + 1) * g.field + idx];
     }
     update(idx, mx, my, mz, A, B, phase[mx + my + mz + 3 * N / 2]);
-    if (mx == 0 && row != 0) {  // the plane mx = N/2 is zero off (N/2,0,0) after the mask
+    if (mx == 0 && row != 0 && !a.frozen) {  // the plane mx = N/2 is zero off (N/2,0,0) after the mask
       const long long inq = row * g.pitch + NH;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {

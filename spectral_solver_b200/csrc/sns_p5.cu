@@ -357,7 +357,7 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
         if (ix < NH) {
           const long long row = (long long)ez * N + my;
           const long long idx = SNS_IDX(row * g.pitch + ix, g.field), inq = SNS_IDX(row * g.pitch + NH, g.field);
-          const bool nyq_zero = ix == 0 && row != 0;  // the plane mx = N/2 is zero off (N/2,0,0)
+          const bool nyq_zero = ix == 0 && row != 0 && !a.frozen;  // the plane mx = N/2 is zero off (N/2,0,0)
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             if (a.mode != 0) {

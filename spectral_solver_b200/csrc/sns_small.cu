@@ -320,7 +320,7 @@ k_zsweep(C* work, C* u, C* gbuf, C* rhs,
       C rr[3];
       one_mode(in, ix, iy, iz, __ldg(&phase[SNS_IDX(ix + iy + iz + 3 * N / 2, 3 * N + 1)]), uu[i], gg[i], rr, lo[i]);
       const long long row = (long long)ez * N + my, idx = row * g.pitch + ix, inq = row * g.pitch + NH;
-      const bool nyq_zero = ix == 0 && row != 0;  // the plane mx = N/2 is zero off (N/2,0,0)
+      const bool nyq_zero = ix == 0 && row != 0 && !a.frozen;  // the plane mx = N/2 is zero off (N/2,0,0)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         if (a.mode != 0) {
