@@ -14,16 +14,17 @@
 // axes, so every global access is a coalesced row segment; TW whole rows for x); the first
 // stage reads global memory, the last one writes it, the stages between meet in shared memory.
 //
-// The solver's transforms are packed two real fields to a complex one.  The reference keeps
+// The dealiased solver's transforms carry two real fields in a complex one.  The reference keeps
 // the real part of every inverse transform, and Re(IDFT(c)) = IDFT(H(c)) with H(c)_m =
 // (c_m + conj(c_-m)) / 2, for any c.  So the first inverse pass reads Z = H(U) + i H(V) from
-// the spectrum (U, V: the plain and the shifted grid of one component, or two components when
-// there is no shifted grid), the x passes work on u + i v, the forward passes read products
-// formed on the fly, and the finishing kernel takes both spectra apart through the mirror
-// mode.  A stage is 3 inverse and 5 forward complex transforms (2 and 3 without the shifted
-// grid) in seven launches; one transform per real field, with a table lookup per DFT
-// term, took 18 and 75 launches.  Six steps at 96 x 80 x 60, host copies included, take 10.8 ms
-// instead of 56.2.
+// the spectrum (U, V: the plain and the shifted grid of one component), the x passes work on
+// u + i v, the forward passes read products formed on the fly, and the finishing kernel takes
+// both spectra apart through the mirror mode.  Two components never share a transform: the
+// round-off of the larger one would reach the smaller (a perturbation of a planar flow, or a
+// component that is exactly zero), so without the shifted grid the imaginary part stays empty.
+// A stage is 3 inverse and 5 forward complex transforms in seven launches; one transform per
+// real field, with a table lookup per DFT term, took 18 and 75 launches.  Six steps at
+// 96 x 80 x 60, host copies included, take 10.8 ms instead of 56.2.
 #include "sns_fft.cuh"
 #include "sns_kernels.cuh"
 #include "../../include/sns_b200.h"
@@ -123,7 +124,7 @@ struct AxisArgs {
   AxisPlan plan;
   const double2* twl;   // W_L^t = exp(-2 pi i t / L)
   Modes md;             // kPack
-  int shifted;          // kPack, kProduct: the packed pair is one component's two grids
+  int shifted;          // kProduct: the input holds both grids, else the plain one (its real part)
   int nprod;            // kProduct: 5 (squares less u_2^2) or 6 products; -1: u_0 u_1 alone
 };
 
@@ -138,60 +139,36 @@ __device__ __forceinline__ double2 herm(double2 a, double2 m) {
   return make_double2(0.5 * (a.x + m.x), 0.5 * (a.y - m.y));
 }
 
-// H(U) + i H(V) at one mode: U, V = u_f on both grids (shifted), or u_2f and u_2f+1 (the last
-// one absent: zero).
+// H(U) + i H(V) at one mode: U, V = u_f on both grids.
 __device__ double2 packed_pair(const AxisArgs& a, int f, int ix, int iy, int iz) {
   const long long id = ((long long)iz * a.d.ny + iy) * a.d.nx + ix;
-  double2 U, V;
-  if (a.shifted) {
-    const double2* u = a.in + f * a.n3;
-    const double2 c = u[id], m = mirror_of(u, ix, iy, iz, a.d);
-    const Mode mo = mode_at(ix, iy, iz, a.md);
-    const double2 ph = phase_of(mo, a.md);
-    // the mirror mode's phase: its wavenumber is -k, except +n/2 on an axis of index n/2
-    const int nx = a.d.nx, ny = a.d.ny, nz = a.d.nz;
-    double2 pm = make_double2(ph.x, -ph.y);
-    if (2 * ix == nx || 2 * iy == ny || 2 * iz == nz)
-      pm = phase_of(mode_at(ix ? nx - ix : 0, iy ? ny - iy : 0, iz ? nz - iz : 0, a.md), a.md);
-    U = herm(c, m);
-    V = herm(cm(c, ph), cm(m, pm));
-  } else {
-    const double2* u = a.in + 2 * f * a.n3;
-    U = herm(u[id], mirror_of(u, ix, iy, iz, a.d));
-    V = make_double2(0.0, 0.0);
-    if (2 * f + 1 < 3) V = herm(u[a.n3 + id], mirror_of(u + a.n3, ix, iy, iz, a.d));
-  }
+  const double2* u = a.in + f * a.n3;
+  const double2 c = u[id], m = mirror_of(u, ix, iy, iz, a.d);
+  const Mode mo = mode_at(ix, iy, iz, a.md);
+  const double2 ph = phase_of(mo, a.md);
+  // the mirror mode's phase: its wavenumber is -k, except +n/2 on an axis of index n/2
+  const int nx = a.d.nx, ny = a.d.ny, nz = a.d.nz;
+  double2 pm = make_double2(ph.x, -ph.y);
+  if (2 * ix == nx || 2 * iy == ny || 2 * iz == nz)
+    pm = phase_of(mode_at(ix ? nx - ix : 0, iy ? ny - iy : 0, iz ? nz - iz : 0, a.md), a.md);
+  const double2 U = herm(c, m), V = herm(cm(c, ph), cm(m, pm));
   return make_double2(U.x - V.y, U.y + V.x);
 }
 
-// Product p of the physical fields at point id: 00, 01, 02, 11, 12, 22, the squares less u_2^2
-// when only 5 are asked for (the difference is a gradient's, which the projection removes).
+// Product f of the physical fields at point id, on both grids or (not shifted) on the plain one:
+// 00, 01, 02, 11, 12, 22, the squares less u_2^2 when only 5 are asked for (the difference is a
+// gradient's, which the projection removes).
 __device__ __forceinline__ double one_product(double a, double b, bool diff) {
   return diff ? (a - b) * (a + b) : a * b;
 }
 __device__ double2 packed_product(const AxisArgs& a, int f, long long id) {
-  auto pair = [&](int p, int* x, int* y) {
-    *x = (p >= 3) + (p >= 5);
-    *y = p < 3 ? p : (p < 5 ? p - 2 : 2);
-    const bool diff = a.nprod == 5 && *x == *y;
-    if (diff) *y = 2;
-    return diff;
-  };
-  int x, y;
-  if (a.shifted) {  // both grids of product f
-    const bool diff = pair(a.nprod < 0 ? 1 : f, &x, &y);
-    const double2 u = a.in[x * a.n3 + id], v = a.in[y * a.n3 + id];
-    return make_double2(one_product(u.x, v.x, diff), one_product(u.y, v.y, diff));
-  }
-  // products 2f and 2f + 1 (or none) on one grid; u_0, u_1 are the parts of field 0, u_2 of 1
-  auto u = [&](int c) { return c == 1 ? a.in[id].y : a.in[(c >> 1) * a.n3 + id].x; };
-  bool diff = pair(2 * f, &x, &y);
-  double2 r = make_double2(one_product(u(x), u(y), diff), 0.0);
-  if (2 * f + 1 < a.nprod) {
-    diff = pair(2 * f + 1, &x, &y);
-    r.y = one_product(u(x), u(y), diff);
-  }
-  return r;
+  const int p = a.nprod < 0 ? 1 : f;
+  const int x = (p >= 3) + (p >= 5);
+  int y = p < 3 ? p : (p < 5 ? p - 2 : 2);
+  const bool diff = a.nprod == 5 && x == y;
+  if (diff) y = 2;
+  const double2 u = a.in[x * a.n3 + id], v = a.in[y * a.n3 + id];
+  return make_double2(one_product(u.x, v.x, diff), a.shifted ? one_product(u.y, v.y, diff) : 0.0);
 }
 
 // One Stockham stage: butterfly j of a sequence reads elements j + p L/R, multiplies by
@@ -378,11 +355,12 @@ __global__ void __launch_bounds__(kNT) k_axis_fft(const AxisArgs a) {
 __device__ double2 product_value(const double2* __restrict__ Z, int p, long long id, int ix, int iy, int iz,
                                  long long n3, Dims d, double2 ph, bool keep, int dealias) {
   if (!keep) return make_double2(0.0, 0.0);
-  const double2* f = Z + (dealias ? p : p / 2) * n3;
-  const double2 z = f[id], m = mirror_of(f, ix, iy, iz, d);
+  const double2* f = Z + p * n3;
+  const double2 z = f[id];
+  if (!dealias) return z;
+  const double2 m = mirror_of(f, ix, iy, iz, d);
   const double2 re = herm(z, m);                                             // the real part's spectrum
   const double2 im = make_double2(0.5 * (z.y + m.y), -0.5 * (z.x - m.x));    // the imaginary part's
-  if (!dealias) return p % 2 ? im : re;
   const double2 sb = cm(im, make_double2(ph.x, -ph.y));
   return make_double2(0.5 * (re.x + sb.x), 0.5 * (re.y + sb.y));
 }
@@ -723,29 +701,27 @@ double* PR(sns_fft3d* h, int f) { return h->pr + (size_t)f * h->n3; }
 // slots of the working set
 constexpr int kU = 0, kG = 3, kH = 6, kP = 9, kS = 15;
 
-// The packed products' spectra of `nu` spectra (first slot kU) into the slots from kP: the
-// physical fields are formed in kS.
-void product_spectra(sns_fft3d* h, int nu, int shifted, int nprod) {
-  const int nin = shifted ? nu : (nu + 1) / 2, nout = shifted ? nprod : (nprod + 1) / 2;
+// The products' spectra of u (slots kU) into the slots from kP, packed with those on the shifted
+// grid (`shifted`); the physical fields are formed in kS.
+void product_spectra(sns_fft3d* h, int shifted, int nprod) {
   AxisArgs a = axis_args(2, SW(h, kU), SW(h, kS), 1.0 / (double)h->n3);
   a.md = modes_of(h);
-  a.shifted = shifted;
-  launch_axis<kPack>(h, +1, a, nin);
-  launch_axis<kComplex>(h, +1, axis_args(1, SW(h, kS), SW(h, kS)), nin);
-  launch_axis<kComplex>(h, +1, axis_args(0, SW(h, kS), SW(h, kS)), nin);
+  if (shifted) launch_axis<kPack>(h, +1, a, 3);
+  else launch_axis<kComplex>(h, +1, a, 3);
+  launch_axis<kComplex>(h, +1, axis_args(1, SW(h, kS), SW(h, kS)), 3);
+  launch_axis<kComplex>(h, +1, axis_args(0, SW(h, kS), SW(h, kS)), 3);
   a = axis_args(0, SW(h, kS), SW(h, kP));
   a.shifted = shifted;
   a.nprod = nprod;
-  launch_axis<kProduct>(h, -1, a, nout);
-  launch_axis<kComplex>(h, -1, axis_args(1, SW(h, kP), SW(h, kP)), nout);
-  launch_axis<kComplex>(h, -1, axis_args(2, SW(h, kP), SW(h, kP)), nout);
+  launch_axis<kProduct>(h, -1, a, nprod);
+  launch_axis<kComplex>(h, -1, axis_args(1, SW(h, kP), SW(h, kP)), nprod);
+  launch_axis<kComplex>(h, -1, axis_args(2, SW(h, kP), SW(h, kP)), nprod);
 }
 
 // The product of the two fields in slots kU, kU + 1, on both grids, into slot kP.
 void pair_spectrum(sns_fft3d* h) {
   AxisArgs a = axis_args(2, SW(h, kU), SW(h, kS), 1.0 / (double)h->n3);
   a.md = modes_of(h);
-  a.shifted = 1;
   launch_axis<kPack>(h, +1, a, 2);
   launch_axis<kComplex>(h, +1, axis_args(1, SW(h, kS), SW(h, kS)), 2);
   launch_axis<kComplex>(h, +1, axis_args(0, SW(h, kS), SW(h, kS)), 2);
@@ -760,7 +736,7 @@ void pair_spectrum(sns_fft3d* h) {
 // The right-hand side of u (slots kU; full = 0: nonlinear_rhs), or one RK stage on it.
 void stage_device(sns_fft3d* h, FinishArgs f) {
   f.nprod = f.full ? 5 : 6;
-  product_spectra(h, 3, f.dealias, f.nprod);
+  product_spectra(h, f.dealias, f.nprod);
   f.Z = SW(h, kP);
   f.u = SW(h, kU);
   k_finish<<<blocks(h->n3, 256), 256, 0, h->stream>>>(f, h->n3, modes_of(h));
