@@ -792,6 +792,11 @@ void initial_field(sns_handle* h, uint64_t seed, double pert_amp, int pert_kmax)
 template <class F>
 int guarded(sns_handle* h, F&& f) {
   if (h == nullptr) return SNS_ERR_INVALID;
+  auto failed = [h](int code, const char* msg) {
+    h->z_ready = h->y_ready = false;  // whatever the work fields held, later calls overwrite it
+    h->err = msg;
+    return code;
+  };
   try {
     check_inject(h);
     ck(cudaSetDevice(h->device), "cudaSetDevice");
@@ -799,14 +804,11 @@ int guarded(sns_handle* h, F&& f) {
     h->err.clear();
     return SNS_OK;
   } catch (const SnsError& e) {
-    h->err = e.msg;
-    return e.code;
+    return failed(e.code, e.what());
   } catch (const std::bad_alloc&) {
-    h->err = "host allocation failed";
-    return SNS_ERR_NOMEM;
+    return failed(SNS_ERR_NOMEM, "host allocation failed");
   } catch (const std::exception& e) {
-    h->err = e.what();
-    return SNS_ERR_INVALID;
+    return failed(SNS_ERR_INVALID, e.what());
   }
 }
 
