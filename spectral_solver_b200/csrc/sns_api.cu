@@ -118,8 +118,15 @@ void fill_twiddles(int L, double2* tw) {
   }
 }
 
-// Message slot that sns_last_error(NULL) reads: failures of calls made without a handle.
-void set_handleless_error(const char* msg) { g_create_error = msg; }
+// Message slot that sns_last_error(NULL) reads: failures of calls made without a handle.  (The
+// message is dropped when there is no memory for it: this runs where nothing may be thrown.)
+void set_handleless_error(const char* msg) noexcept {
+  try {
+    g_create_error = msg;
+  } catch (...) {
+    g_create_error.clear();
+  }
+}
 
 }  // namespace sns
 

@@ -33,7 +33,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdio>
 #include <exception>
 #include <new>
 #include <string>
@@ -816,34 +815,24 @@ int sns_fft3d_create(int nx, int ny, int nz, double lx, double ly, double lz, sn
   }
   const int n[3] = {nx, ny, nz};
   AxisPlan plans[3];
-  for (int a = 0; a < 3; ++a) {
-    if (!factor(n[a], plans[a])) {
-      sns::set_handleless_error("FFT axis length has too many factors");
-      return SNS_ERR_UNSUPPORTED;
-    }
-    int tw = 8;
-    while (tw > 1 && 2 * (size_t)n[a] * tw * sizeof(double2) > kSmemBudget) tw /= 2;
-    if (2 * (size_t)n[a] * tw * sizeof(double2) > kSmemBudget) {
-      char buf[160];
-      std::snprintf(buf, sizeof buf, "FFT axis length %d is above the %zu points one CTA's shared memory holds", n[a],
-                    kSmemBudget / (2 * sizeof(double2)));
-      sns::set_handleless_error(buf);
-      return SNS_ERR_UNSUPPORTED;
-    }
-    plans[a].tw = tw;
-  }
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    sns::set_handleless_error("no CUDA device visible");
-    return SNS_ERR_NO_DEVICE;
-  }
-  sns_fft3d* h = new (std::nothrow) sns_fft3d();
-  if (h == nullptr) {
-    sns::set_handleless_error("host allocation failed");
-    return SNS_ERR_NOMEM;
-  }
+  sns_fft3d* h = nullptr;
   try {
+    for (int a = 0; a < 3; ++a) {
+      if (!factor(n[a], plans[a])) throw GenericError(SNS_ERR_UNSUPPORTED, "FFT axis length has too many factors");
+      int tw = 8;
+      while (tw > 1 && 2 * (size_t)n[a] * tw * sizeof(double2) > kSmemBudget) tw /= 2;
+      if (2 * (size_t)n[a] * tw * sizeof(double2) > kSmemBudget)
+        throw GenericError(SNS_ERR_UNSUPPORTED, "FFT axis length " + std::to_string(n[a]) + " is above the " +
+                                                    std::to_string(kSmemBudget / (2 * sizeof(double2))) +
+                                                    " points one CTA's shared memory holds");
+      plans[a].tw = tw;
+    }
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+      cudaGetLastError();
+      throw GenericError(SNS_ERR_NO_DEVICE, "no CUDA device visible");
+    }
+    h = new sns_fft3d();
     gck(cudaGetDevice(&h->device), "cudaGetDevice");
     h->d = Dims{nx, ny, nz};
     h->len[0] = lx;
@@ -880,6 +869,10 @@ int sns_fft3d_create(int nx, int ny, int nz, double lx, double ly, double lz, sn
     sns::set_handleless_error(e.msg.c_str());
     release(h);
     return e.code;
+  } catch (const std::exception&) {  // std::bad_alloc
+    sns::set_handleless_error("host allocation failed");
+    release(h);
+    return SNS_ERR_NOMEM;
   }
   *out = h;
   return SNS_OK;

@@ -178,7 +178,7 @@ int reset_handle(sns_handle* h, double nu, uint64_t seed, double pert_amp, int p
 
 // Host helpers shared by the C-ABI files (sns_api.cu).
 void fill_twiddles(int L, double2* tw);        // exp(-2*pi*i*t/L), t < L
-void set_handleless_error(const char* msg);    // message for sns_last_error(NULL)
+void set_handleless_error(const char* msg) noexcept;  // message for sns_last_error(NULL)
 
 constexpr int kXDiagPartials = 2;   // (sum 0.5|u|^2, max |u|^2) per row
 constexpr int kSpecDiagPartials = 2;  // (sum w*|H(omega)|^2, max |k.u|) per block
