@@ -251,6 +251,14 @@ size_t comp_bytes(int n, int precision) {
   return (size_t)3 * n * n * sns::pitch_for(n, 8) * sizeof(sns::CompWord);
 }
 
+// Nyquist-plane partial sums per product field: one per CTA of the x pass, up to N^2 / 4 of them on
+// small grids.  kPersistentCtas bounds the persistent x passes' (two CTAs on each of 148 SMs).
+constexpr int kPersistentCtas = 512;
+size_t nyq_slots(int n, int precision) {
+  const sns::SmallOps* o = small_rule(n) ? sns::small_for(n, precision) : nullptr;
+  return (size_t)std::max(o ? std::max(o->nparts, o->rparts) : 1, n >= 128 ? kPersistentCtas : 1);
+}
+
 size_t partial_slots(int n) {
   const size_t rows = (size_t)n * n;
   return 2 * rows + 4096;
@@ -920,8 +928,8 @@ int sns_grid_supported(int n) { return n > 0 && sns::ops_for(n, 0) != nullptr ? 
 size_t sns_bytes_required(int n, int precision) {
   if (n <= 0 || (precision != SNS_PRECISION_FP64 && precision != SNS_PRECISION_FP32)) return 0;
   return 18 * field_bytes(n, precision) + comp_bytes(n, precision) + partial_slots(n) * sizeof(double) +
-         (size_t)(4 * n + 64) * complex_bytes(precision) + (size_t)n * (n / 16 + 1) * sizeof(int) +
-         2 * sns::kClockWords * sizeof(double);
+         12 * nyq_slots(n, precision) * sizeof(double) + (size_t)(5 * n + 64) * complex_bytes(precision) +
+         (size_t)n * (n / 16 + 1) * sizeof(int) + 2 * sns::kClockWords * sizeof(double);
 }
 
 int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed, double pert_amp, int pert_kmax,
@@ -1025,8 +1033,8 @@ int sns_create(int n, double nu, int precision, int viscous_mode, uint64_t seed,
       h->small = sns::small_for(n, precision);
       h->small->init();
     }
-    const int nparts = std::max(std::max(1, h->x2_grid), h->small ? std::max(h->small->nparts, h->small->rparts) : 1);
-    alloc((void**)&h->nyq_part, (size_t)12 * nparts * sizeof(double));
+    const size_t slots = std::max(nyq_slots(n, precision), (size_t)h->x2_grid);
+    alloc((void**)&h->nyq_part, 12 * slots * sizeof(double));
     alloc((void**)&h->tw2, (size_t)n * h->cbytes);
     {
       // tw2[r*16 + j] = exp(-2*pi*i*r*j/n) for r < n/16, j < 16
