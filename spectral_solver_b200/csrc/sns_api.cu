@@ -529,7 +529,7 @@ void run_stage_small(sns_handle* h, char* u_src, char* g_buf, int stage, double 
   else o->xpass(h->work, u_src, h->phase, h->tw, h->inv_size(), h->nyq_part, 0, h->g, st);
   mark(pm, 3, st);
   mark(pm, 4, st);
-  o->yfwd(h->work, h->tw, rot, h->g, st);
+  o->yfwd(h->work, h->tw, rot ? 6 : 10, h->g, st);
   mark(pm, 5, st);
   mark(pm, 6, st);
   h->y_ready = false;
@@ -541,7 +541,7 @@ void run_stage_small(sns_handle* h, char* u_src, char* g_buf, int stage, double 
 
 // One RK3 stage (or the RHS only, mode 1; the unprojected nonlinear term, mode 2) on u_src: the
 // five fused passes.  The projected forms run on 5 products (the squares less u_2^2, a
-// gradient's difference that the projection removes), mode 2 on all 6, as separate kernels.
+// gradient's difference that the projection removes), mode 2 on all 6.
 void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, int mode, char* rhs_out,
                PassMarks* pm = nullptr) {
   // (the rotational form has one nonlinear term for every mode)
@@ -560,7 +560,9 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   const int tiles_in = h->nyq_clean ? h->tiles_data() : h->tiles_all();
   const int f_src = (int)((size_t)(u_src - h->state) / h->fbytes);  // u (0) or the g slot (3)
   const int np = mode == 2 ? 6 : 5;
-  const bool fused = h->p5_grid > 0 && np == 5;
+  // mode 2 on a small grid: the z and y passes of its own stage, on all pencils
+  const bool small = h->small && h->nyq_clean;
+  const bool fused = h->p5_grid > 0;
   // Sphere pruning (RK update with the fused P5 only).  A column-block tile (my, cb) outside
   // the disk 4 ((cb * TW)^2 + my^2) <= N^2 holds only modes outside the sphere: u is zero
   // there before the stage (sphere_known) and the stage leaves it zero.  So P5 neither loads,
@@ -570,13 +572,15 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
   const bool clean = mode == 0 && h->nyq_clean && h->nlive > 0 && sphere_known(h, stage);
   const bool prune = fused && clean;
   mark(pm, 0, st);
-  yz_pass(h, h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), clean);
+  if (small) h->small->zphase(u_src, h->work, h->phase, h->tw, h->inv_size(), 0, 0, g, st);
+  else yz_pass(h, h->map_state_z, 2, +1, 1, tma_args(h, f_src, 3, tiles_in, h->work, 0, h->inv_size()), clean);
   mark(pm, 1, st);
-  yz_pass(h, h->map_work_y, 1, +1, 0, tma_args(h, 0, 6, tiles_in, h->work, 0, 1.0), clean);
+  if (small) h->small->yinv(h->work, h->tw, 2, 0, g, st);
+  else yz_pass(h, h->map_work_y, 1, +1, 0, tma_args(h, 0, 6, tiles_in, h->work, 0, 1.0), clean);
   mark(pm, 2, st);
   int nparts = 1;
-  if (h->x2_grid > 0 && np == 5) {
-    o->xpass2(h->work, u_src, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->nyq_part, h->tw2, g, h->x2_grid,
+  if (h->x2_grid > 0) {
+    o->xpass2(h->work, np, u_src, h->phase, h->inv_size(), h->nyq_clean ? 1 : 0, h->nyq_part, h->tw2, g, h->x2_grid,
               h->err_word, st);
     nparts = h->x2_grid;
     mark(pm, 3, st);
@@ -586,14 +590,15 @@ void run_stage(sns_handle* h, char* u_src, char* g_buf, int stage, double dt, in
     o->nyq_reduce(h->work, 2 * np, h->nyq_part, g, st);
   }
   mark(pm, 4, st);
-  yz_pass(h, h->map_work_y, 1, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0));
+  if (small) h->small->yfwd(h->work, h->tw, 2 * np, g, st);
+  else yz_pass(h, h->map_work_y, 1, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 5, st);
   if (!fused)
     yz_pass(h, h->map_work_z, 2, -1, 0, tma_args(h, 0, 2 * np, h->tiles_data(), h->work, 0, 1.0));
   mark(pm, 6, st);
   const sns::SweepArgs a = stage_args(h, stage, dt, mode, u_src);
   if (fused)
-    h->p5->run(h->map_work_z, h->map_p5_state, f_src, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->tw, h->phase, a,
+    h->p5->run(h->map_work_z, h->map_p5_state, np, f_src, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->tw, h->phase, a,
                h->tiles_data(), prune ? h->live : nullptr, prune ? h->nlive : 0, g, h->p5_grid, h->err_word, st);
   else
     o->sweep(h->work, np, u_src, g_buf, rhs_out, h->nyq_part, nparts, h->phase, a, g, st);

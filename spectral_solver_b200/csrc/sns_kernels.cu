@@ -415,7 +415,7 @@ k_xpass_products(C* __restrict__ work, const C* __restrict__ unyq, const C* __re
 // group is done, its staging buffer is refilled) and between the inverse and forward
 // FFTs (each product reads two components).
 // The (N/2,0,0) sums of the 12 product planes accumulate in registers per CTA.
-template <int N, class C>
+template <int N, class C, int PRODUCTS = 5>
 struct XP {
   static constexpr int M = N / 16;                 // stage-B radix
   static constexpr bool PAIR = (M == 32);          // radix 32 as two radix-16 halves + shuffle
@@ -425,14 +425,14 @@ struct XP {
   // warps busy in the inverse stages but one CTA per SM, measured slower)
   static constexpr int ROWS = (N == 256) ? 2 : 1;
   static constexpr int SP = N + N / 16;            // padded sequence (one slot per 16)
-  static constexpr int NP = 5;                     // products (u_2^2 subtracted from the squares)
+  static constexpr int NP = PRODUCTS;              // 5 (u_2^2 subtracted from the squares) or 6
   static constexpr int NT = 32 * NP;               // one warp (half-warp per row at N = 256) per product
   // resident CTAs per SM the register budget is built for
   static constexpr int MINB = 2;
   // staged row of one field: NH + 1 values rounded up to 16 bytes (the bulk-copy unit)
   static constexpr int RS = (int)(((NH + 1) * sizeof(C) + 15) / 16 * 16 / sizeof(C));
   static constexpr int ROWIN = 6 * RS;
-  static constexpr int STG = (ROWIN > 2 * SP ? ROWIN : 2 * SP);
+  static constexpr int STG = (ROWIN > (NP - 3) * SP ? ROWIN : (NP - 3) * SP);
   static constexpr uint32_t kRowBytes = RS * sizeof(C);
   static constexpr size_t smem = (size_t)(2 * ROWS * STG + ROWS * 6 * SP + N) * sizeof(C) + 128 +
                                  2 * sizeof(uint64_t);
@@ -440,12 +440,12 @@ struct XP {
 
 __device__ __forceinline__ int pp16(int e) { return e + (e >> 4); }
 
-template <int N, class C>
-__global__ void __launch_bounds__(XP<N, C>::NT, XP<N, C>::MINB)
+template <int N, class C, int NP = 5>
+__global__ void __launch_bounds__(XP<N, C, NP>::NT, XP<N, C, NP>::MINB)
 k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__ phase,
          double scale, int nyq_scalar, double* __restrict__ nyq_part, const C* __restrict__ tw2_g, Geom g,
          int* err) {
-  using X = XP<N, C>;
+  using X = XP<N, C, NP>;
   constexpr int M = X::M, NH = X::NH, ROWS = X::ROWS, SP = X::SP, STG = X::STG, RS = X::RS;
   extern __shared__ unsigned char smraw[];
   __shared__ int s_fail;
@@ -585,9 +585,8 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
       {
         // forward stage A: products fused into the loads
         const int t = tid % M, ab = (tid / M) % X::NP, r = r0 + tid / (X::NP * M);
-        // 00 - 22, 01, 02, 11 - 22, 12
-        const bool sq = ab == 0 || ab == 3;
-        const int ca = ab >= 3 ? 1 : 0, cb = (sq || ab == 4) ? 2 : ab;
+        int ca, cb;
+        const bool sq = product_pair<NP>(ab, &ca, &cb);
         const C* Za = W + (r * 6 + 3 + ca) * SP;
         const C* Zb = W + (r * 6 + 3 + cb) * SP;
         C v[16];
@@ -720,7 +719,7 @@ k_xpass2(C* __restrict__ work, const C* __restrict__ unyq, const C* __restrict__
 //                    W_N^(j k1) / 2 (the r2c unpack's factor 1/2, exact); out to P[ab][j][k1]
 //   forward stage B  lane k1: the 16-point DFT over j, outputs k1 + M k2; r2c unpack of the
 //                    two grids through the partner lane (N - k), 128-byte stores to HBM
-// The products run in two parts (00 - 22, 01, 02, then 11 - 22, 12), each through Wc and its
+// The products run in two parts (00 - 22, 01, 02, then 11 - 22, 12; NP = 6: 00, 01, 02, then the rest), each through Wc and its
 // forward stage B, so a warp holds one staged row group and one transposition buffer.  Every
 // transposition goes through shared memory once, XOR-swizzled (no bank conflicts); the
 // products never do.  The kernel is bound by instruction issue, so its complex additions run
@@ -739,7 +738,7 @@ struct XW {
   static constexpr uint32_t kRowBytes = RS * sizeof(C);
   static constexpr int TWT = 16 * 32;     // four-step twiddles [i][lane], then the same halved
   static constexpr size_t smem = (size_t)(WARPS * PER_WARP + 2 * TWT) * sizeof(C) + 128 +
-                                 WARPS * (sizeof(uint64_t) + R * 10 * sizeof(double));
+                                 WARPS * (sizeof(uint64_t) + R * 12 * sizeof(double));
   static_assert(R * M == 32, "a warp covers its rows' lanes");
 };
 
@@ -748,7 +747,7 @@ struct XW {
 // sequences u_0 + i u_1 and u_2 meet in registers, each row's sum of |u|^2 / 2 and max of
 // |u|^2 are reduced over its lanes, and the CTA's totals (rows in a fixed order per warp,
 // warps in order) go to part[2 cta], part[2 cta + 1].
-template <int N, bool DIAG = false>
+template <int N, bool DIAG = false, int NP = 5>
 __global__ void __launch_bounds__(32 * XW<N>::WARPS, 1)
 k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const float2* __restrict__ phase, double scale,
           int nyq_scalar, double* __restrict__ nyq_part, const float2* __restrict__ tw2_g, Geom g, int* err) {
@@ -766,8 +765,8 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
   C* const twh = twt + X::TWT;                   // [16][32], times 1/2
   uint64_t* const bar = reinterpret_cast<uint64_t*>(twh + X::TWT) + warp;
   double* const s_nyq = reinterpret_cast<double*>(reinterpret_cast<uint64_t*>(twh + X::TWT) + X::WARPS);
-  double* const my_nyq = s_nyq + warp * R * 10;  // [WARPS][R][10]
-  for (int e = lane; e < R * 10; e += 32) my_nyq[e] = 0.0;
+  double* const my_nyq = s_nyq + warp * R * 2 * NP;  // [WARPS][R][2 NP]
+  for (int e = lane; e < R * 2 * NP; e += 32) my_nyq[e] = 0.0;
   if (lane == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -949,16 +948,15 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
 
 #pragma unroll
     for (int half = 0; half < (DIAG ? 0 : 2); ++half) {
-      const int ab0 = 3 * half, ab1 = half ? 5 : 3;
+      const int ab0 = 3 * half, ab1 = half ? NP : 3;
       // ---- products and forward stage A: P[ab % 3][j][k1] in Wc at pslot(j, k1, row)
 #pragma unroll
       for (int p = 0; p < MP; ++p) {
         const int rB = row_b(p);
 #pragma unroll
         for (int ab = ab0; ab < ab1; ++ab) {
-          // 00 - 22, 01, 02, 11 - 22, 12
-          const bool sq = ab == 0 || ab == 3;
-          const int ca = ab >= 3 ? 1 : 0, cb = (sq || ab == 4) ? 2 : ab;
+          int ca, cb;
+          const bool sq = product_pair<NP>(ab, &ca, &cb);
           C v[NZ];
 #pragma unroll
           for (int q = 0; q < NZ; ++q) {
@@ -1016,8 +1014,8 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
               o0[SNS_IDX(kk, g.pitch)] = A;
               o1[SNS_IDX(kk, g.pitch)] = B;
               if (kk == NH) {
-                my_nyq[r * 10 + 2 * ab] += A.x;
-                my_nyq[r * 10 + 2 * ab + 1] += B.x;
+                my_nyq[r * 2 * NP + 2 * ab] += A.x;
+                my_nyq[r * 2 * NP + 2 * ab + 1] += B.x;
               }
             }
           }
@@ -1053,10 +1051,10 @@ k_xpass_w(float2* __restrict__ work, const float2* __restrict__ unyq, const floa
   }
   // per-CTA Nyquist partials, fixed order: [field][cta]
   __syncthreads();
-  if (tid < 10) {
+  if (tid < 2 * NP) {
     double s = 0.0;
 #pragma unroll 1
-    for (int w = 0; w < X::WARPS * R; ++w) s += s_nyq[w * 10 + tid];
+    for (int w = 0; w < X::WARPS * R; ++w) s += s_nyq[w * 2 * NP + tid];
     nyq_part[tid * gridDim.x + blockIdx.x] = s;
   }
 }
@@ -1774,15 +1772,22 @@ struct Launch {
     k<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(F(work), F(u), F(gbuf), F(rhs), nyq_part, nparts, F(phase), a,
                                                        g);
   }
-  static void xpass2(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar, double* nyq_part,
-                     const void* tw2, Geom g, int grid, int* err, cudaStream_t st) {
+  template <int NP>
+  static void xpass2_launch(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar,
+                            double* nyq_part, const void* tw2, Geom g, int grid, int* err, cudaStream_t st) {
     if constexpr ((N == 128 || N == 256 || N == 512) && std::is_same_v<C, float2>) {
-      k_xpass_w<N><<<grid, 32 * XW<N>::WARPS, XW<N>::smem, st>>>(F(work), F(unyq), F(phase), scale, nyq_scalar,
-                                                                 nyq_part, F(tw2), g, err);
+      k_xpass_w<N, false, NP><<<grid, 32 * XW<N>::WARPS, XW<N>::smem, st>>>(F(work), F(unyq), F(phase), scale,
+                                                                            nyq_scalar, nyq_part, F(tw2), g, err);
     } else if constexpr (N == 256 || N == 512) {
-      k_xpass2<N, C><<<grid, XP<N, C>::NT, XP<N, C>::smem, st>>>(F(work), F(unyq), F(phase), scale, nyq_scalar,
-                                                                  nyq_part, F(tw2), g, err);
+      using X = XP<N, C, NP>;
+      k_xpass2<N, C, NP><<<grid, X::NT, X::smem, st>>>(F(work), F(unyq), F(phase), scale, nyq_scalar, nyq_part,
+                                                       F(tw2), g, err);
     }
+  }
+  static void xpass2(void* work, int np, const void* unyq, const void* phase, double scale, int nyq_scalar,
+                     double* nyq_part, const void* tw2, Geom g, int grid, int* err, cudaStream_t st) {
+    auto launch = np == 6 ? xpass2_launch<6> : xpass2_launch<5>;
+    launch(work, unyq, phase, scale, nyq_scalar, nyq_part, tw2, g, grid, err, st);
   }
   // Persistent grid of the two-stage x pass (0: this size uses the generic x pass).
   static int xpass2_grid(int nsm) {
@@ -1884,9 +1889,13 @@ struct Launch {
   static void init() {
     if constexpr ((N == 128 || N == 256 || N == 512) && std::is_same_v<C, float2>) {
       set_smem(k_xpass_w<N>, XW<N>::smem);
+      set_smem(k_xpass_w<N, false, 6>, XW<N>::smem);
       set_smem(k_xpass_w<N, true>, XW<N>::smem);
     }
-    else if constexpr (N == 256 || N == 512) set_smem(k_xpass2<N, C>, XP<N, C>::smem);
+    else if constexpr (N == 256 || N == 512) {
+      set_smem(k_xpass2<N, C>, XP<N, C>::smem);
+      set_smem(k_xpass2<N, C, 6>, XP<N, C, 6>::smem);
+    }
     set_smem(k_yz_tma<N, 1, -1, 0, C>, tma_smem<N, C>());
     if constexpr (kAllYz) {
       set_smem(k_yz_tma<N, 2, +1, 1, C>, tma_smem<N, C>());

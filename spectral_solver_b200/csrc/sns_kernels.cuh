@@ -110,9 +110,10 @@ struct Ops {
   void (*yz_tma)(const CUtensorMap& map, int axis, int dir, int variant, TmaArgs a, const void* tw,
                  const void* phase, Geom g, int grid, cudaStream_t st);
   int (*tma_blocks_per_sm)();
-  // two-stage persistent x pass (N = 256, 512), 5 products; writes [10][grid] Nyquist partials
-  void (*xpass2)(void* work, const void* unyq, const void* phase, double scale, int nyq_scalar, double* nyq_part,
-                 const void* tw2, Geom g, int grid, int* err, cudaStream_t st);
+  // two-stage persistent x pass (N = 256, 512; FP32 128 too), np products as xpass_products;
+  // writes [2 np][grid] Nyquist partials
+  void (*xpass2)(void* work, int np, const void* unyq, const void* phase, double scale, int nyq_scalar,
+                 double* nyq_part, const void* tw2, Geom g, int grid, int* err, cudaStream_t st);
   int (*xpass2_grid)(int nsm);
   // rotational form: omega_hat = i k x u_hat (3 fields); the x pass forming u x omega on both
   // grids (12 inputs -> 6 outputs in work fields 0..5); the sweep combining the two grids

@@ -1,4 +1,4 @@
-// P5 of the large grids (N = 256, 512): forward z pass of the 10 product fields and the whole
+// P5 of the large grids (N = 256, 512): forward z pass of the 10 (12) product fields and the whole
 // k-space sweep in one persistent kernel, so the transformed products never return to HBM.
 //
 // A tile is 128 bytes of columns (TW = 8 complex doubles or 16 complex floats) x all mz at one
@@ -7,7 +7,7 @@
 // of three shared-memory slots, each
 // filled by TMA while the two before it are worked on:
 //   units 0 .. 9   : the product fields, the plain grid's five first (work fields 0, 2, .. 8),
-//                    then the shifted grid's (1, 3, .. 9)
+//                    then the shifted grid's (1, 3, .. 9); six each for the unprojected term
 //   units 10 .. 17 : the state of an eighth of the tile's rows: u, and g after the first stage
 // so memory is read at every moment, also while the sweep computes and stores.
 //
@@ -38,7 +38,7 @@ namespace {
 // The self-conjugate mode (N/2, 0, 0): one warp sums the x pass's per-CTA plane sums in a
 // fixed order and runs the sweep on that single mode (column N/2 of row 0, which no P5 tile
 // touches).
-template <int N, class C>
+template <int N, class C, int NP>
 __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restrict__ gbuf, C* __restrict__ rhs,
                                                  const double* __restrict__ nyq_part, int nparts,
                                                  const C* __restrict__ phase, SweepArgs a0, Geom g) {
@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restric
   constexpr int NH = N / 2;
   const int tid = threadIdx.x;
   const bool load_g = a.stage > 0;
-  double part[10];
+  double part[2 * NP];
 #pragma unroll
-  for (int f = 0; f < 10; ++f) {
+  for (int f = 0; f < 2 * NP; ++f) {
     double acc = 0.0;
     for (int i = tid; i < nparts; i += 32) acc += nyq_part[f * nparts + i];
 #pragma unroll
@@ -56,9 +56,9 @@ __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restric
     part[f] = acc;
   }
   if (tid != 0) return;
-  ModeIn<C, 5> in;
+  ModeIn<C, NP> in;
 #pragma unroll
-  for (int p = 0; p < 5; ++p) {
+  for (int p = 0; p < NP; ++p) {
     in.p0[p] = cmk((real_of<C>)part[2 * p], real_of<C>(0));
     in.ps[p] = cmk((real_of<C>)part[2 * p + 1], real_of<C>(0));
   }
@@ -83,8 +83,9 @@ __global__ void __launch_bounds__(32) k_nyq_mode(C* __restrict__ u, C* __restric
   }
 }
 
-template <int N, class C>
+template <int N, class C, int PRODUCTS = 5>
 struct P5 {
+  static constexpr int NP = PRODUCTS;
   static constexpr int TW = (int)(128 / sizeof(C));
   static constexpr int LTW = TW == 16 ? 4 : 3;
   static constexpr int R2 = N / 16;
@@ -95,7 +96,7 @@ struct P5 {
   static constexpr int NCH = 8;                 // state units of a tile
   static constexpr int QC = M / NCH;            // modes of a thread per state unit
   static constexpr int CR = 16 * QC;            // consecutive rows of a state unit (H such runs)
-  static constexpr int kF = 10, kU = kF + NCH;  // units of a tile
+  static constexpr int kF = 2 * NP, kU = kF + NCH;  // units of a tile
   static constexpr int SLOTS = 3;
   static constexpr int TILE = TW * N;
   static constexpr uint32_t kTileBytes = 128u * N;
@@ -113,15 +114,15 @@ struct P5 {
   static_assert(6 * H * CR * TW <= TILE, "a state unit fits a slot");
 };
 
-template <int N, class C>
+template <int N, class C, int PRODUCTS = 5>
 __global__ void __launch_bounds__(P5<N, C>::NT, P5<N, C>::MINB)
 k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap smap, int f_u, C* __restrict__ u,
      C* __restrict__ gbuf, C* __restrict__ rhs, const C* __restrict__ tw, const C* __restrict__ phase, SweepArgs a0,
      int ncb, const int* __restrict__ live, int nlive, Geom g, int* err) {
-  using P = P5<N, C>;
+  using P = P5<N, C, PRODUCTS>;
   using RT = real_of<C>;
   constexpr int NT = P::NT, TW = P::TW, R2 = P::R2, M = P::M, CW = P::CW, WPC = P::WPC, TILE = P::TILE, NH = N / 2;
-  constexpr int QC = P::QC, CR = P::CR, H = P::H, kF = P::kF, kU = P::kU, SLOTS = P::SLOTS;
+  constexpr int QC = P::QC, CR = P::CR, H = P::H, NP = P::NP, kF = P::kF, kU = P::kU, SLOTS = P::SLOTS;
   const SweepArgs a = resolve_step(a0);
   extern __shared__ unsigned char smraw[];
   __shared__ uint32_t s_tmem;
@@ -168,7 +169,7 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
     }
     C* const dst = ring + ib * TILE;
     if (ik < kF) {
-      const int f = ik < 5 ? 2 * ik : 2 * (ik - 5) + 1;
+      const int f = ik < NP ? 2 * ik : 2 * (ik - NP) + 1;
       mbar_arrive_expect_tx(&bars[ib], P::kTileBytes);
 #pragma unroll
       for (int i = 0; i < N / P::BR; ++i)
@@ -284,15 +285,17 @@ k_p5(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMa
       using I0 = std::integral_constant<int, 0>;
       using I1 = std::integral_constant<int, 1>;
       using I2 = std::integral_constant<int, 2>;
-      const bool f0 = k < 5;  // r_x, r_y, r_z are first touched by 00, 01, 02 of the plain grid
-      switch (k < 5 ? k : k - 5) {
-        case 0: add(I0{}, I0{}, f0); break;                             // 00 - 22
+      const bool f0 = k < NP;  // r_x, r_y, r_z are first touched by 00, 01, 02 of the plain grid
+      switch (k < NP ? k : k - NP) {
+        case 0: add(I0{}, I0{}, f0); break;                             // 00 (less 22 of 5)
         case 1: add(I0{}, I1{}, false); add(I1{}, I0{}, f0); break;     // 01
         case 2: add(I0{}, I2{}, false); add(I2{}, I0{}, f0); break;     // 02
-        case 3: add(I1{}, I1{}, false); break;                          // 11 - 22
-        default: add(I1{}, I2{}, false); add(I2{}, I1{}, false); break; // 12
+        case 3: add(I1{}, I1{}, false); break;                          // 11 (less 22 of 5)
+        case 4: add(I1{}, I2{}, false); add(I2{}, I1{}, false); break;  // 12
+        default:
+          if constexpr (NP == 6) add(I2{}, I2{}, false);                // 22
       }
-      if (k == 4) {  // the plain grid's part takes the phase before the shifted grid's comes
+      if (k == NP - 1) {  // the plain grid's part takes the phase before the shifted grid's comes
         tmem_wait_st();
 #pragma unroll 1
         for (int q0 = 0; q0 < M; q0 += 4) {
@@ -403,10 +406,15 @@ struct LaunchP5 {
   using P = P5<N, C>;
   static C* F(void* p) { return static_cast<C*>(p); }
   static const C* F(const void* p) { return static_cast<const C*>(p); }
-  static void init() {
-    cudaFuncSetAttribute(k_p5<N, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem);
-    cudaFuncSetAttribute(k_p5<N, C>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  template <int NP>
+  static void prepare() {
+    cudaFuncSetAttribute(k_p5<N, C, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem);
+    cudaFuncSetAttribute(k_p5<N, C, NP>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);
+  }
+  static void init() {
+    prepare<5>();
+    prepare<6>();
   }
   // The runtime's occupancy query reports one CTA per SM for a tensor-memory kernel whatever
   // its allocation, so residency is computed from the kernel's own limits: shared memory,
@@ -428,12 +436,19 @@ struct LaunchP5 {
     nb = std::min(nb, thr_sm / P::NT);
     return nsm * (nb < 1 ? 1 : nb);
   }
-  static void run(const CUtensorMap& work, const CUtensorMap& state, int f_u, void* u, void* gbuf, void* rhs,
+  template <int NP>
+  static void go(const CUtensorMap& work, const CUtensorMap& state, int f_u, void* u, void* gbuf, void* rhs,
+                 const double* nyq_part, int nparts, const void* tw, const void* phase, SweepArgs a, int ncb,
+                 const int* live, int nlive, Geom g, int grid, int* err, cudaStream_t st) {
+    k_nyq_mode<N, C, NP><<<1, 32, 0, st>>>(F(u), F(gbuf), F(rhs), nyq_part, nparts, F(phase), a, g);
+    k_p5<N, C, NP><<<grid, P::NT, P::smem, st>>>(work, state, f_u, F(u), F(gbuf), F(rhs), F(tw), F(phase), a, ncb,
+                                                 live, nlive, g, err);
+  }
+  static void run(const CUtensorMap& work, const CUtensorMap& state, int np, int f_u, void* u, void* gbuf, void* rhs,
                   const double* nyq_part, int nparts, const void* tw, const void* phase, SweepArgs a, int ncb,
                   const int* live, int nlive, Geom g, int grid, int* err, cudaStream_t st) {
-    k_nyq_mode<N, C><<<1, 32, 0, st>>>(F(u), F(gbuf), F(rhs), nyq_part, nparts, F(phase), a, g);
-    k_p5<N, C><<<grid, P::NT, P::smem, st>>>(work, state, f_u, F(u), F(gbuf), F(rhs), F(tw), F(phase), a, ncb, live,
-                                             nlive, g, err);
+    auto launch = np == 6 ? go<6> : go<5>;
+    launch(work, state, f_u, u, gbuf, rhs, nyq_part, nparts, tw, phase, a, ncb, live, nlive, g, grid, err, st);
   }
   static const P5Ops* table() {
     static const P5Ops ops = {init, grid, P::CR, run};

@@ -13,8 +13,8 @@ struct P5Ops {
   // work: z-pencil map of the work fields (128 bytes x up to 256 rows); state: the same of
   // u[3], g[3] with chunk_rows rows; f_u: the field u_src is in it (0, or 3 for a state in
   // the g slots); `live` (nlive entries of my * ncb + cb) restricts the pass to those tiles,
-  // null: all
-  void (*run)(const CUtensorMap& work, const CUtensorMap& state, int f_u, void* u, void* gbuf, void* rhs,
+  // null: all; np = 6: all six products (the unprojected nonlinear term, a.mode 2), else 5
+  void (*run)(const CUtensorMap& work, const CUtensorMap& state, int np, int f_u, void* u, void* gbuf, void* rhs,
               const double* nyq_part, int nparts, const void* tw, const void* phase, SweepArgs a, int ncb,
               const int* live, int nlive, Geom g, int grid, int* err, cudaStream_t st);
 };

@@ -448,8 +448,7 @@ k_ysmall(C* work, const C* __restrict__ tw, int clean, Geom g) {
   C* const buf = s_tw + N;
   const int tid = threadIdx.x, mx0 = blockIdx.x * TW;
   const long long plane = (long long)blockIdx.y * N;
-  // groups 0, 1: fields 0, 2, .. and 1, 3, ..; groups 2, 3 (the rotational form's vorticity):
-  // fields 6, 8, 10 and 7, 9, 11
+  // groups 0, 1: fields 0, 2, .. and 1, 3, ..; groups 2, 3 (12 fields): 6, 8, 10 and 7, 9, 11
   C* const fld = work + (long long)(blockIdx.z < 2 ? blockIdx.z : blockIdx.z + 4) * g.field;
   for (int t = tid; t < N; t += NT) s_tw[t] = tw[t];
   predecessor_wait();
@@ -954,11 +953,11 @@ struct Small {
     using Y = YT<N, C, +1, 3>;
     launch(k_ysmall<N, C, +1, 3>, dim3(Y::NCB, N, groups), Y::NT, Y::smem, st, F(work), F(tw), clean, g);
   }
-  static void yfwd(void* work, const void* tw, int rot, Geom g, cudaStream_t st) {
+  static void yfwd(void* work, const void* tw, int fields, Geom g, cudaStream_t st) {
     using Y5 = YT<N, C, -1, 5>;
     using Y3 = YT<N, C, -1, 3>;
-    if (rot) launch(k_ysmall<N, C, -1, 3>, dim3(Y3::NCB, N, 2), Y3::NT, Y3::smem, st, F(work), F(tw), 0, g);
-    else launch(k_ysmall<N, C, -1, 5>, dim3(Y5::NCB, N, 2), Y5::NT, Y5::smem, st, F(work), F(tw), 0, g);
+    if (fields == 10) launch(k_ysmall<N, C, -1, 5>, dim3(Y5::NCB, N, 2), Y5::NT, Y5::smem, st, F(work), F(tw), 0, g);
+    else launch(k_ysmall<N, C, -1, 3>, dim3(Y3::NCB, N, fields / 3), Y3::NT, Y3::smem, st, F(work), F(tw), 0, g);
   }
   static void xrot(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part, Geom g,
                    cudaStream_t st) {

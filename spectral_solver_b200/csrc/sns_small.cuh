@@ -20,14 +20,14 @@ struct SmallOps {
   // vorticity shifted); the x pass to
   // the 10 product half spectra, [10][nparts] Nyquist sums in `part` (diag: nparts
   // (sum |u|^2 / 2, max |u|^2) pairs instead, work unchanged); the rotational
-  // form's x pass (12 fields -> the 6 of u x omega, [6][rparts] sums); forward y of the 10 (6)
-  // fields
+  // form's x pass (12 fields -> the 6 of u x omega, [6][rparts] sums); forward y of the first
+  // `fields` (6, 10 or 12)
   void (*yinv)(void* work, const void* tw, int groups, int clean, Geom g, cudaStream_t st);
   void (*xpass)(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part, int diag,
                 Geom g, cudaStream_t st);
   void (*xrot)(void* work, const void* unyq, const void* phase, const void* tw, double scale, double* part, Geom g,
                cudaStream_t st);
-  void (*yfwd)(void* work, const void* tw, int rot, Geom g, cudaStream_t st);
+  void (*yfwd)(void* work, const void* tw, int fields, Geom g, cudaStream_t st);
   // forward z, the sweep (prune: tiles outside the sphere are skipped) and, with emit, the
   // next stage's zphase
   void (*zsweep)(void* work, void* u, void* gbuf, void* rhs, const double* part, int nparts, const void* phase,

@@ -24,6 +24,15 @@ __device__ __forceinline__ C diff_squares(C a, C b) {
   return cmk((a.x - b.x) * (a.x + b.x), (a.y - b.y) * (a.y + b.y));
 }
 
+// Product ab of NP: a u_a u_b, or (NP = 5, `sq`) u_a^2 - u_b^2: 00 - 22, 01, 02, 11 - 22, 12.
+template <int NP>
+__device__ __forceinline__ bool product_pair(int ab, int* a, int* b) {
+  const bool sq = NP == 5 && (ab == 0 || ab == 3);
+  *a = ab < 3 ? 0 : (ab < 5 ? 1 : 2);
+  *b = sq ? 2 : (ab < 3 ? ab : (ab < 5 ? ab - 2 : 2));
+  return sq;
+}
+
 // ------------------------------------------------------------------------------------
 // P5 sweep: per mode, the reference's accumulate (:926-936), add_viscous_project
 // (:955-974), RK stage update (:994-1033) and project_truncate (:825-844).
@@ -145,9 +154,8 @@ __device__ __forceinline__ void finish_mode(C r[3], int ix, int iy, int iz, int 
   const double inv = 1.0 / k2;
   const RT rinv = (RT)inv;
   if (a.mode == 2) {  // nonlinear term only: masked, neither viscous term nor projection
-    rr[0] = r[0];
-    rr[1] = r[1];
-    rr[2] = r[2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) rr[c] = keep ? r[c] : czero<C>();
     return;
   }
   if (!a.visc_if) {
