@@ -221,12 +221,13 @@ int sns_batch_size(const sns_batch* b);
 const char* sns_batch_last_error(const sns_batch* b);
 
 /* Launch-shape autotuner (no counterpart in the reference).  Times the pass variants a
- * handle can run -- the x pass as the two-stage 16 x M plan or the generic Stockham plan
- * (N = 256, 512), the forward z pass fused with the k-space sweep or as two kernels
- * (N >= 128), and the persistent grid of the TMA y/z passes (1 .. max CTAs per SM) -- over
- * `trial_steps` steps each (the state advances; results do not depend on the choice) and
- * keeps the fastest.  With a non-NULL cache_path the choice is read from / appended to that
- * file, one line per (device, N, precision) key, so later handles skip the trials.
+ * handle of N = 256 or 512 can run -- the x pass as the two-stage 16 x M plan or the generic
+ * Stockham plan, the forward z pass fused with the k-space sweep or as two kernels, and the
+ * persistent grid of the TMA y/z passes (1 .. max CTAs per SM) -- over `trial_steps` steps
+ * each (the state advances; results do not depend on the choice) and keeps the fastest.
+ * Smaller grids run one shape: nothing is timed, the state stays, and the shape is reported
+ * and cached as it is.  With a non-NULL cache_path the choice is read from / appended to
+ * that file, one line per (device, N, precision) key, so later handles skip the trials.
  * out_config (may be NULL) receives {tma_grid, x2_grid, p5_grid}. */
 int sns_autotune(sns_handle* h, int trial_steps, const char* cache_path, int* out_config);
 

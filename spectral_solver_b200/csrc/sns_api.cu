@@ -161,7 +161,7 @@ struct sns_handle {
   // fixed_step (a fixed step inside a step graph), or null (the step is an argument)
   const double* step_src = nullptr;
   // Step graphs (use_graph): one RK3 step at the size held in fixed_step, and one adaptive
-  // step on the clock.  `key` is the launch configuration a graph was captured with.
+  // step on the clock.  `key` is what a graph was captured with.
   double* fixed_step = nullptr;
   double fixed_dt = 0.0, fixed_nu = -1.0;  // what fixed_step holds
   struct StepGraph {
@@ -641,11 +641,11 @@ bool use_graph(const sns_handle* h) {
   return h->n <= kGraphMaxN && h->nyq_clean && h->sphere_clean && h->warm_steps > 1;
 }
 
-// Capture (once per launch configuration) and replay one step; false when the capture failed,
-// the step then runs launch by launch.
+// Capture (once per form, pruning and compensation) and replay one step; false when the capture
+// failed, the step then runs launch by launch.
 bool replay_step(sns_handle* h, bool on_clock) {
   auto& sg = h->graph[on_clock ? 1 : 0];
-  const std::vector<int> key = {h->form, h->prune, h->comp, h->tma_grid, h->x2_grid, h->p5_grid};
+  const std::vector<int> key = {h->form, h->prune, h->comp};
   if (sg.exec == nullptr || sg.key != key) {
     if (sg.exec) cudaGraphExecDestroy(sg.exec);
     sg.exec = nullptr;
@@ -883,11 +883,9 @@ int finish_handle(sns_handle* h, const char* what) {
   }
 }
 const char* handle_error(const sns_handle* h) { return h->err.c_str(); }
-// Persistent grid of the TMA passes for a small grid (N <= 128): at most max(16, 2N) CTAs.
-// Such solves run many at a time (ensembles, the server), and a pass whose grid covers every
-// SM for a few microseconds of work leaves no room for the other solves' passes; with 2N
-// CTAs the 64-solve ensemble (N = 32..128) steps 11 % faster in FP32, 4 % in FP64.  A lone
-// small solve tuned by sns_autotune keeps the tuned grid.
+// Persistent grid of the TMA passes for a small grid (N <= 128): at most max(16, 2N) CTAs, so that
+// a pass of a few microseconds leaves SMs to other solves.  Small grids run them in sns_nonlinear
+// and in the first stage from a state with content on the plane mx = N/2 only.
 int small_grid_cap(int n, int grid) { return n <= 128 ? std::min(grid, std::max(16, 2 * n)) : grid; }
 
 // Launch shape {tma_grid, x2_grid, p5_grid} as sns_autotune reports it; false if the handle
@@ -897,7 +895,7 @@ bool set_launch_shape(sns_handle* h, const int* cfg) {
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return false;
   const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
   const int tma_max = yz_blocks_per_sm(h);
-  if (cfg[0] < nsm || cfg[0] > nsm * tma_max || (cfg[1] != 0 && cfg[1] != x2_full) ||
+  if (cfg[0] < (h->small ? 1 : nsm) || cfg[0] > nsm * tma_max || (cfg[1] != 0 && cfg[1] != x2_full) ||
       (cfg[2] != 0 && cfg[2] != p5_full))
     return false;
   h->tma_grid = small_grid_cap(h->n, cfg[0]);
@@ -1199,10 +1197,10 @@ int sns_autotune(sns_handle* h, int trial_steps, const char* cache_path, int* ou
     int nsm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "cudaDeviceGetAttribute");
     const int x2_full = h->ops->xpass2_grid(nsm), p5_full = h->p5 ? h->p5->grid(nsm) : 0;
-    const int tma_max = yz_blocks_per_sm(h);
+    const int tma_max = yz_blocks_per_sm(h), tma_min = h->small ? 1 : nsm;
     auto apply = [&](int tma, int x2, int p5) {
       // only shapes this handle was built for: its Nyquist partial buffer is sized for x2_full
-      if (tma < nsm || tma > nsm * tma_max || (x2 != 0 && x2 != x2_full) || (p5 != 0 && p5 != p5_full))
+      if (tma < tma_min || tma > nsm * tma_max || (x2 != 0 && x2 != x2_full) || (p5 != 0 && p5 != p5_full))
         return false;
       h->tma_grid = tma;
       h->x2_grid = x2;
@@ -1227,8 +1225,8 @@ int sns_autotune(sns_handle* h, int trial_steps, const char* cache_path, int* ou
       struct Shape {
         int tma, x2, p5;
       };
-      std::vector<Shape> shapes;
-      for (int k = 1; k <= tma_max && k <= 4; ++k)
+      std::vector<Shape> shapes;  // (none for small grids: their stage has no shape to choose)
+      for (int k = 1; k <= tma_max && k <= 4 && !h->small; ++k)
         for (int x2 : {x2_full, 0})
           for (int p5 : {p5_full, 0}) {
             const Shape sh{nsm * k, x2, p5};
