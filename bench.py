@@ -45,10 +45,11 @@ DT = 1e-3
 # stage, hence 21 on average).
 PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 16, "p3_nyq": 0,
                 "p4_yfwd": 20, "p5_zfwd": 20, "p5_sweep": 21}
-# The fixed byte model of the roofline figure: the same passes with all six products (12 fields).
+# The same passes with all six products (12 fields).
 MODEL_PASS_BYTES_S = {"p1_zinv_phase": 9, "p2_yinv": 12, "p3_xpass": 18, "p3_nyq": 0,
                       "p4_yfwd": 24, "p5_zfwd": 24, "p5_sweep": 23}
-# S per step of that model, nothing pruned (step_bytes_s(1)).
+# S per step of the fixed byte model of the roofline figure: six products, nothing pruned, and g
+# counted as read in every stage, 3 x (9 + 12 + 18 + 24 + 24) = step_bytes_s(1).
 MODEL_BYTES_S = 261
 
 
@@ -75,7 +76,7 @@ def pruned_pass_bytes(n, w):
 
 def step_bytes_s(L):
     """Bytes per RK3 step of the fixed six-product model in units of S: 3 x (P1 9, P2 12, P3 18,
-    P4 24, P5 24L), which is 261 without pruning (L = 1)."""
+    P4 24, P5 24L, g read in every stage), which is 261 without pruning (L = 1)."""
     return 189 + 72 * L
 
 
@@ -354,11 +355,11 @@ def measure_form(args, n, precision, local, pg):
     prof = s.profile_passes(DT, 1)
     w = 8 if precision == 0 else 4
     S = n ** 3 * w
-    # roofline.achieved uses the per-pass algorithmic bytes, the model fraction the fixed model
-    # (261 N^3 w per step); the bytes that the sphere-pruned passes move are reported beside
+    # roofline.achieved uses the bytes that the sphere-pruned pass moves, the model fraction the
+    # fixed model (261 N^3 w per step); the pass's bytes without pruning are reported beside
     pass_bytes, L = moved_pass_bytes(n, w)
     top = max(prof, key=prof.get)
-    achieved = PASS_BYTES_S[top] * S / (prof[top] / 1e3) / 1e9
+    achieved = pass_bytes[top] * S / (prof[top] / 1e3) / 1e9
     peak, peak_kind = load_peaks()
     traffic_table = TRAFFIC_PER_POINT if precision == 0 else TRAFFIC_PER_POINT_FP32
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
