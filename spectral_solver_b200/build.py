@@ -16,6 +16,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -67,14 +68,14 @@ def build_cuda(verbose=False, ptxas_verbose=False, check=False):
         return lib
     objdir = os.path.join(PKG, "_build", "check" if check else "")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
+    objs = [os.path.join(objdir, os.path.basename(cu) + ".o") for cu in cus]
     defs = ["-DSNS_BOUNDS_CHECK"] if check else []
-    for cu in cus:
-        obj = os.path.join(objdir, os.path.basename(cu) + ".o")
-        extra = ["-Xptxas", "-v"] if ptxas_verbose else []
-        if _stale(obj, [cu] + _sources(CSRC, (".cuh", ".h")) + _sources(INC, (".h",))) or ptxas_verbose:
-            _run([NVCC, *ARCH, *NVFLAGS, *defs, *extra, "-I", INC, "-c", cu, "-o", obj], verbose or ptxas_verbose)
-        objs.append(obj)
+    extra = ["-Xptxas", "-v"] if ptxas_verbose else []
+    hdrs = _sources(CSRC, (".cuh", ".h")) + _sources(INC, (".h",))
+    todo = [(cu, obj) for cu, obj in zip(cus, objs) if ptxas_verbose or _stale(obj, [cu] + hdrs)]
+    with ThreadPoolExecutor(max_workers=os.cpu_count()) as pool:  # one nvcc per file
+        list(pool.map(lambda t: _run([NVCC, *ARCH, *NVFLAGS, *defs, *extra, "-I", INC, "-c", t[0], "-o", t[1]],
+                                     verbose or ptxas_verbose), todo))
     _run([NVCC, *ARCH, "-shared", "-o", lib, *objs, "-lcudart"], verbose)
     return lib
 
