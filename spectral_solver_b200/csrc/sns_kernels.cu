@@ -3,15 +3,16 @@
 // form (fields stored in FP32; reductions, Nyquist sums and diagnostics accumulate in FP64).
 //
 // One RK3 stage of the reference (ava_taylor_green_impl.hpp:847-977 compute_rhs plus the
-// stage update :994-1039) is five streaming passes over HBM:
-//   P1 zpass_inv_phase : inverse z transform of u_hat, both grids from one read
-//                        (the phase-shift kernel :866-873 fused in), 1/N^3 folded in
-//   P2 ypass (inverse) : 6 fields
-//   P3 xpass_products  : inverse x (c2r), the 5 products on both grids (6 for the
+// stage update :994-1039) is five streaming passes over HBM (grids of N <= 128 have a stage of
+// their own in sns_small.cu; P1, P2 and P5 of N = 256, 512 are in sns_stream.cu and sns_p5.cu):
+//   P1 inverse z       : u_hat on both grids from one read (the phase-shift kernel
+//                        :866-873 fused in), 1/N^3 folded in
+//   P2 inverse y       : 6 fields
+//   P3 x pass          : inverse x (c2r), the 5 products on both grids (6 for the
 //                        unprojected term), forward x (r2c) of all 10 (product kernel
 //                        :903-906 fused)
-//   P4 ypass (forward) : 10 fields
-//   P5 zpass (forward) + sweep : dealias combine, mask, -i k, viscous term, Leray
+//   P4 forward y       : 10 fields
+//   P5 forward z + sweep : dealias combine, mask, -i k, viscous term, Leray
 //                        projection, low-storage RK3 update, projection of u
 //                        (accumulate :926-936, add_viscous_project :955-974,
 //                        RK update :994-1033, project_truncate :825-844)
@@ -46,65 +47,6 @@ template <int N>
 constexpr int nt_x() { return ((N / 2 < 32 ? 32 : (N / 2 > 256 ? 256 : N / 2)) + 31) / 32 * 32; }
 
 // ------------------------------------------------------------------------------------
-// P1: inverse z transform with the fused phase shift.
-// grid (ntiles, N [my], 3 [component]); tile = kT columns (one 128-byte row segment) x N rows (mz).
-template <int N, class C>
-__global__ void __launch_bounds__(nt_yz<N>())
-k_zpass_inv_phase(const C* __restrict__ u, C* __restrict__ work, const C* __restrict__ tw,
-                  const C* __restrict__ phase, double scale, Geom g) {
-  constexpr int NT = nt_yz<N>();
-  constexpr int kT = tile_cols<C>();
-  extern __shared__ __align__(16) unsigned char smraw_yz[];
-  C* smem = reinterpret_cast<C*>(smraw_yz);
-  C* s_tw = smem;
-  C* tile = smem + N;
-  const int tid = threadIdx.x;
-  load_twiddles<N>(s_tw, tw, tid, NT);
-  const int mx0 = blockIdx.x * kT;
-  const int my = blockIdx.y;
-  const int c = blockIdx.z;
-  const C* src = u + (long long)c * g.field;
-  C* dst0 = work + (long long)(2 * c) * g.field;
-  C* dst1 = work + (long long)(2 * c + 1) * g.field;
-  for (int e = tid; e < kT * N; e += NT) {
-    const int row = e / kT, col = e % kT;
-    tile[e] = cscale(src[((long long)row * N + my) * g.pitch + mx0 + col], scale);
-  }
-  __syncthreads();
-  smem_fft<N, +1, kT, NT, ColTile<kT>>(tile, s_tw, tid);
-  for (int e = tid; e < kT * N; e += NT) {
-    const int row = e / kT, col = e % kT;
-    dst0[((long long)row * N + my) * g.pitch + mx0 + col] = tile[e];
-  }
-  __syncthreads();
-  const int smy = signed_mode(my, N);
-  for (int e = tid; e < kT * N; e += NT) {
-    const int row = e / kT, col = e % kT;
-    // padding columns (> N/2) carry nothing; the Nyquist column mx = N/2 is transformed
-    // too (consumed only when the state's Nyquist plane has content off (N/2,0,0))
-    // Modes with 0 < mx < N/2 and index N/2 in exactly one of y, z: signed_mode gives +N/2
-    // to the mode and to its mirror, so phase(-m) = -conj(phase(m)) and the reference's
-    // shifted field is anti-Hermitian there; the real part it keeps of their inverse
-    // transform is zero.  (With N/2 in both the two shifts cancel.  All of these modes
-    // are zero in a masked state.)
-    const int mx = mx0 + col;
-    const bool anti = mx > 0 && mx < N / 2 && ((my == N / 2) != (row == N / 2));
-    if (mx <= N / 2 && !anti) {
-      const int msum = mx + smy + signed_mode(row, N);
-      const C v = cscale(src[((long long)row * N + my) * g.pitch + mx], scale);
-      tile[e] = cmul(v, phase[msum + 3 * N / 2]);
-    } else {
-      tile[e] = czero<C>();
-    }
-  }
-  __syncthreads();
-  smem_fft<N, +1, kT, NT, ColTile<kT>>(tile, s_tw, tid);
-  for (int e = tid; e < kT * N; e += NT) {
-    const int row = e / kT, col = e % kT;
-    dst1[((long long)row * N + my) * g.pitch + mx0 + col] = tile[e];
-  }
-}
-
 // y pass, in place.  grid (ntiles, N [z], nf).
 template <int N, int DIR, class C>
 __global__ void __launch_bounds__(nt_yz<N>())
@@ -414,7 +356,7 @@ k_xpass_products(C* __restrict__ work, const C* __restrict__ unyq, const C* __re
 // __syncwarp; the CTA synchronises twice per row group: before it starts (the previous
 // group is done, its staging buffer is refilled) and between the inverse and forward
 // FFTs (each product reads two components).
-// The (N/2,0,0) sums of the 12 product planes accumulate in registers per CTA.
+// The (N/2,0,0) sums of the 10 (NP = 6: 12) product planes accumulate in registers per CTA.
 template <int N, class C, int PRODUCTS = 5>
 struct XP {
   static constexpr int M = N / 16;                 // stage-B radix
@@ -1735,11 +1677,6 @@ struct Launch {
   static C* F(void* p) { return static_cast<C*>(p); }
   static const C* F(const void* p) { return static_cast<const C*>(p); }
 
-  static void zpass_inv_phase(const void* u, void* work, const void* tw, const void* phase, double scale,
-                              int ntiles, Geom g, cudaStream_t st) {
-    dim3 grid(ntiles, N, 3);
-    k_zpass_inv_phase<N, C><<<grid, nt_yz<N>(), yz_smem(), st>>>(F(u), F(work), F(tw), F(phase), scale, g);
-  }
   static void ypass(void* f, int nf, int dir, int ntiles, const void* tw, Geom g, cudaStream_t st) {
     dim3 grid(ntiles, N, nf);
     if (dir < 0) {
@@ -1903,7 +1840,6 @@ struct Launch {
       set_smem(k_yz_tma<N, 2, -1, 0, C>, tma_smem<N, C>());
       set_smem(k_yz_tma<N, 2, +1, 0, C>, tma_smem<N, C>());
     }
-    set_smem(k_zpass_inv_phase<N, C>, yz_smem());
     set_smem(k_ypass<N, -1, C>, yz_smem());
     set_smem(k_ypass<N, +1, C>, yz_smem());
     set_smem(k_zpass<N, -1, C>, yz_smem());
@@ -1916,7 +1852,7 @@ struct Launch {
     set_smem(k_xpass_rot<N, C>, x_smem(6));
   }
   static const Ops* table() {
-    static const Ops ops = {N,  (int)sizeof(C), kT, init, zpass_inv_phase, ypass, zpass, xpass_products, nyq_reduce,
+    static const Ops ops = {N,  (int)sizeof(C), kT, init, ypass, zpass, xpass_products, nyq_reduce,
                             sweep, xpass_r2c, xpass_c2r, xpass_diag, yz_tma, tma_blocks_per_sm, xpass2, xpass2_grid,
                             omega_hat, xpass_rot, sweep_rot, xpass_diag2};
     return &ops;

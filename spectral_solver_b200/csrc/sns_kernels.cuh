@@ -81,9 +81,6 @@ struct Ops {
   int complex_bytes;  // 16 (FP64) or 8 (FP32)
   int tile_cols;      // columns per y/z tile (one 128-byte row segment)
   void (*init)();     // kernel attributes; call once per device before the first launch
-  // inverse z pass of u[3] with the phase shift: work fields 2c (U_c), 2c+1 (phase*U_c)
-  void (*zpass_inv_phase)(const void* u, void* work, const void* tw, const void* phase, double scale, int ntiles,
-                          Geom g, cudaStream_t st);
   // y pass (dir -1 forward, +1 inverse) of `nf` consecutive fields, in place; `ntiles` column tiles
   void (*ypass)(void* f, int nf, int dir, int ntiles, const void* tw, Geom g, cudaStream_t st);
   // z pass src -> dst (may alias), optional scale applied on load
