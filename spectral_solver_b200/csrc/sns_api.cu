@@ -3,11 +3,12 @@
 // Device memory of a handle, in half fields of N*N*pitch complex values (double2 in the FP64
 // plain form, float2 in the FP32 precision form):
 //   state : u[3], g[3]            (the reference's u_hat and g, ava_taylor_green_impl.hpp:665-667)
-//   work  : 12 fields             (inverse-transformed velocity on both grids, then the
-//                                  12 product spectra; the fused x pass reads 6 and writes
-//                                  12 rows in place, so one buffer serves both)
+//   work  : 12 fields             (inverse-transformed velocity on both grids, then the 10
+//                                  product spectra, 12 for the unprojected term; the x pass
+//                                  reads 6 and writes 10 or 12 rows in place, so one buffer
+//                                  serves both)
 //   tables: twiddles (N), phase exp(i*pi*(mx+my+mz)/N) for mx+my+mz in [-3N/2, 3N/2],
-//           reduction partials, the 12 Nyquist-plane sums.
+//           reduction partials, the Nyquist-plane partial sums.
 #include "sns_kernels.cuh"
 #include "sns_p5.cuh"
 #include "sns_small.cuh"

@@ -1,8 +1,7 @@
 // The RK3 stage of small grids (N <= 128).  At these sizes the fields sit in L2 and a pass is
 // a few microseconds: what counts is how many launches a stage takes, and that each has every
 // load in flight at once and enough small CTAs to fill the chip.  So no persistent loops and no
-// TMA pipelines here (they serve the large grids in sns_kernels.cu, where a stage takes seven
-// launches at these sizes): four launches a stage,
+// TMA pipelines here (they serve the large grids, six launches a stage): four launches a stage,
 //   k_ysmall : inverse y of the six fields
 //   k_xsmall : inverse x, the five products on both grids, forward x
 //   k_ysmall : forward y of the ten product fields

@@ -17,8 +17,9 @@ __device__ __forceinline__ int signed_mode(int i, int n) { return i <= n / 2 ? i
 // (stepping, sns_rhs) runs on 5: u_0^2 - u_2^2, u_0 u_1, u_0 u_2, u_1^2 - u_2^2, u_1 u_2 --
 // 10 instead of 12 fields through the forward passes.  sns_nonlinear returns the term
 // unprojected and takes the 6.  The differences are formed as (a - b)(a + b), whose rounding
-// error is relative to the difference.  A stage moves 79 instead of 87 N^3 words: a step at
-// 512^3 29.1 -> 26.7 ms (FP32), at 256^3 7.1 -> 6.5 ms (FP64), error against 64 bits unchanged.
+// error is relative to the difference.  A stage moves 78 instead of 86 N^3 words (g read in two
+// stages of three, nothing pruned): a step at 512^3 29.1 -> 26.7 ms (FP32), at 256^3 7.1 -> 6.5 ms
+// (FP64), error against 64 bits unchanged.
 template <class C>
 __device__ __forceinline__ C diff_squares(C a, C b) {
   return cmk((a.x - b.x) * (a.x + b.x), (a.y - b.y) * (a.y + b.y));
