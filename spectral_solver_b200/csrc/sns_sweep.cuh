@@ -25,13 +25,19 @@ __device__ __forceinline__ C diff_squares(C a, C b) {
   return cmk((a.x - b.x) * (a.x + b.x), (a.y - b.y) * (a.y + b.y));
 }
 
-// Product ab of NP: a u_a u_b, or (NP = 5, `sq`) u_a^2 - u_b^2: 00 - 22, 01, 02, 11 - 22, 12.
+// Product ab of NP: u_a u_b, or (NP = 5, true returned) u_a^2 - u_b^2: 00 - 22, 01, 02, 11 - 22, 12.
 template <int NP>
 __device__ __forceinline__ bool product_pair(int ab, int* a, int* b) {
-  const bool sq = NP == 5 && (ab == 0 || ab == 3);
-  *a = ab < 3 ? 0 : (ab < 5 ? 1 : 2);
-  *b = sq ? 2 : (ab < 3 ? ab : (ab < 5 ? ab - 2 : 2));
-  return sq;
+  if constexpr (NP == 5) {
+    const bool sq = ab == 0 || ab == 3;
+    *a = ab >= 3 ? 1 : 0;
+    *b = (sq || ab == 4) ? 2 : ab;
+    return sq;
+  } else {
+    *a = ab < 3 ? 0 : (ab < 5 ? 1 : 2);
+    *b = ab < 3 ? ab : (ab < 5 ? ab - 2 : 2);
+    return false;
+  }
 }
 
 // ------------------------------------------------------------------------------------
